@@ -235,14 +235,18 @@ class Context:
               "t_rebuild", "t_s1_argmin", "t_s2_merge_detect", "t_s3_lists_targets_window", "t_s3_overflow",
               "t_s3c_summaries", "t_kin_rapidity", "t_detect_s2", "t_steps", "t_events", "exact_key", "exact_nn",
               "t_targets", "t_target_steps", "t_list_update", "t_targets_warp1", "t_window_thread0",
-              "t_resolve_new_jet", "t_summary_new_jet_tile", "t_summaries_warp1")
+              "t_resolve_new_jet", "t_summary_new_jet_tile", "t_summaries_warp1",
+              "r_setup", "r_candidates", "r_range", "r_keys", "r_b", "r_c", "r_d", "r_e", "r_f", "r_sort", "r_outputs",
+              "r_rounds", "r_steps", "r_events", "r_retries", "r_cands",
+              "r_conflict_a", "r_conflict_b", "r_conflict_d", "r_targets", "r_kin",
+              "r_role0", "r_role1", "r_role2", "r_scan", "r_new_jet", "r_search", "r_dead", "r_overflows")
 
     def phase_clocks(self, reset=False):
         """Per-step phase counters of the clustering kernels (only in the
         -DFJG_PHASE_CLOCKS build, see fastjet_gpu_gb300.phases): a dict of
         summed clock cycles per phase, steps and events (t_*: tiled kernel)."""
-        buf = (ctypes.c_ulonglong * 32)()
-        self._check(lib().fjg_phase_clocks(self._h, buf, 32, 1 if reset else 0))
+        buf = (ctypes.c_ulonglong * len(self.PHASES))()
+        self._check(lib().fjg_phase_clocks(self._h, buf, len(self.PHASES), 1 if reset else 0))
         return {k: int(buf[i]) for i, k in enumerate(self.PHASES) if k}
 
     def _after_torch(self, device):

@@ -50,7 +50,7 @@ cudaError_t ScratchSet::reserve_lists(int n_events) {
   if (sc.order && sc.cap_events >= n_events) return cudaSuccess;
   int cap = n_events + n_events / 4 + 64;
   const size_t hist_bytes = (sizeof(int32_t) * kHistBins + 255) & ~size_t(255);
-  size_t bytes = sizeof(int32_t) * (size_t)kNumQueues * cap + 256 + hist_bytes;
+  size_t bytes = sizeof(int32_t) * (size_t)kNumLists * cap + 256 + hist_bytes;
   cudaError_t err = lists.reserve(bytes);
   if (err != cudaSuccess) return err;
   char* p = static_cast<char*>(lists.ptr);
@@ -85,6 +85,18 @@ cudaError_t ScratchSet::reserve_large(int64_t particles) {
   sc.large_ws = static_cast<unsigned char*>(large.ptr);
   sc.large_ws_particles = (int64_t)((large.cap - 256) / kLargeWsBytesPerParticle);
   return cudaSuccess;
+}
+
+void ScratchSet::reserve_rounds(int64_t particles) {
+  if (sc.round_ws && sc.round_ws_particles >= particles) return;
+  sc.round_ws = nullptr;
+  sc.round_ws_particles = 0;
+  if (rounds.reserve((size_t)kRoundBytesPerParticle * (size_t)particles + 256) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  sc.round_ws = static_cast<unsigned char*>(rounds.ptr);
+  sc.round_ws_particles = (int64_t)((rounds.cap - 256) / kRoundBytesPerParticle);
 }
 
 }  // namespace fjg
@@ -142,7 +154,7 @@ fjg_status fjg_ctx_create(int device, fjg_ctx** out) {
   DeviceGuard g(device);
   err = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-  for (int b = 0; b < fjg::kNumQueues && err == cudaSuccess; ++b) {
+  for (int b = 0; b < fjg::kNumSide && err == cudaSuccess; ++b) {
     err = cudaStreamCreateWithFlags(&ctx->side[b], cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&ctx->ev_join[b], cudaEventDisableTiming);
   }
@@ -165,7 +177,7 @@ void fjg_ctx_destroy(fjg_ctx* ctx) {
   if (!ctx) return;
   DeviceGuard g(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  for (int b = 0; b < fjg::kNumQueues; ++b) {
+  for (int b = 0; b < fjg::kNumSide; ++b) {
     if (ctx->side[b]) {
       cudaStreamSynchronize(ctx->side[b]);
       cudaStreamDestroy(ctx->side[b]);
@@ -200,7 +212,7 @@ fjg_status fjg_phase_clocks(fjg_ctx* ctx, unsigned long long* out, int n, int re
 fjg_status fjg_ctx_check(fjg_ctx* ctx) {
   if (!ctx) return set_error(nullptr, FJG_EINVAL, "ctx is null");
   DeviceGuard g(ctx->device);
-  for (int b = 0; b < fjg::kNumQueues; ++b) cudaStreamSynchronize(ctx->side[b]);
+  for (int b = 0; b < fjg::kNumSide; ++b) cudaStreamSynchronize(ctx->side[b]);
   return take_status(ctx, ctx->stream);
 }
 
@@ -217,6 +229,7 @@ fjg_status fjg_cluster_batch(fjg_ctx* ctx, const double* p4, const int64_t* offs
   cudaError_t err = ctx->scratch.reserve_lists(n_events);
   if (err == cudaSuccess) err = ctx->scratch.reserve_ws(total);
   if (err == cudaSuccess) err = ctx->scratch.reserve_large(total);
+  if (err == cudaSuccess) ctx->scratch.reserve_rounds(total);
   if (err != cudaSuccess) return cuda_error(ctx, err, "scratch allocation");
   cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
   BatchArgs A{};
@@ -317,6 +330,7 @@ fjg_status fjg_cluster_event(fjg_ctx* ctx, const double* p4, int n, int algo, do
   if (n > fjg::kLargeMaxN) return set_error(ctx, FJG_ETOOBIG, "event exceeds the supported particle count");
   cudaError_t werr = ctx->scratch.reserve_ws(n);
   if (werr == cudaSuccess) werr = ctx->scratch.reserve_large(n);
+  if (werr == cudaSuccess) ctx->scratch.reserve_rounds(n);
   if (werr != cudaSuccess) return cuda_error(ctx, werr, "workspace allocation");
   BatchArgs A{};
   A.phase = ctx->phase;
@@ -363,6 +377,7 @@ fjg_status fjg_cluster_pseudojets(fjg_ctx* ctx, fjg_pseudojet* particles, int si
   cudaError_t err = ctx->single.reserve(b_jets + b_lab + 256);
   if (err == cudaSuccess) err = ctx->scratch.reserve_ws(size);
   if (err == cudaSuccess) err = ctx->scratch.reserve_large(size);
+  if (err == cudaSuccess) ctx->scratch.reserve_rounds(size);
   if (err != cudaSuccess) return cuda_error(ctx, err, "device buffers");
   char* d = static_cast<char*>(ctx->single.ptr);
   double* jets = reinterpret_cast<double*>(d);

@@ -68,7 +68,14 @@ enum PhaseSlot {
   // targets, thread 0's share of the window pass; warp 0's resolution of the
   // new jet's neighbour and its tile's summary, warp 1's other summaries
   kPhTListUpd = 26, kPhTTargetsW1, kPhTWindowT0, kPhTResolveA, kPhTSumA, kPhTSumW1,
-  kPhSlots = 32
+  // the rounds kernel: set-up, the phases A (candidates; range test; keys), B to
+  // F of a round, sort, outputs; rounds, steps, events, events left to the
+  // step-by-step kernels
+  kPhRSetup = 32, kPhRCand, kPhRRange, kPhRKeys, kPhRB, kPhRC, kPhRD, kPhRE, kPhRF, kPhRSort, kPhROut, kPhRRounds,
+  kPhRSteps, kPhREvents, kPhRRetries, kPhRCands,
+  kPhRConflictA, kPhRConflictB, kPhRConflictD, kPhRTargets, kPhRKin,
+  kPhRRole0, kPhRRole1, kPhRRole2, kPhRScan, kPhRNewJet, kPhRSearch, kPhRDead, kPhROverflows,
+  kPhSlots = 61
 };
 #ifdef FJG_PHASE_CLOCKS
 #define FJG_PH(...) __VA_ARGS__
@@ -105,6 +112,12 @@ struct BatchArgs {
   int32_t* owner;          // [total] or null
   int* status;             // device error flag (0 = ok)
   unsigned char* large_ws; // tiled-path workspace: event e at large_ws + 96 * offsets[e] (null: none)
+  int rounds_mode;         // which events the rounds kernel takes (rounds_take); the others skip them
+  unsigned char* round_ws; // rounds kernel's workspace: event e at round_ws + kRoundBytesPerParticle * offsets[e]
+  int round_tiles, round_cells, round_slots;  // rounds kernel: what its shared memory has room for (tiles,
+                                              // tiles with their frame, slots)
+  int32_t* retry;          // rounds kernel: events left to the step-by-step kernels, and their count
+  int32_t* n_retry;
   double tile_factor;      // tiled path: tile side >= tile_factor * R (>= 1)
   int serve_order;         // launch priority (host side): 0 largest events first, 1 smallest first
   int pairs;               // offsets hold (start, end) pairs: events need not be contiguous

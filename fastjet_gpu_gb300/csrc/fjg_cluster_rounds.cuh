@@ -1,0 +1,1699 @@
+// Clustering of one event per CTA in rounds of independent steps (sm_103a).
+//
+// The sequential algorithm takes one merge or promotion per step, the one with
+// the smallest key.  What it does in one place of the rapidity-azimuth plane
+// depends only on what happened within R of there, so steps far enough apart
+// commute: their order decides the order of the output records, not what is
+// merged.  This kernel fires many steps per round, each where it is the next
+// one of its surroundings, checks that firing them early changed nothing, and
+// sorts the records into the sequential order at the end.  A step-by-step
+// kernel spends its time in latency (an FP64 kinematics chain, reductions,
+// barriers); a round pays that once for all its steps.
+//
+// Sequential time.  The step E that merges c and j (or promotes c) with exact
+// key k and label l (the winner's label; the lower one of mutual neighbours)
+// has the time
+//     T(E) = (k, l, 0)               if (k, l) > (M, m) of T(c) and T(j),
+//            the larger of T(c), T(j) with its depth one higher   otherwise,
+// where T(c) = (M, m, depth) is the time of the step that made c (before every
+// time for an input particle).  In the sequential run the times of the steps
+// increase: a step whose key is below an earlier one's became possible only
+// with the step that made one of its pseudojets, and follows it directly.
+// Conversely a set of steps sorted by T is the sequential run if, whenever two
+// pseudojets x and y exist at the same time and E is the first step (in T) that
+// takes either, then T(E) < T(x, y), the time the pair would have, and
+// T(E) < the time of the promotion of the one it takes -- E being that pair or
+// promotion excepted: the sequential run would otherwise have taken the pair or
+// promotion first.  Two checks establish this; each compares in FP32 intervals
+// and in FP64 where those cannot decide:
+//   D1  when E fires: against every pseudojet within R of c and of j that
+//       exists in the same round (before the round's steps are applied);
+//   D2  when E makes a new jet a: against every pseudojet within R of a that a
+//       step with a later time than T(E) has already taken.
+// Two pseudojets that exist in the same round are covered by D1 of the first
+// step that takes one of them, two that never do by D2 of the later one.
+// T(x, y) >= d_xy, so with thr = k for the one whose own time sets a chained
+// T(E) and thr = T(E)'s key part for the other, a pair is a conflict only if
+// d_xy <= thr (an exact tie counts), d_xy is at most both weights and the other
+// is not younger than E.  An event with a conflict is handed to the
+// step-by-step kernel (retry list) and this kernel's work on it is dropped, so
+// the rule that picks the steps of a round only has to be good, not proven.
+//
+// Choice of a round's steps.  Tiles of side >= R/2; per tile the slot with the
+// smallest (P, key), P being the FP32 lower bound of its step's time.  A tile
+// whose minimum is the smallest of its 5x5 tiles is a candidate; it fires if
+// no tile closer to c than 1.5 R and the distance of c and j (from the point to
+// the tile) has an earlier minimum.  For kt and C/A, whose weights do not fall
+// in a merge, the range shrinks to that of pairs with d below the candidate's
+// P.  Steps a round on the benchmark's kind of events: anti-kt R = 0.4 4 at 200
+// particles, 10 at 1500, 8 to 6 at 8000 to 40,000 dense ones, R = 0.8 3; kt R =
+// 0.6 12 at 1000, 14 at 20,000; C/A R = 0.8 8 at 1000.  Conflicts: none in 1100
+// events of up to 4000 particles (anti-kt R = 0.4, kt, C/A), in about 2 % of
+// anti-kt R = 0.8 events of 3000, in 2 to 6 % of dense anti-kt R = 0.4 events of
+// 8000 to 15,000 and in half of those of 30,000 and more, where a hard jet's
+// chain of steps reaches further; those begin with a range of 2 R (none in 120
+// events).
+//
+// A round (F steps), eight warps or so:
+//   A   candidates (a thread per tile); range test (eight lanes per candidate),
+//       and the keys, times and thresholds of the steps that pass.
+//   B   new jets' azimuth, rapidity and weight: three warps, a lane per step;
+//       meanwhile the other warps go over the windows of c and j: D1, and the
+//       slots whose neighbour is taken ("targets").
+//   C   the new jets' state and the tile lists (a lane per step).
+//   D   the new jets' windows (their neighbours; slots they are closer to), the
+//       targets' searches, and D2 over the dead of the new jets' windows, by
+//       groups of 8 or 32 lanes.
+//   E   slots to which two new jets were closer: searched.
+//   F   changed tiles: lists compacted, minima taken.
+//
+// Windows are the 5x5 tiles around a slot's tile; they hold everything within
+// R (1 + 1e-4).  fjg_cluster_tiled.cuh proves that windowed neighbours select
+// what the all-pairs rule selects.
+#pragma once
+
+#include <type_traits>
+
+#include "fjg_cluster.cuh"
+
+namespace fjg {
+
+// Which events the rounds kernel takes.  Its gain is the number of steps a round
+// holds, which falls with R^2 (the area a step keeps to itself), and a round
+// costs about three steps of the step-by-step kernels.  kRoundsFew: an SM or
+// more per event, the event's latency counts; kRoundsMany: the SMs are shared,
+// instructions count, of which a round's fixed part is many for small events.
+// Measured (GB300; step by step -> rounds, anti-kt unless noted):
+//   one event    R 0.4: 80 particles 0.44 -> 0.50 ms, 120 0.56 -> 0.53, 250 1.18 -> 0.67, 3000 14.6 -> 4.5
+//                R 0.8: 300 1.87 -> 1.31, 3000 15.3 -> 12.4;  R 1.0: 800 4.2 -> 3.3, 1500 6.8 -> 7.9
+//                C/A R 1.2: 300 1.95 -> 1.23, 3000 16.3 -> 10.4
+//   batches      R 0.4: 2000 of 260-512 6.9 -> 6.3, 1000 of 600-1000 11.1 -> 5.9, 600 of 1100-2000 18.0 -> 6.9
+//                R 0.6: 1000 of 600-1000 11.1 -> 9.3, 600 of 1100-2000 17.8 -> 17.9
+//                kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
+//                kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
+//   above 4096   R 0.4: 9000 93 -> 31;  R 0.6: 92 -> 54;  R 0.8: 97 -> 74, where later steps conflict more often
+enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsFew = 2 };
+
+__host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
+  if (mode == kRoundsNone) return false;
+  if (n > 4096) return algo == -1 ? R <= 0.65 : R <= 1.5;
+  if (mode == kRoundsFew) return n >= 112 && (algo == -1 ? R <= 0.85 || (R <= 1.05 && n <= 1024) : R <= 1.5);
+  if (n <= 512) return n >= 400 && R <= (algo == -1 ? 0.42 : 0.6);
+  return R <= (algo == -1 ? 0.55 : n <= 1024 ? 1.0 : 1.3);
+}
+
+// The same for an event of a batch.
+__device__ __forceinline__ bool rounds_event(const BatchArgs& A, int e) {
+  if (A.rounds_mode == kRoundsNone) return false;
+  int64_t off;
+  int n;
+  event_range(A, e, off, n);
+  return rounds_take(A.rounds_mode, n, A.algo ? A.algo[e] : A.algo_all, A.radius ? A.radius[e] : A.r_all);
+}
+
+constexpr int kRoundSteps = 32;               // steps per round, at most (a lane each)
+constexpr int kRoundBytesPerParticle = 240;   // workspace
+constexpr int kRoundMaxDirty = 512;
+constexpr int kRoundMaxTargets = 256;
+constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, also in one row
+// range of the choice of steps, in units of R (see above): the first attempt at
+// an event, the second (the first for the largest anti-kt events), the last
+__constant__ const float kRoundReach[3] = {1.5f, 2.0f, 2.5f};
+constexpr int kRoundWideFrom = 20000;
+constexpr int kRoundMaxTiles = 2048;
+constexpr int kRoundMaxCells = 3072;          // with the frame
+constexpr int kRoundFrame = 5;                // tiles around the grid: the range test's 1.5 R + R
+constexpr int kRoundDense = 4;                // live slots per tile from which a warp reads lists together
+constexpr int kRoundSmemMaxN = 4096;
+constexpr int kRoundSlotBytes = 36;           // shared memory per slot
+
+// One step, stored at the slot it removes.
+struct alignas(16) RoundRec {
+  double M;   // its time: (M, l, depth)
+  double d;   // recorded distance
+  int l, depth;
+  int a;      // merged into slot a, or -1 (promotion)
+  int pad;
+};
+
+struct RoundTime {
+  double M;
+  int l, depth;
+};
+
+__device__ __forceinline__ bool time_less(const RoundTime& x, const RoundTime& y) {
+  if (x.M != y.M) return x.M < y.M;
+  if (x.l != y.l) return x.l < y.l;
+  return x.depth < y.depth;
+}
+
+constexpr unsigned kRoundNone = 0xffffffffu;  // a tile without slots (P as a bit pattern; P >= 0 orders as integer)
+
+// The event's state: what every round reads in shared memory (SM: events of up
+// to kRoundSmemMaxN particles, 36 bytes a slot, so that two CTAs share an SM) or
+// in the global workspace; what single slots need, the dead and the records
+// always in the workspace.
+template <bool SM>
+struct RoundWs {
+  using Idx = typename std::conditional<SM, unsigned short, int>::type;  // slots, tiles, list positions
+  static constexpr int kRoom = SM ? 3 : 4;  // list entries per particle
+  static constexpr int kNone = SM ? 0xffff : -1;
+  // neighbour field: slot, or kNoSlot; a target of this round; the key is the pair distance
+  static constexpr int kSlotMask = SM ? 0x1fff : 0x1ffffff, kNoSlot = kSlotMask;
+  static constexpr int kTarget = SM ? 0x4000 : 0x20000000, kPair = SM ? 0x8000 : 0x40000000;
+  float2* xy;     // [N] rap32, phi32
+  float2* key;    // [N] lower bounds of the key, and of its step's time (P)
+  float* nhi;     // [N] neighbour distance, upper bound
+  float* wlo;     // [N] weight, lower bound; negated: the upper bound is the next float up
+  Idx* nn;        // [N] neighbour field
+  Idx* tile;      // [N] kNone: taken
+  Idx* at;        // [N] position in its tile's list
+  Idx* members;   // [kRoom * N]
+  float2* lxy;    // [kRoom * N] coordinates in list order, read with consecutive lanes (not SM)
+  double2* pos;   // [N] rapidity, azimuth
+  float* nlo;     // [N] neighbour distance, lower bound
+  float* tlo;     // [N] birth time's M, rounded down
+  double* tm;     // [N] birth time M
+  int2* tl;       // [N] birth time l, depth
+  int2* stamp;    // [N] round in which it was taken by a step, or given a new neighbour (SM: bits in S)
+  float4* dgeo;   // [2N] dead: rap32, phi32, wlo, threshold rounded up; 2b and 2b+1: what the step
+                  //      that removed slot b took
+  int4* dgrp;     // [2N] groups of the dead of one tile with the same M and l: next group (by descending
+                  //      M), its M rounded up (float), first member, l
+  int* dnext;     // [2N] next member
+  RoundRec* rec;  // [N]
+  // coordinates of slot u, entry i of the lists
+  __device__ __forceinline__ float2 entry(int u, int i) const { return SM ? xy[u] : lxy[i]; }
+  __device__ __forceinline__ void place(int i, int u, float2 g) const {
+    members[i] = (Idx)u;
+    if (!SM) lxy[i] = g;
+  }
+  __device__ __forceinline__ double dr2(int s, int t) const {
+    const double2 a = pos[s], b = pos[t];
+    return dr2_64(a.x, a.y, b.x, b.y);
+  }
+};
+
+template <bool SM>
+__device__ __forceinline__ RoundWs<SM> round_ws(unsigned char* base, unsigned char* smem, int N, int cap) {
+  RoundWs<SM> W;
+  using Idx = typename RoundWs<SM>::Idx;
+  const int64_t n = N;
+  W.dgeo = reinterpret_cast<float4*>(base);
+  W.dgrp = reinterpret_cast<int4*>(base + 32 * n);
+  W.rec = reinterpret_cast<RoundRec*>(base + 64 * n);
+  W.pos = reinterpret_cast<double2*>(base + 96 * n);
+  W.tm = reinterpret_cast<double*>(base + 112 * n);
+  W.tl = reinterpret_cast<int2*>(base + 120 * n);
+  W.stamp = reinterpret_cast<int2*>(base + 128 * n);
+  W.dnext = reinterpret_cast<int*>(base + 136 * n);
+  W.nlo = reinterpret_cast<float*>(base + 144 * n);
+  W.tlo = W.nlo + n;
+  W.lxy = reinterpret_cast<float2*>(base + 152 * n);
+  // 184 n bytes; then, in the workspace, 52 n more
+  unsigned char* p = SM ? smem : base + 184 * n;
+  const int64_t m = SM ? cap : N;
+  W.xy = reinterpret_cast<float2*>(p);
+  W.key = W.xy + m;
+  W.nhi = reinterpret_cast<float*>(W.key + m);
+  W.wlo = W.nhi + m;
+  W.nn = reinterpret_cast<Idx*>(W.wlo + m);
+  W.tile = W.nn + m;
+  W.at = W.tile + m;
+  W.members = W.at + m;
+  return W;
+}
+
+__device__ __forceinline__ float round_wlo(float w) { return fabsf(w); }
+__device__ __forceinline__ float round_whi(float w) {
+  return __float_as_int(w) < 0 ? __int_as_float((__float_as_int(w) & 0x7fffffff) + 1) : w;
+}
+__device__ __forceinline__ float round_weight(double w) {
+  const float lo = __double2float_rd(w);
+  return __double2float_ru(w) == lo ? lo : -lo;
+}
+
+// Fixed part of a CTA's shared memory.
+struct RoundShared {
+  // the event, for the routines that stay out of line
+  EventCtx X;
+  unsigned char* ws;
+  float r2hi;  // R^2 rounded up, a little more
+  int tiles, cells, slots;  // room
+  double rmin, inv_side_r, inv_side_phi;
+  int nrap, nphi, sh, nt, pw;  // tile (u, v) is u << sh | v; nt = nrap << sh
+  int lut[16];                 // 2^16 / k, rounded up
+  double red[3][16];
+  int scan_tmp[16];
+  int event, overflow;
+  // conflict flags of a round's phases A, B and D: each is read after the
+  // barrier that closes its phase and written again only a round later, so
+  // every thread of the CTA takes the same way
+  int conflict[3];
+  int n_cand, n_fire, n_targets, n_dirty;
+  int task[2];
+  // the round's steps: c, j (-1: promotion), tile and list position of the
+  // slots they remove and keep, tile of the new jet
+  int c[kRoundSteps], j[kRoundSteps], l[kRoundSteps], depth[kRoundSteps];
+  int2 tp_b[kRoundSteps], tp_a[kRoundSteps];
+  int new_u[kRoundSteps], new_v[kRoundSteps];
+  double M[kRoundSteps], key[kRoundSteps], thr_c[kRoundSteps], thr_j[kRoundSteps];
+  double phi[kRoundSteps], rap[kRoundSteps], w[kRoundSteps], p4[4][kRoundSteps];
+  int targets[kRoundMaxTargets];
+  unsigned short cand[kRoundMaxCand];  // tiles
+  unsigned short dirty[kRoundMaxDirty];
+  unsigned dirty_bits[kRoundMaxTiles / 32];
+  // SM: slots taken by a step of this round, and given a new neighbour
+  unsigned taken[kRoundSmemMaxN / 32], claimed[kRoundSmemMaxN / 32];
+};
+
+// After it, `cells` minima of P with the grid's frame (kRoundFrame on each side;
+// columns of the frame repeat the tiles across the azimuth seam, so that a
+// neighbourhood is read without wrapping) and 5-tile row minima, then `tiles`
+// entries of the per-tile arrays, then the slots.
+__host__ __device__ __forceinline__ size_t round_tile_bytes(int tiles, int cells) {
+  return ((size_t)cells * 12 + (size_t)tiles * 20 + 16 + 15) & ~size_t(15);
+}
+__host__ __device__ __forceinline__ size_t round_tile_bytes_sm(int tiles, int cells) {
+  return ((size_t)cells * 8 + (size_t)tiles * 16 + 16 + 15) & ~size_t(15);
+}
+__host__ __device__ __forceinline__ size_t round_tiles_at() { return (sizeof(RoundShared) + 15) & ~size_t(15); }
+template <bool SM>
+__host__ __device__ __forceinline__ size_t round_slots_at(int tiles, int cells) {
+  return round_tiles_at() + (SM ? round_tile_bytes_sm(tiles, cells) : round_tile_bytes(tiles, cells));
+}
+template <bool SM>
+__host__ __device__ __forceinline__ size_t round_smem_bytes(int tiles, int cells, int slots) {
+  return round_slots_at<SM>(tiles, cells) + (size_t)slots * kRoundSlotBytes;
+}
+
+template <bool SM>
+struct RoundCtx {
+  using Idx = typename RoundWs<SM>::Idx;
+  RoundShared* S;
+  unsigned* tmin;  // [cells] smallest P of the tile's slots
+  unsigned* row;   // [cells] smallest P of the five tiles around, in the row
+  unsigned* near;  // [cells] smallest P of a step that takes a slot of the tile (SM: tmin)
+  int* count;      // [nt]
+  int* head;       // [nt] groups of the dead
+  float* head_m;   // [nt] the first one's M (0: none)
+  Idx* slot;       // [nt] the slot of the minimum
+  Idx* start;      // [nt + 1]
+  RoundWs<SM> W;
+};
+
+// The context, from shared memory (the per-slot pointers need the event set).
+template <bool SM>
+__device__ __forceinline__ RoundCtx<SM> round_ctx() {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RoundCtx<SM> C;
+  C.S = reinterpret_cast<RoundShared*>(smem_raw);
+  const int tiles = C.S->tiles, cells = C.S->cells;
+  C.tmin = reinterpret_cast<unsigned*>(smem_raw + round_tiles_at());
+  C.row = C.tmin + cells;
+  C.near = SM ? C.tmin : C.row + cells;
+  C.count = reinterpret_cast<int*>(C.row + (SM ? cells : 2 * cells));
+  C.head = C.count + tiles;
+  C.head_m = reinterpret_cast<float*>(C.head + tiles);
+  C.slot = reinterpret_cast<typename RoundCtx<SM>::Idx*>(C.head_m + tiles);
+  C.start = C.slot + tiles;
+  C.W = round_ws<SM>(C.S->ws, smem_raw + round_slots_at<SM>(tiles, cells), C.S->X.N, C.S->slots);
+  return C;
+}
+
+__device__ __forceinline__ int round_u(const RoundShared& S, double rap) {
+  const int u = (int)floor((rap - S.rmin) * S.inv_side_r);
+  return u < 0 ? 0 : (u >= S.nrap ? S.nrap - 1 : u);
+}
+
+__device__ __forceinline__ int round_v(const RoundShared& S, double phi) {
+  const int v = (int)floor(phi * S.inv_side_phi);
+  return v < 0 ? 0 : (v >= S.nphi ? S.nphi - 1 : v);
+}
+
+// A box of tiles: nu rows from u0, nv columns from v0 (wrapping; nv <= 9).
+struct RoundBox {
+  int u0, nu, v0, nv;
+};
+
+// The smallest box holding the windows (5x5 tiles) of tiles t1 and t2, which
+// lie within each other's.
+__device__ __forceinline__ RoundBox round_box(const RoundShared& S, int t1, int t2) {
+  const int u1 = t1 >> S.sh, v1 = t1 & ((1 << S.sh) - 1);
+  const int u2 = t2 >> S.sh, v2 = t2 & ((1 << S.sh) - 1);
+  RoundBox b;
+  b.u0 = max(min(u1, u2) - 2, 0);
+  b.nu = min(max(u1, u2) + 2, S.nrap - 1) - b.u0 + 1;
+  int dv = v2 - v1;
+  if (2 * dv > S.nphi) dv -= S.nphi;
+  if (2 * dv < -S.nphi) dv += S.nphi;
+  b.nv = 5 + abs(dv);
+  b.v0 = v1 - 2 + min(dv, 0);
+  if (b.v0 < 0) b.v0 += S.nphi;
+  if (b.nv >= S.nphi) {
+    b.v0 = 0;
+    b.nv = S.nphi;
+  }
+  return b;
+}
+
+// Tile k of a box.
+__device__ __forceinline__ int box_tile(const RoundShared& S, const RoundBox& b, int k) {
+  const int du = (k * S.lut[b.nv]) >> 16;
+  int v = b.v0 + (k - du * b.nv);
+  if (v >= S.nphi) v -= S.nphi;
+  return ((b.u0 + du) << S.sh) + v;
+}
+
+// fn(slot, load(slot, entry)) for every list entry of the box's tiles k0 .. n-1,
+// by a group of G lanes (G = 8 or 32, the same in the whole warp; the functions
+// hold no warp collectives).  Dense lists in the workspace (G = 32): five tiles
+// at a time, a lane per member, so that five loads are in flight.  Otherwise a
+// lane per tile, two members at a time.  List lengths are bounded by the
+// tile's room.
+template <bool SM, class Load, class Fn>
+__device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox& b, int k0, int n, int G, bool dense,
+                                          Load load, Fn fn) {
+  const RoundShared& S = *C.S;
+  constexpr int kNone = RoundWs<SM>::kNone;
+  if (!SM && dense) {
+    constexpr int B = 5;
+#pragma unroll 1
+    for (; k0 < n; k0 += B) {
+      int st[B], ln[B], most = 0;
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        const int t = box_tile(S, b, k0 + q < n ? k0 + q : k0);
+        st[q] = C.start[t];
+        ln[q] = k0 + q < n ? min(C.count[t], (int)C.start[t + 1] - st[q]) : 0;
+        most = max(most, ln[q]);
+      }
+#pragma unroll 1
+      for (int i = threadIdx.x & 31; i < most; i += 32) {
+        int u[B];
+        decltype(load(0, 0)) d[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q) u[q] = i < ln[q] ? (int)C.W.members[st[q] + i] : kNone;
+#pragma unroll
+        for (int q = 0; q < B; ++q) d[q] = load(u[q] != kNone ? u[q] : 0, st[q] + (i < ln[q] ? i : 0));
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+          if (u[q] != kNone) fn(u[q], d[q]);
+      }
+    }
+  } else {
+#pragma unroll 1
+    for (int k = k0 + (threadIdx.x & (G - 1)); k < n; k += G) {
+      const int t = box_tile(S, b, k);
+      const int st = C.start[t], m = min(C.count[t], (int)C.start[t + 1] - st);
+#pragma unroll 1
+      for (int i = 0; i < m; i += 2) {
+        const int u0 = C.W.members[st + i], u1 = i + 1 < m ? (int)C.W.members[st + i + 1] : kNone;
+        const auto d0 = load(u0 != kNone ? u0 : 0, st + i), d1 = load(u1 != kNone ? u1 : 0, st + i + (i + 1 < m ? 1 : 0));
+        if (u0 != kNone) fn(u0, d0);
+        if (u1 != kNone) fn(u1, d1);
+      }
+    }
+  }
+  __syncwarp();
+}
+
+template <bool SM, class Load, class Fn>
+__device__ __forceinline__ void for_box(const RoundCtx<SM>& C, const RoundBox& b, int G, bool dense, Load load, Fn fn) {
+  for_tiles(C, b, 0, b.nu * b.nv, G, dense, load, fn);
+}
+
+// Combination of certificates over groups of G lanes (all lanes call).
+__device__ __forceinline__ Cert cert_group(Cert c, int G) {
+  if (G == 32) return cert_warp(c);
+#pragma unroll 1
+  for (int o = G / 2; o; o >>= 1) {
+    Cert y;
+    y.m1 = __shfl_xor_sync(kFull, c.m1, o);
+    y.i1 = __shfl_xor_sync(kFull, c.i1, o);
+    y.u1 = __shfl_xor_sync(kFull, c.u1, o);
+    y.m2 = __shfl_xor_sync(kFull, c.m2, o);
+    if (y.m1 < c.m1 || (y.m1 == c.m1 && (unsigned)y.i1 < (unsigned)c.i1)) {
+      y.m2 = fminf(y.m2, c.m1);
+      c = y;
+    } else {
+      c.m2 = fminf(c.m2, y.m1);
+    }
+  }
+  return c;
+}
+
+__device__ __forceinline__ void round_dirty(RoundShared& S, int t) {
+  const unsigned bit = 1u << (t & 31);
+  if (!(atomicOr(&S.dirty_bits[t >> 5], bit) & bit)) {
+    const int k = atomicAdd(&S.n_dirty, 1);
+    if (k < kRoundMaxDirty) S.dirty[k] = (unsigned short)t;
+  }
+}
+
+__device__ __forceinline__ void round_target(RoundShared& S, int t) {
+  const int k = atomicAdd(&S.n_targets, 1);
+  if (k < kRoundMaxTargets) S.targets[k] = t;
+}
+
+// True for the first caller of a round: slot s is taken by a step (claim = 0),
+// or given a new neighbour (1).
+template <bool SM>
+__device__ __forceinline__ bool round_first(const RoundCtx<SM>& C, int s, int round, int claim) {
+  if (SM) {
+    const unsigned bit = 1u << (s & 31);
+    return !(atomicOr((claim ? C.S->claimed : C.S->taken) + (s >> 5), bit) & bit);
+  }
+  return atomicExch(claim ? &C.W.stamp[s].y : &C.W.stamp[s].x, round) != round;
+}
+
+// The routines that a round's lanes call for single slots stay out of line: the
+// kernel's straight-line code would not fit the instruction caches otherwise
+// (400 KB inlined; a round took 1.5 to 2 times as long).
+
+// Slot t's neighbour nn with distance interval [lo, hi]: neighbour, key and P;
+// the tile is marked as changed.  The FP32 filter's interval is wide for close
+// pairs (its bound is absolute), which FP64 settles, so that keys compare well.
+template <bool SM>
+__device__ __noinline__ void round_set(int t, int nn, float lo, float hi) {
+  using Ws_ = RoundWs<SM>;
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const EventCtx& X = C.S->X;
+  const float w = C.W.wlo[t], tlo = C.W.tlo[t];
+  round_dirty(*C.S, C.W.tile[t]);
+  float klo = round_wlo(w), p = fmaxf(klo, tlo);
+  int field = Ws_::kNoSlot;
+  if (nn < 0) {
+    lo = hi = __int_as_float(0x7f800000);
+  } else {
+    const float wn = C.W.wlo[nn], tn = C.W.tlo[nn];
+    if (hi - lo > lo * 0x1p-16f) {
+      const double d = C.W.dr2(t, nn);
+      lo = __double2float_rd(d);
+      hi = __double2float_ru(d);
+    }
+    float khi;
+    int kind = key_interval(klo, round_whi(w), round_wlo(wn), round_whi(wn), lo, hi, X.ilo, X.ihi, klo, khi);
+    if (kind < 0) {
+      const double w64 = X.g.at(kW, t);
+      const double dp = pair_distance(w64, X.g.at(kW, nn), C.W.dr2(t, nn), X.inv_r2);
+      kind = dp < w64 ? 1 : 0;
+      klo = __double2float_rd(kind ? dp : w64);
+    }
+    p = fmaxf(klo, tlo);
+    if (kind) p = fmaxf(p, tn);
+    field = nn | (kind ? Ws_::kPair : 0);
+  }
+  C.W.key[t] = make_float2(klo, p);
+  C.W.nhi[t] = hi;
+  C.W.nlo[t] = lo;
+  // the field last: a reader that sees it without the target bit sees the rest
+  __threadfence_block();
+  C.W.nn[t] = (typename Ws_::Idx)field;
+}
+
+// Slot t's neighbour by the exact minimum (dR2, label) over its window (whole
+// warp), among those whose FP32 lower bound does not exceed u1.
+template <bool SM>
+__device__ __noinline__ int round_exact(int t, float u1) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const int tile = C.W.tile[t];
+  const RoundBox b = round_box(*C.S, tile, tile);
+  const float2 gt = C.W.xy[t];
+  const Bound bd = C.S->X.bd;
+  unsigned long long bk = ~0ull;
+  int bi = 0x7fffffff;
+  for_box(C, b, 32, false, [&](int u, int i) { return C.W.entry(u, i); },
+          [&](int u, float2 gu) {
+            float l, h;
+            dr2_32(gt.x, gt.y, gu.x, gu.y, bd, l, h);
+            if (u == t || !(l <= u1)) return;
+            const unsigned long long k = dbits(C.W.dr2(t, u));
+            if (arg_less(k, u, bk, bi)) {
+              bk = k;
+              bi = u;
+            }
+          });
+  return arg_warp(bk, bi, bi).idx;
+}
+
+// Stores slot t's neighbour from its group's certificate (every lane calls;
+// lane `first` of the group holds the work, have: it has some).
+template <bool SM>
+__device__ __forceinline__ void round_settle(bool have, bool first, int t, const Cert& c) {
+  const bool exact = have && first && c.i1 >= 0 && !cert_ok(c);
+  unsigned todo = __ballot_sync(kFull, exact);
+  if (have && first && !exact) round_set<SM>(t, c.i1, c.m1, c.u1);
+  __syncwarp();
+  while (todo) {
+    const int q = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int tq = __shfl_sync(kFull, t, q);
+    const int nn = round_exact<SM>(tq, __shfl_sync(kFull, c.u1, q));
+    // (an empty interval: the FP64 value is taken)
+    if ((threadIdx.x & 31) == q) round_set<SM>(tq, nn, 0.0f, __int_as_float(0x7f800000));
+    __syncwarp();
+  }
+}
+
+// Slot t's neighbour in its window, and its key (groups of G lanes).
+template <bool SM>
+__device__ __noinline__ void round_search(bool have, int t, int G, bool dense) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const int tile = have ? (int)C.W.tile[t] : 0;
+  RoundBox b = round_box(*C.S, tile, tile);
+  if (!have) b.nu = 0;
+  const float2 gt = C.W.xy[t];
+  const Bound bd = C.S->X.bd;
+  Cert x = cert_empty();
+  for_box(C, b, G, dense, [&](int u, int i) { return C.W.entry(u, i); },
+          [&](int u, float2 gu) {
+            float lo, hi;
+            dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
+            if (u != t) cert_add(x, lo, hi, u);
+          });
+  x = cert_group(x, G);
+  round_settle<SM>(have, (threadIdx.x & (G - 1)) == 0, t, x);
+}
+
+// New jet a, with FP32 distance interval [lo, hi] to slot y, may be closer to y
+// than its neighbour.  (y's neighbour field had no target bit when it was
+// read; if it has just been searched, which offered it a, nothing changes.)
+template <bool SM>
+__device__ __noinline__ void round_offer(int y, int a, float lo, float hi, int round) {
+  using Ws_ = RoundWs<SM>;
+  const RoundCtx<SM> C = round_ctx<SM>();
+  __threadfence_block();
+  if (!(hi < *(volatile float*)(C.W.nlo + y))) {
+    const int cn = *(volatile typename Ws_::Idx*)(C.W.nn + y) & Ws_::kSlotMask;
+    const double da = C.W.dr2(y, a);
+    if (cn != Ws_::kNoSlot) {
+      const double dc = C.W.dr2(y, cn);
+      if (!(da < dc || (da == dc && a < cn))) return;
+    }
+  }
+  if (round_first(C, y, round, 1))
+    round_set<SM>(y, a, lo, hi);
+  else
+    round_target(*C.S, y);  // another new jet was closer to it as well: a full search (phase E)
+}
+
+// D1 in FP64 (see the header): pseudojet x of a step with time part M and
+// threshold thr against slot y.
+template <bool SM>
+__device__ __noinline__ bool round_d1_exact(int x, int y, double thr, double M) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const EventCtx& X = C.S->X;
+  const double wx = X.g.at(kW, x), wy = X.g.at(kW, y), ty = C.W.tm[y];
+  const double d = pair_distance(wx, wy, C.W.dr2(x, y), X.inv_r2);
+  return d <= thr && d <= fmin(wx, wy) && !(ty > M);
+}
+
+// The minimum of tile t into its cell and the frame's copies of it.
+template <bool SM>
+__device__ __forceinline__ void round_store_min(const RoundCtx<SM>& C, int t, unsigned p, int slot) {
+  const RoundShared& S = *C.S;
+  const int u = t >> S.sh, v = t & ((1 << S.sh) - 1);
+  unsigned* row = C.tmin + (u + kRoundFrame) * S.pw + kRoundFrame;
+  C.slot[t] = (typename RoundCtx<SM>::Idx)slot;
+  row[v] = p;
+#pragma unroll 1
+  for (int w = v - S.nphi; w >= -kRoundFrame; w -= S.nphi) row[w] = p;
+#pragma unroll 1
+  for (int w = v + S.nphi; w < S.nphi + kRoundFrame; w += S.nphi) row[w] = p;
+}
+
+__device__ __forceinline__ bool round_before(float2 x, int sx, float2 y, int sy) {
+  return sy < 0 || x.y < y.y || (x.y == y.y && (x.x < y.x || (x.x == y.x && sx < sy)));
+}
+
+// Tile t's list compacted and its minimum (P, key, slot): a whole warp, or one
+// thread.
+template <bool SM>
+__device__ __noinline__ void round_summary_warp(int t) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  using Idx = typename RoundWs<SM>::Idx;
+  constexpr int kNone = RoundWs<SM>::kNone;
+  if ((t & ((1 << C.S->sh) - 1)) >= C.S->nphi) return;
+  const int lane = threadIdx.x & 31;
+  const int st = C.start[t], m = min(C.count[t], (int)C.start[t + 1] - st);
+  float2 best = make_float2(0.0f, 0.0f);
+  int slot = -1, out = 0;
+#pragma unroll 1
+  for (int i0 = 0; i0 < m; i0 += 32) {
+    const int i = i0 + lane;
+    const int u = i < m ? (int)C.W.members[st + i] : kNone;
+    const float2 gu = i < m ? C.W.entry(0, st + i) : make_float2(0.0f, 0.0f);
+    const unsigned ball = __ballot_sync(kFull, u != kNone);
+    if (u != kNone) {
+      const int p = out + __popc(ball & ((1u << lane) - 1));
+      if (p != i) {
+        C.W.place(st + p, u, gu);
+        C.W.at[u] = (Idx)p;
+      }
+      const float2 k = C.W.key[u];
+      if (round_before(k, u, best, slot)) {
+        best = k;
+        slot = u;
+      }
+    }
+    out += __popc(ball);
+    __syncwarp();
+  }
+  const unsigned p = slot >= 0 ? __float_as_uint(best.y) : kRoundNone;
+  const unsigned pb = __reduce_min_sync(kFull, p);
+  const unsigned k = slot >= 0 && p == pb ? __float_as_uint(best.x) : kRoundNone;
+  const unsigned kb = __reduce_min_sync(kFull, k);
+  const unsigned sb = __reduce_min_sync(kFull, slot >= 0 && p == pb && k == kb ? (unsigned)slot : kRoundNone);
+  if (lane == 0) {
+    round_store_min(C, t, pb, (int)sb);
+    C.count[t] = out;
+  }
+}
+
+template <bool SM>
+__device__ __noinline__ void round_summary_thread(int t) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  using Idx = typename RoundWs<SM>::Idx;
+  if ((t & ((1 << C.S->sh) - 1)) >= C.S->nphi) return;
+  const int st = C.start[t], m = min(C.count[t], (int)C.start[t + 1] - st);
+  float2 best = make_float2(0.0f, 0.0f);
+  int slot = -1, out = 0;
+#pragma unroll 1
+  for (int i = 0; i < m; ++i) {
+    const int u = C.W.members[st + i];
+    if (u == RoundWs<SM>::kNone) continue;
+    if (out != i) {
+      C.W.place(st + out, u, C.W.entry(0, st + i));
+      C.W.at[u] = (Idx)out;
+    }
+    ++out;
+    const float2 k = C.W.key[u];
+    if (round_before(k, u, best, slot)) {
+      best = k;
+      slot = u;
+    }
+  }
+  round_store_min(C, t, slot >= 0 ? __float_as_uint(best.y) : kRoundNone, slot);
+  C.count[t] = out;
+}
+
+// Tile lists from the live slots (whole CTA).  What the list area spares is
+// spread over the lists as room for more.
+template <bool SM>
+__device__ __noinline__ void round_lists(int n) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  RoundShared& S = *C.S;
+  using Idx = typename RoundWs<SM>::Idx;
+  constexpr int kNone = RoundWs<SM>::kNone;
+  const int N = S.X.N, T = blockDim.x, W = T / 32, nt = S.nt;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slack = (RoundWs<SM>::kRoom * N - n) / (S.nrap * S.nphi), vm = (1 << S.sh) - 1;
+  for (int t = tid; t < nt; t += T) C.count[t] = 0;
+  __syncthreads();
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    const int t = C.W.tile[s];
+    if (t != kNone) C.W.at[s] = (Idx)atomicAdd(&C.count[t], 1);
+  }
+  __syncthreads();
+  int carry = 0;
+#pragma unroll 1
+  for (int base = 0; base < nt; base += T) {
+    const int t = base + tid;
+    const int v = t < nt && (t & vm) < S.nphi ? C.count[t] + slack : 0;
+    int incl = v;
+#pragma unroll 1
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += x;
+    }
+    if (lane == 31) S.scan_tmp[warp] = incl;
+    __syncthreads();
+    int pre = 0, total = 0;
+#pragma unroll 1
+    for (int k = 0; k < W; ++k) {
+      if (k < warp) pre += S.scan_tmp[k];
+      total += S.scan_tmp[k];
+    }
+    if (t < nt) C.start[t] = (Idx)(carry + pre + incl - v);
+    carry += total;
+    __syncthreads();
+  }
+  if (tid == 0) C.start[nt] = (Idx)carry;
+  __syncthreads();
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    const int t = C.W.tile[s];
+    if (t != kNone) C.W.place(C.start[t] + C.W.at[s], s, C.W.xy[s]);
+  }
+  __syncthreads();
+}
+
+// Lane's dead node idx, taken by a step of time part m_hi (rounded up) and label
+// l, into its tile's groups (lanes with the same tile go one after another).
+// Groups are kept by descending M, so that a walk for times from some M on ends
+// at the first that is before it.  What a jet absorbs one after another has the
+// same (M, l) while its steps are chained: one group, which the jet's own
+// checks pass at once.  (One list of single nodes: 25 to 90 kcycles a round on
+// dense anti-kt events, most of it a jet walking over its own constituents.)
+template <bool SM>
+__device__ __noinline__ void round_bury(bool have, int tile, int idx, float4 g, float m_hi, int l) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const int most = 2 * C.S->X.N;
+  bool todo = have;
+  while (__any_sync(kFull, todo)) {
+    const unsigned same = __match_any_sync(kFull, todo ? tile : -1 - (int)(threadIdx.x & 31));
+    if (todo && (threadIdx.x & 31) == (unsigned)(__ffs(same) - 1)) {
+      todo = false;
+      C.W.dgeo[idx] = g;
+      int prev = -1, x = C.head[tile];
+      float xm = C.head_m[tile];
+#pragma unroll 1
+      for (int guard = 0; x >= 0 && xm > m_hi && guard < most; ++guard) {
+        const int4 r = C.W.dgrp[x];
+        prev = x;
+        x = r.x;
+        xm = __int_as_float(r.y);
+      }
+      int q = x;
+      float qm = xm;
+      bool found = false;
+#pragma unroll 1
+      for (int guard = 0; q >= 0 && qm == m_hi && !found && guard < most; ++guard) {
+        const int4 r = C.W.dgrp[q];
+        if (r.w == l) {
+          C.W.dnext[idx] = r.z;
+          C.W.dgrp[q].z = idx;
+          found = true;
+        }
+        q = r.x;
+        qm = __int_as_float(r.y);
+      }
+      if (!found) {
+        C.W.dnext[idx] = -1;
+        C.W.dgrp[idx] = make_int4(x, __float_as_int(xm), idx, l);
+        if (prev < 0) {
+          C.head[tile] = idx;
+          C.head_m[tile] = m_hi;
+        } else {
+          *reinterpret_cast<int2*>(C.W.dgrp + prev) = make_int2(idx, __float_as_int(m_hi));
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// D2 over one tile's groups for the new jet a of the step at time (M, l, depth)
+// (see the header), from its first group x on.  The dead of a's own line (label
+// l) went before it.
+template <bool SM>
+__device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const EventCtx& X = C.S->X;
+  const float m_lo = __double2float_rd(M), wa = round_wlo(C.W.wlo[a]), r2hi = C.S->r2hi, ilo = X.ilo;
+  const float2 ga = C.W.xy[a];
+  const Bound bd = X.bd;
+  bool bad = false;
+#pragma unroll 1
+  for (int guard = 0; x >= 0 && guard < 2 * X.N; ++guard) {
+    const int4 r = C.W.dgrp[x];
+    if (r.w != l) {
+      int y = r.z;
+#pragma unroll 1
+      for (int g2 = 0; y >= 0 && g2 < 2 * X.N; ++g2) {
+        const float4 dg = C.W.dgeo[y];
+        float lo, hi;
+        dr2_32(dg.x, dg.y, ga.x, ga.y, bd, lo, hi);
+        const float plo = __fmul_rd(__fmul_rd(__fmul_rd(fminf(wa, dg.z), lo), ilo), 0.99999976158142089844f);
+        if (lo <= r2hi && !(plo > dg.w)) {
+          const RoundRec q = C.W.rec[y >> 1];
+          bad |= time_less(RoundTime{M, l, depth}, RoundTime{q.M, q.l, q.depth});
+        }
+        y = C.W.dnext[y];
+      }
+    }
+    if (__int_as_float(r.y) < m_lo) break;
+    x = r.x;
+  }
+  return bad;
+}
+
+// Initial neighbours: a thread per slot, or (dense) a warp per tile -- a lane per
+// member, the window's slots gathered by the lanes and passed around.
+template <bool SM>
+__device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
+  const RoundShared& S = *C.S;
+  const int lane = threadIdx.x & 31, N = S.X.N;
+  const Bound bd = S.X.bd;
+  if (!SM && dense) {
+#pragma unroll 1
+    for (int tile = threadIdx.x >> 5; tile < S.nt; tile += blockDim.x >> 5) {
+      const int st0 = C.start[tile], m0 = C.count[tile];
+      if (!m0) continue;
+      const RoundBox b = round_box(S, tile, tile);
+      const int nb = b.nu * b.nv;
+#pragma unroll 1
+      for (int i0 = 0; i0 < m0; i0 += 32) {
+        const bool have = i0 + lane < m0;
+        const int t = C.W.members[st0 + (have ? i0 + lane : i0)];
+        const float2 gt = C.W.xy[t];
+        Cert c = cert_empty();
+#pragma unroll 1
+        for (int k = 0; k < nb; ++k) {
+          const int tt = box_tile(S, b, k);
+          const int st = C.start[tt], m = C.count[tt];
+#pragma unroll 1
+          for (int q0 = 0; q0 < m; q0 += 32) {
+            const int left = min(m - q0, 32);
+            const int iq = st + q0 + (lane < left ? lane : 0);
+            const int uq = C.W.members[iq];
+            const float2 gq = C.W.entry(uq, iq);
+#pragma unroll 4
+            for (int q = 0; q < left; ++q) {
+              const int u = __shfl_sync(kFull, uq, q);
+              float lo, hi;
+              dr2_32(gt.x, gt.y, __shfl_sync(kFull, gq.x, q), __shfl_sync(kFull, gq.y, q), bd, lo, hi);
+              if (u != t) cert_add(c, lo, hi, u);
+            }
+          }
+        }
+        round_settle<SM>(have, true, t, c);
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int s0 = threadIdx.x & ~31; s0 < N; s0 += blockDim.x) {
+    const int t = s0 + lane;
+    const bool have = t < N;
+    Cert c = cert_empty();
+    if (have) {
+      const int tile = C.W.tile[t];
+      const RoundBox b = round_box(S, tile, tile);
+      const int nb = b.nu * b.nv;
+      const float2 gt = C.W.xy[t];
+#pragma unroll 1
+      for (int k = 0; k < nb; ++k) {
+        const int tt = box_tile(S, b, k);
+        const int st = C.start[tt], m = C.count[tt];
+#pragma unroll 2
+        for (int i = 0; i < m; ++i) {
+          const int u = C.W.members[st + i];
+          const float2 gu = C.W.entry(u, st + i);
+          float lo, hi;
+          dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
+          if (u != t) cert_add(c, lo, hi, u);
+        }
+      }
+    }
+    __syncwarp();
+    round_settle<SM>(have, true, t, c);
+  }
+}
+
+__device__ __forceinline__ float plain_dr2(float2 a, float2 b) {
+  const float dr = a.x - b.x;
+  float dp = fabsf(a.y - b.y);
+  dp = fminf(dp, kTwoPiF - dp);
+  return dr * dr + dp * dp;
+}
+
+// Phase B for the steps, by groups of G lanes: D1, and the slots whose neighbour
+// is taken.  With few steps their windows are cut in parts.
+template <bool SM>
+__device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int G, bool dense, int parts) {
+  using Ws_ = RoundWs<SM>;
+  RoundShared& S = *C.S;
+  const Ws_& Wk = C.W;
+  const int lane = threadIdx.x & 31;
+  const Bound bd = S.X.bd;
+  const float ilo = S.X.ilo, r2hi = S.r2hi, far2 = r2hi * 1.001f + 1e-6f;
+#pragma unroll 1
+  for (;;) {
+    int i = 0;
+    if (lane == 0) i = atomicAdd(&S.task[0], 32 / G);
+    i = __shfl_sync(kFull, i, 0);
+    if (i >= F * parts) break;
+    const int part = i % parts;  // (several parts: G = 32)
+    i = G == 32 ? i / parts : i + lane / 8;
+    const bool have = i < F;
+    const int c = have ? S.c[i] : 0, j = have ? S.j[i] : -1, jc = j >= 0 ? j : c;
+    const float2 gc = Wk.xy[c], gj = Wk.xy[jc];
+    const float wc = round_wlo(Wk.wlo[c]), wj = round_wlo(Wk.wlo[jc]);
+    RoundBox b{0, 0, 0, 1};
+    double M = 0.0, thr_c = 0.0, thr_j = 0.0;
+    if (have) {
+      M = S.M[i];
+      thr_c = S.thr_c[i];
+      thr_j = S.thr_j[i];
+      b = round_box(S, Wk.tile[c], Wk.tile[jc]);
+    }
+    const float tc_hi = __double2float_ru(thr_c), tj_hi = __double2float_ru(thr_j);
+    struct Slot {
+      float2 g;
+      float w;
+      int nn;
+    };
+    bool bad = false;
+    const int nb = b.nu * b.nv;
+    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, dense,
+            [&](int y, int i) { return Slot{Wk.entry(y, i), Wk.wlo[y], Wk.nn[y]}; },
+            [&](int y, const Slot& s) {
+              if (y == c || y == j) return;
+              const int nn = s.nn & Ws_::kSlotMask;
+              if (nn == c || (j >= 0 && nn == j)) {
+                Wk.nn[y] = (typename Ws_::Idx)(s.nn | Ws_::kTarget);
+                round_target(S, y);
+              }
+              // beyond R of c and of j (the FP32 distance is good to 1e-5 there)?
+              if (fminf(plain_dr2(gc, s.g), plain_dr2(gj, s.g)) > far2) return;
+              const float w = round_wlo(s.w);
+#pragma unroll 1
+              for (int q = 0; q < 2; ++q) {
+                const float2 gx = q ? gj : gc;
+                float lo, hi;
+                dr2_32(gx.x, gx.y, s.g.x, s.g.y, bd, lo, hi);
+                const float plo =
+                    __fmul_rd(__fmul_rd(__fmul_rd(fminf(q ? wj : wc, w), lo), ilo), 0.99999976158142089844f);
+                if (!(lo > r2hi) && !(plo > (q ? tj_hi : tc_hi)))
+                  bad |= round_d1_exact<SM>(q ? j : c, y, q ? thr_j : thr_c, M);
+                if (j < 0) break;
+              }
+            });
+    if (bad) S.conflict[1] = 1;
+  }
+}
+
+// Phase D for one step that made jet a (groups of G lanes): the jet's window.
+template <bool SM>
+__device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, int i, int round, int G, bool dense) {
+  using Ws_ = RoundWs<SM>;
+  RoundShared& S = *C.S;
+  const Ws_& Wk = C.W;
+  const int lane = threadIdx.x & 31;
+  const Bound bd = S.X.bd;
+  const int a = have ? min(S.c[i], S.j[i]) : 0;
+  const int tile = have ? (S.new_u[i] << S.sh) + S.new_v[i] : 0;
+  RoundBox b = round_box(S, tile, tile);
+  if (!have) b.nu = 0;
+  const float2 ga = Wk.xy[a];
+  struct Slot {
+    float2 g;
+    float nhi;
+    int nn;
+  };
+  Cert ca = cert_empty();
+  for_box(C, b, G, dense, [&](int y, int i) { return Slot{Wk.entry(y, i), Wk.nhi[y], Wk.nn[y]}; },
+          [&](int y, const Slot& s) {
+            if (y == a) return;
+            float lo, hi;
+            dr2_32(s.g.x, s.g.y, ga.x, ga.y, bd, lo, hi);
+            cert_add(ca, lo, hi, y);
+            // not closer, or searched anyway?
+            if (!(lo > s.nhi) && !(s.nn & Ws_::kTarget)) round_offer<SM>(y, a, lo, hi, round);
+          });
+  ca = cert_group(ca, G);
+  round_settle<SM>(have, (lane & (G - 1)) == 0, a, ca);
+}
+
+// Records of at most 4096 slots in time order: bitonic sort in shared memory
+// (the tile arrays' room).  Labels and depths are below 4096.
+constexpr int kRoundSortMax = 4096;
+constexpr size_t kRoundSortBytes = 14;  // per record, of a power of two
+
+template <bool SM>
+__device__ __forceinline__ void round_sort_smem(const RoundCtx<SM>& C, int N, int n2,
+                                                typename RoundWs<SM>::Idx* order) {
+  const int T = blockDim.x;
+  unsigned long long* M = reinterpret_cast<unsigned long long*>(C.tmin);
+  unsigned* sec = reinterpret_cast<unsigned*>(M + n2);
+  unsigned short* id = reinterpret_cast<unsigned short*>(sec + n2);
+#pragma unroll 1
+  for (int s = threadIdx.x; s < n2; s += T) {
+    M[s] = ~0ull;
+    sec[s] = kRoundNone;
+    id[s] = (unsigned short)s;
+    if (s < N) {
+      const RoundRec r = C.W.rec[s];
+      M[s] = dbits(r.M);  // non-negative: ordered as integers
+      sec[s] = ((unsigned)r.l << 12) | (unsigned)r.depth;
+    }
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int size = 2; size <= n2; size <<= 1) {
+#pragma unroll 1
+    for (int stride = size >> 1, sh = 31 - __clz(size >> 1); stride > 0; stride >>= 1, --sh) {
+#pragma unroll 2
+      for (int k = threadIdx.x; k < n2 / 2; k += T) {
+        const int i = ((k >> sh) << (sh + 1)) + (k & (stride - 1)), j = i + stride;
+        const bool up = (i & size) == 0;
+        const unsigned long long x = M[i], y = M[j];
+        const unsigned sx = sec[i], sy = sec[j];
+        const bool gt = x > y || (x == y && sx > sy);
+        if (gt == up) {
+          M[i] = y;
+          M[j] = x;
+          sec[i] = sy;
+          sec[j] = sx;
+          const unsigned short t = id[i];
+          id[i] = id[j];
+          id[j] = t;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (int s = threadIdx.x; s < N; s += T) order[s] = id[s];
+  __syncthreads();
+}
+
+// Any number of records, in the workspace.  The first stride of a size pairs
+// mirrored entries, so that every run ascends and the missing entries past N
+// act as the largest.
+template <bool SM>
+__device__ __forceinline__ void round_sort(const RoundCtx<SM>& C, int N, int n2, typename RoundWs<SM>::Idx* order) {
+  using Idx = typename RoundWs<SM>::Idx;
+  const int T = blockDim.x;
+  for (int s = threadIdx.x; s < N; s += T) order[s] = (Idx)s;
+  __syncthreads();
+#pragma unroll 1
+  for (int size = 2; size <= n2; size <<= 1) {
+#pragma unroll 1
+    for (int stride = size >> 1, sh = 31 - __clz(size >> 1); stride > 0; stride >>= 1, --sh) {
+      const bool flip = stride == size >> 1;
+#pragma unroll 2
+      for (int k = threadIdx.x; k < n2 / 2; k += T) {
+        const int base = (k >> sh) << (sh + 1), r = k & (stride - 1);
+        const int lo = base + r, hi = flip ? base + 2 * stride - 1 - r : lo + stride;
+        if (hi < N) {
+          const Idx x = order[lo], y = order[hi];
+          const RoundRec& rx = C.W.rec[x];
+          const RoundRec& ry = C.W.rec[y];
+          if (time_less(RoundTime{ry.M, ry.l, ry.depth}, RoundTime{rx.M, rx.l, rx.depth})) {
+            order[lo] = y;
+            order[hi] = x;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Clusters event e; false: a conflict (nothing of the event's outputs was
+// written).  S.tiles, cells and slots are set; reach: the range of the choice
+// of steps, in units of R.
+template <int T, bool SM>
+__device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const BatchArgs& A, int e, float reach) {
+  constexpr int W = T / 32;
+  using Ws_ = RoundWs<SM>;
+  using Idx = typename Ws_::Idx;
+  constexpr int kNone = Ws_::kNone;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float inf = __int_as_float(0x7f800000);
+  FJG_PH(long long ph[kPhSlots - kPhRSetup] = {}; long long ph_t = clock64();
+         auto mark = [&](int slot) { const long long now = clock64(); ph[slot - kPhRSetup] += now - ph_t; ph_t = now; };)
+  int64_t off;
+  int N;
+  event_range(A, e, off, N);
+  const int algo = A.algo ? A.algo[e] : A.algo_all;
+  const double R = A.radius ? A.radius[e] : A.r_all;
+  Ws g;
+  g.base = A.ws + off;
+  g.stride = A.ws_stride;
+  if (tid == 0) {
+    S.X.N = N;
+    S.X.algo = algo;
+    S.X.inv_r2 = 1.0 / (R * R);
+    S.X.ilo = __double2float_rd(S.X.inv_r2);
+    S.X.ihi = __double2float_ru(S.X.inv_r2);
+    S.X.g = g;
+    S.ws = A.round_ws + off * kRoundBytesPerParticle;
+    S.r2hi = __double2float_ru(R * R) * 1.0001f;
+  }
+  __syncthreads();
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const Ws_& Wk = C.W;
+
+  // ---- load and kinematics
+  double rlo = 1e300, rhi = -1e300, amax = 0.0;
+  bool weightless = false;  // a pair distance of 0 at any distance (kt, no pT): left to the other kernels
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    const double* p = A.p4 + (off + s) * A.p4_stride;
+    const double px = p[0], py = p[1], pz = p[2], E = p[3];
+    const Kin kin = kinematics(px, py, pz, E, algo);
+    g.at(kPx, s) = px;
+    g.at(kPy, s) = py;
+    g.at(kPz, s) = pz;
+    g.at(kE, s) = E;
+    g.at(kW, s) = kin.w;
+    Wk.pos[s] = make_double2(kin.rap, kin.phi);
+    Wk.xy[s] = make_float2(__double2float_rn(kin.rap), __double2float_rn(kin.phi));
+    Wk.wlo[s] = round_weight(kin.w);
+    Wk.tlo[s] = 0.0f;
+    Wk.tm[s] = -1.0;
+    Wk.tl[s] = make_int2(-1, 0);
+    if (!SM) Wk.stamp[s] = make_int2(-1, -1);
+    rlo = fmin(rlo, kin.rap);
+    rhi = fmax(rhi, kin.rap);
+    amax = fmax(amax, fabs(kin.rap));
+    weightless |= !(kin.w > 0.0);
+  }
+#pragma unroll 1
+  for (int o = 16; o; o >>= 1) {
+    rlo = fmin(rlo, __shfl_xor_sync(kFull, rlo, o));
+    rhi = fmax(rhi, __shfl_xor_sync(kFull, rhi, o));
+    amax = fmax(amax, __shfl_xor_sync(kFull, amax, o));
+  }
+  if (lane == 0) {
+    S.red[0][warp] = rlo;
+    S.red[1][warp] = rhi;
+    S.red[2][warp] = amax;
+  }
+  for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
+  for (int k = tid; k < kRoundSmemMaxN / 32; k += T) S.taken[k] = S.claimed[k] = 0;
+  if (tid < 16) S.lut[tid] = tid ? (65536 + tid - 1) / tid : 0;
+  if (__syncthreads_or(weightless)) return false;
+  if (tid == 0) {
+    double lo = 1e300, hi = -1e300, rmax = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < W; ++k) {
+      lo = fmin(lo, S.red[0][k]);
+      hi = fmax(hi, S.red[1][k]);
+      rmax = fmax(rmax, S.red[2][k]);
+    }
+    S.X.bd = make_bound(rmax);
+    lo = fmax(lo, -15.0);
+    hi = fmin(hi, 15.0);
+    if (!(hi >= lo)) hi = lo;
+    // side: at least R / 2, so that the 5x5 window holds R; coarser where that
+    // would give more tiles than there is room for, or than 1.5 per particle
+    // (empty tiles only cost)
+    int cap = N + N / 2;
+    cap = cap > S.tiles ? S.tiles : cap;
+    cap = cap < 1 ? 1 : cap;
+    const double side_min = 0.5 * R * (1.0 + 1e-4) + 1e-5;
+    const double area = fmax(hi - lo, side_min) * 6.283185307179586;
+    const double side = fmax(side_min, sqrt(area / (double)cap));
+    int nphi = (int)fmin(floor(6.283185307179586 / side), 4096.0);
+    nphi = nphi < 1 ? 1 : nphi;
+    int nrap = (int)fmin(floor((hi - lo) / side), 4096.0);
+    nrap = nrap < 1 ? 1 : nrap;
+    int sh = 0;
+#pragma unroll 1
+    for (;;) {  // ends: one tile always has room
+      sh = 0;
+      while ((1 << sh) < nphi) ++sh;
+      if ((nrap << sh) <= S.tiles && nrap * nphi <= cap &&
+          (nrap + 2 * kRoundFrame) * (nphi + 2 * kRoundFrame) <= S.cells)
+        break;
+      if (nrap >= nphi)
+        nrap = nrap > 8 ? nrap - nrap / 8 : nrap - 1;
+      else
+        nphi = nphi > 8 ? nphi - nphi / 8 : nphi - 1;
+    }
+    S.nrap = nrap;
+    S.nphi = nphi;
+    S.sh = sh;
+    S.nt = nrap << sh;
+    S.pw = nphi + 2 * kRoundFrame;
+    S.rmin = lo;
+    S.inv_side_r = (double)nrap / fmax(hi - lo, side);
+    S.inv_side_phi = (double)nphi / 6.283185307179586;
+    S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
+    S.overflow = 0;
+    S.n_cand = S.n_fire = S.n_targets = S.n_dirty = 0;
+    S.task[0] = S.task[1] = 0;
+  }
+  __syncthreads();
+  FJG_PH(mark(kPhRKin);)
+  const int nt = S.nt, pw = S.pw, sh = S.sh, nphi = S.nphi;
+  for (int t = tid; t < nt; t += T) {
+    C.head[t] = -1;
+    C.head_m[t] = 0.0f;
+  }
+  for (int t = tid; t < (S.nrap + 2 * kRoundFrame) * pw; t += T) C.tmin[t] = C.row[t] = kRoundNone;
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    const double2 p = Wk.pos[s];
+    Wk.tile[s] = (Idx)((round_u(S, p.x) << sh) + round_v(S, p.y));
+  }
+  __syncthreads();
+  round_lists<SM>(N);
+
+  // ---- initial neighbours (round_set marks tiles as changed: cleared after)
+  round_init(C, N >= kRoundDense * nt);
+  __syncthreads();
+  for (int t = tid; t < nt; t += T) round_summary_thread<SM>(t);
+  for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
+  __syncthreads();
+  if (tid == 0) S.n_dirty = 0;
+  FJG_PH(mark(kPhRSetup);)
+
+  // ---- rounds
+  int n = N;
+  const float side_r = (float)(1.0 / S.inv_side_r), side_phi = (float)(1.0 / S.inv_side_phi);
+  const float range = reach * (float)R, rmin = (float)S.rmin, inv_side = 1.0f / fminf(side_r, side_phi);
+#pragma unroll 1
+  for (int round = 0; n > 0; ++round) {
+    const bool dense = !SM && n >= kRoundDense * nt;
+    // A: candidates.  Smallest P of five tiles along the row, then of five
+    // rows (empty tiles hold the largest value)
+#pragma unroll 1
+    for (int t = tid; t < nt; t += T) {
+      const int u = t >> sh, v = t & ((1 << sh) - 1);
+      if (v >= nphi) continue;
+      const int k = (u + kRoundFrame) * pw + kRoundFrame + v;
+      C.row[k] = min(min(min(C.tmin[k - 2], C.tmin[k - 1]), min(C.tmin[k + 1], C.tmin[k + 2])), C.tmin[k]);
+    }
+    if (!SM)
+      for (int k = tid; k < (S.nrap + 2 * kRoundFrame) * pw; k += T) C.near[k] = C.tmin[k];
+    __syncthreads();
+#pragma unroll 1
+    for (int t = tid; t < nt; t += T) {
+      const int u = t >> sh, v = t & ((1 << sh) - 1);
+      if (v >= nphi) continue;
+      const int k = (u + kRoundFrame) * pw + kRoundFrame + v;
+      const unsigned me = C.tmin[k];
+      if (me == kRoundNone) continue;
+      if (!SM) {
+        // a step also counts where its partner is: a hard jet's own key may
+        // belong to a later step (its neighbour is younger) while an earlier
+        // one takes it from the far side of its reach
+        const int f = Wk.nn[C.slot[t]];
+        const int tj = f & Ws_::kPair ? (int)Wk.tile[f & Ws_::kSlotMask] : t;
+        if (tj != t) {
+          const int vj = tj & ((1 << sh) - 1);
+          unsigned* cell = C.near + ((tj >> sh) + kRoundFrame) * pw + kRoundFrame;
+          for (int w = vj % nphi - (kRoundFrame / nphi + 1) * nphi; w < nphi + kRoundFrame; w += nphi)
+            if (w >= -kRoundFrame) atomicMin(cell + w, me);
+        }
+      }
+      if (me == min(min(min(C.row[k - 2 * pw], C.row[k - pw]), min(C.row[k + pw], C.row[k + 2 * pw])), C.row[k])) {
+        const int q = atomicAdd(&S.n_cand, 1);
+        if (q < kRoundMaxCand) S.cand[q] = (unsigned short)t;
+      }
+    }
+    if (SM)
+      for (int k = tid; k < (N + 31) / 32; k += T) S.taken[k] = S.claimed[k] = 0;
+    __syncthreads();
+    FJG_PH(mark(kPhRCand);)
+    const int nc = min(S.n_cand, kRoundMaxCand);
+    // range test, eight lanes per candidate, and the keys, times and thresholds
+    // of the steps that pass
+#pragma unroll 1
+    for (int k0 = 4 * warp; k0 < nc; k0 += 4 * W) {
+      const int k = k0 + lane / 8;
+      const int t = k < nc ? S.cand[k] : S.cand[k0];
+      const int u = t >> sh, v = t & ((1 << sh) - 1);
+      const int cell = (u + kRoundFrame) * pw + kRoundFrame + v;
+      const unsigned me = C.tmin[cell];
+      int c = C.slot[t];
+      const int fc = Wk.nn[c];
+      int j = fc & Ws_::kPair ? fc & Ws_::kSlotMask : -1;
+      const float2 gc = Wk.xy[c];
+      const float ckey = Wk.key[c].x;
+      // distance within which an earlier step could matter: to c, or to its
+      // partner as far from c as that is
+      const float beside = j >= 0 ? sqrtf(Wk.nhi[c]) : 0.0f, lim = range + beside;
+      float near2 = lim * lim;
+      if (algo != -1) {
+        float w = round_wlo(Wk.wlo[c]);
+        if (j >= 0) w = fminf(w, round_wlo(Wk.wlo[j]));
+        const float l = range * sqrtf(fminf(1.0f, __uint_as_float(me) / (0.7f * w))) + beside;
+        near2 = l * l;
+      }
+      const float fu = (gc.x - rmin) - u * side_r, fv = gc.y - v * side_phi;  // within its tile
+      const float lim2 = lim * lim;
+      const int far = min((int)(lim * inv_side) + 1, kRoundFrame), side = 2 * far + 1, lut = S.lut[side];
+      bool blocked = false;
+#pragma unroll 1
+      for (int i = lane & 7; i < side * side; i += 8) {
+        const int row = (i * lut) >> 16, du = row - far, dv = i - side * row - far;
+        const unsigned o = C.near[cell + du * pw + dv];
+        if (o > me) continue;
+        const float dr = du > 0 ? du * side_r - fu : du < 0 ? fu - (du + 1) * side_r : 0.0f;
+        const float dp = dv > 0 ? dv * side_phi - fv : dv < 0 ? fv - (dv + 1) * side_phi : 0.0f;
+        const float d2 = dr * dr + dp * dp;
+        if (d2 > lim2) continue;
+        int ov = v + dv;
+        ov = ov < 0 ? ov + nphi : ov >= nphi ? ov - nphi : ov;
+        if (d2 > near2) {  // (kt, C/A) near enough for the other one's weight?
+          if (o == me || ov < 0 || ov >= nphi) continue;
+          const int so = C.slot[((u + du) << sh) + ov];
+          if (so == kNone) continue;  // (a step counted at its partner)
+          const float l = range * sqrtf(fminf(1.0f, __uint_as_float(me) / (0.7f * round_wlo(Wk.wlo[so])))) + beside;
+          blocked |= d2 <= l * l;
+        } else if (o < me) {
+          blocked = true;
+        } else if (SM || o == C.tmin[cell + du * pw + dv]) {  // equal P: the smaller key goes first
+          if (ov >= 0 && ov < nphi) blocked |= Wk.key[C.slot[((u + du) << sh) + ov]].x < ckey;
+        }
+      }
+      const unsigned ball = __ballot_sync(kFull, blocked);
+      if (k < nc && (lane & 7) == 0 && !((ball >> (lane & 24)) & 0xffu)) {
+        // two steps never share a slot: the lower slot is claimed first, so of
+        // several that want the same ones, one gets both of its own
+        const int jc = j >= 0 ? j : c;
+        bool ok = round_first(C, min(c, jc), round, 0);
+        if (ok && j >= 0) ok = round_first(C, max(c, j), round, 0);
+        const int i = ok ? atomicAdd(&S.n_fire, 1) : kRoundSteps;
+        if (i < kRoundSteps) {
+          const int fj = Wk.nn[jc];
+          const bool mutual = j >= 0 && (fj & Ws_::kPair) && (fj & Ws_::kSlotMask) == c;
+          const double wc = g.at(kW, c), wj = g.at(kW, jc);
+          const double mc = Wk.tm[c], mj = Wk.tm[jc];
+          const int2 lc = Wk.tl[c], lj = Wk.tl[jc];
+          double key = wc;
+          RoundTime tc{mc, lc.x, lc.y}, tj{-2.0, -1, 0};
+          if (j >= 0) {
+            key = pair_distance(wc, wj, Wk.dr2(c, j), S.X.inv_r2);
+            tj = RoundTime{mj, lj.x, lj.y};
+            if (wj <= key && wj < wc) {
+              // a partner at R, up to FP32: its promotion goes first
+              c = j;
+              j = -1;
+              key = wj;
+              tc = tj;
+              tj = RoundTime{-2.0, -1, 0};
+            }
+          }
+          const bool from_j = time_less(tc, tj);
+          const RoundTime tp = from_j ? tj : tc;
+          RoundTime te{key, mutual && j >= 0 ? min(c, j) : c, 0};
+          const bool chained = te.M < tp.M || (te.M == tp.M && te.l <= tp.l);
+          if (chained) te = RoundTime{tp.M, tp.l, tp.depth + 1};
+          const double thr_c = chained && !from_j ? key : te.M;
+          const double thr_j = chained && from_j ? key : te.M;
+          // the promotions of c and j come later
+          if (j >= 0 && (wc <= thr_c || wj <= thr_j)) S.conflict[0] = 1;
+          S.c[i] = c;
+          S.j[i] = j;
+          S.key[i] = key;
+          S.M[i] = te.M;
+          S.l[i] = te.l;
+          S.depth[i] = te.depth;
+          S.thr_c[i] = thr_c;
+          S.thr_j[i] = thr_j;
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+    const int F = min(S.n_fire, kRoundSteps);
+    if (!F || S.conflict[0]) {  // (F = 0: cannot happen)
+      if (tid == 0) S.conflict[1] = 1;
+      break;
+    }
+    FJG_PH(mark(kPhRRange); ++ph[kPhRRounds - kPhRSetup]; ph[kPhRSteps - kPhRSetup] += F; ph[kPhRCands - kPhRSetup] += nc;)
+    // lanes per step: few steps, a warp each
+    const int G = SM && F > W ? 8 : 32;
+
+    // B: kinematics of the new jets, a lane per step
+#pragma unroll 1
+    for (int role = warp; role < 3; role += W) {
+      FJG_PH(const long long q0 = clock64();)
+      const int i = lane;
+      const bool have = i < F;
+      const int c = have ? S.c[i] : 0, j = have ? S.j[i] : -1;
+      if (role == 2) {
+        // weight, record, and the dead of the step
+        int tile_c = 0, tile_j = 0, b = 0;
+        float4 dc{}, dj{};
+        float m_hi = 0.0f;
+        if (have) {
+          b = max(c, j);
+          m_hi = __double2float_ru(S.M[i]);
+          const float2 gc = Wk.xy[c];
+          dc = make_float4(gc.x, gc.y, round_wlo(Wk.wlo[c]), __double2float_ru(S.thr_c[i]));
+          const int2 tpc = make_int2(Wk.tile[c], Wk.at[c]);
+          tile_c = tpc.x;
+          S.tp_b[i] = tpc;
+          if (j >= 0) {
+            const float2 gj = Wk.xy[j];
+            dj = make_float4(gj.x, gj.y, round_wlo(Wk.wlo[j]), __double2float_ru(S.thr_j[i]));
+            const int2 tpj = make_int2(Wk.tile[j], Wk.at[j]);
+            tile_j = tpj.x;
+            S.tp_b[i] = c > j ? tpc : tpj;
+            S.tp_a[i] = c > j ? tpj : tpc;
+            const double w =
+                fjk_weight(__dadd_rn(g.at(kPx, c), g.at(kPx, j)), __dadd_rn(g.at(kPy, c), g.at(kPy, j)), algo);
+            S.w[i] = w;
+            if (!(w > 0.0)) S.conflict[1] = 1;
+          }
+          RoundRec r;
+          r.M = S.M[i];
+          r.d = S.key[i];
+          r.l = S.l[i];
+          r.depth = S.depth[i];
+          r.a = j >= 0 ? min(c, j) : -1;
+          r.pad = 0;
+          Wk.rec[b] = r;
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int q = 0; q < 2; ++q)
+          round_bury<SM>(have && (!q || j >= 0), q ? tile_j : tile_c, 2 * b + q, q ? dj : dc, m_hi,
+                         have ? S.l[i] : 0);
+      } else if (have && j >= 0) {
+        const double px = __dadd_rn(g.at(kPx, c), g.at(kPx, j)), py = __dadd_rn(g.at(kPy, c), g.at(kPy, j));
+        if (role == 0) {
+          const double phi = fjk_phi(px, py);
+          S.phi[i] = phi;
+          S.new_v[i] = round_v(S, phi);
+        } else {
+          const double pz = __dadd_rn(g.at(kPz, c), g.at(kPz, j)), E = __dadd_rn(g.at(kE, c), g.at(kE, j));
+          const double rap = fjk_rap(px, py, pz, E);
+          S.p4[0][i] = px;
+          S.p4[1][i] = py;
+          S.p4[2][i] = pz;
+          S.p4[3][i] = E;
+          S.rap[i] = rap;
+          S.new_u[i] = round_u(S, rap);
+        }
+      }
+      __syncwarp();
+      FJG_PH(if (lane == 0 && A.phase) atomicAdd(A.phase + kPhRRole0 + role, (unsigned long long)(clock64() - q0));)
+    }
+    // D1 and the targets
+    FJG_PH(const long long qb = clock64();)
+    round_phase_b(C, F, G, dense, G == 32 ? max(1, (W - 3) / F) : 1);
+    FJG_PH(if (tid == T - 32 && A.phase) atomicAdd(A.phase + kPhRScan, (unsigned long long)(clock64() - qb));)
+    __syncthreads();
+    FJG_PH(mark(kPhRB);)
+
+    // C: the new state, a lane per step
+    if (warp == 0) {
+      if (lane < F) {
+        const int i = lane;
+        const int c = S.c[i], j = S.j[i];
+        const int b = max(c, j);
+        const int2 tb = S.tp_b[i];
+        Wk.members[C.start[tb.x] + tb.y] = (Idx)kNone;
+        Wk.tile[b] = (Idx)kNone;
+        round_dirty(S, tb.x);
+        if (j >= 0) {
+          const int a = min(c, j);
+          const int2 ta = S.tp_a[i];
+          const int t = (S.new_u[i] << sh) + S.new_v[i];
+          if (ta.x != tb.x) round_dirty(S, ta.x);
+          if (t != ta.x) {
+            Wk.members[C.start[ta.x] + ta.y] = (Idx)kNone;
+            const int p = atomicAdd(&C.count[t], 1);
+            if (C.start[t] + p < C.start[t + 1])
+              Wk.place(C.start[t] + p, a, make_float2(__double2float_rn(S.rap[i]), __double2float_rn(S.phi[i])));
+            else
+              S.overflow = 1;
+            Wk.tile[a] = (Idx)t;
+            Wk.at[a] = (Idx)p;
+          } else if (!SM) {
+            Wk.place(C.start[t] + ta.y, a, make_float2(__double2float_rn(S.rap[i]), __double2float_rn(S.phi[i])));
+          }
+        }
+      }
+      if (lane == 0) {
+        S.n_cand = 0;
+        S.task[0] = 0;
+      }
+    } else if (warp == 1) {
+      if (lane < F && S.j[lane] >= 0) {
+        const int i = lane;
+        const int a = min(S.c[i], S.j[i]);
+        const double rap = S.rap[i], phi = S.phi[i], w = S.w[i];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) g.at(kPx + q, a) = S.p4[q][i];
+        g.at(kW, a) = w;
+        Wk.pos[a] = make_double2(rap, phi);
+        Wk.xy[a] = make_float2(__double2float_rn(rap), __double2float_rn(phi));
+        Wk.nhi[a] = inf;
+        Wk.wlo[a] = round_weight(w);
+        Wk.tlo[a] = fmaxf(__double2float_rd(S.M[i]), 0.0f);
+        Wk.tm[a] = S.M[i];
+        Wk.tl[a] = make_int2(S.l[i], S.depth[i]);
+        Wk.nn[a] = (Idx)(Ws_::kNoSlot | Ws_::kTarget);  // its own group searches its neighbour
+      }
+    }
+    __syncthreads();
+    if (S.conflict[1]) break;
+    n -= F;
+    if (S.overflow) {  // a list is full: all lists again
+      round_lists<SM>(n);
+      if (tid == 0) S.overflow = 0;
+      FJG_PH(++ph[kPhROverflows - kPhRSetup];)
+    }
+    FJG_PH(mark(kPhRC);)
+
+    // D and E: each new jet against its window; the targets' searches (one may
+    // have been taken by another step, or be a new jet); the dead of each new
+    // jet's window (D2).  A warp takes 32 / G of a kind at a time.
+    const int ntg = min(S.n_targets, kRoundMaxTargets);
+    __syncthreads();  // D adds targets
+    const int per = 32 / G, uf = (F + per - 1) / per, ut = (ntg + per - 1) / per;
+#pragma unroll 1
+    for (;;) {
+      int u = 0;
+      if (lane == 0) u = atomicAdd(&S.task[1], 1);
+      u = __shfl_sync(kFull, u, 0);
+      if (u >= 2 * uf + ut) break;
+      FJG_PH(const long long qd = clock64();)
+      const int q = G == 32 ? 0 : lane / 8;
+      if (u < uf) {
+        const int i = per * u + q;
+        round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, round, G, dense);
+      } else if (u < uf + ut) {
+        const int k = per * (u - uf) + q;
+        const int t = S.targets[k < ntg ? k : 0];
+        const bool live = k < ntg && (int)Wk.tile[t] != kNone &&
+                          (Wk.nn[t] & (Ws_::kSlotMask | Ws_::kTarget)) != (Ws_::kNoSlot | Ws_::kTarget);
+        round_search<SM>(live, t, G, dense);
+      } else {
+        const int i = per * (u - uf - ut) + q;
+        if (i < F && S.j[i] >= 0) {
+          const double M = S.M[i];
+          const float m_lo = __double2float_rd(M);
+          const int tile = (S.new_u[i] << sh) + S.new_v[i];
+          const RoundBox b = round_box(S, tile, tile);
+          const int nb = b.nu * b.nv;
+          bool bad = false;
+#pragma unroll 1
+          for (int k = lane & (G - 1); k < nb; k += G) {
+            const int t = box_tile(S, b, k);
+            const int x = C.head[t];
+            if (x >= 0 && C.head_m[t] >= m_lo) bad |= round_d2<SM>(x, min(S.c[i], S.j[i]), M, S.l[i], S.depth[i]);
+          }
+          if (bad) S.conflict[2] = 1;
+        }
+        __syncwarp();
+      }
+      FJG_PH(if (lane == 0 && A.phase) atomicAdd(A.phase + (u < uf ? kPhRNewJet : u < uf + ut ? kPhRSearch : kPhRDead), (unsigned long long)(clock64() - qd));)
+    }
+    __syncthreads();
+    const int ntg2 = S.n_targets;
+    FJG_PH(mark(kPhRD); ph[kPhRTargets - kPhRSetup] += ntg2;)
+    // (more targets than listed: only degenerate inputs)
+    if (S.conflict[2] || ntg2 > kRoundMaxTargets) {
+      if (tid == 0) S.conflict[0] = 1;
+      break;
+    }
+    if (ntg2 > ntg) {  // slots that two new jets wanted
+#pragma unroll 1
+      for (int k = ntg + warp; k < ntg2; k += W) round_search<SM>(true, S.targets[k], 32, dense);
+      __syncthreads();
+    }
+    FJG_PH(mark(kPhRE);)
+
+    // F: changed tiles
+    const int nd = S.n_dirty, ndt = nd <= kRoundMaxDirty ? nd : nt;
+    if (dense) {
+#pragma unroll 1
+      for (int k = warp; k < ndt; k += W) round_summary_warp<SM>(nd <= kRoundMaxDirty ? S.dirty[k] : k);
+    } else {
+#pragma unroll 1
+      for (int k = tid; k < ndt; k += T) round_summary_thread<SM>(nd <= kRoundMaxDirty ? S.dirty[k] : k);
+    }
+    for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
+    __syncthreads();
+    FJG_PH(mark(kPhRF);)
+    if (tid == 0) {
+      S.n_dirty = S.n_targets = S.n_fire = 0;
+      S.task[1] = 0;
+    }
+    // (the next writers of these follow the next barriers)
+  }
+  __syncthreads();
+  if (S.conflict[0] | S.conflict[1] | S.conflict[2]) {
+    FJG_PH(if (A.phase && tid == 0) {
+      atomicAdd(A.phase + kPhRRetries, 1ull);
+      for (int k = 0; k < 3; ++k) atomicAdd(A.phase + kPhRConflictA + k, (unsigned long long)(S.conflict[k] != 0));
+    })
+    return false;
+  }
+
+  // ---- records in sequential order
+  Idx* order = Wk.members;
+  int n2 = 1;
+  while (n2 < N) n2 <<= 1;
+  if (n2 <= kRoundSortMax &&
+      n2 * kRoundSortBytes <= (SM ? round_tile_bytes_sm(S.tiles, S.cells) : round_tile_bytes(S.tiles, S.cells)))
+    round_sort_smem<SM>(C, N, n2, order);
+  else
+    round_sort<SM>(C, N, n2, order);
+  FJG_PH(mark(kPhRSort);)
+  // ---- outputs
+  int* parent = Wk.dnext;  // [N] of 2N
+  int jets = 0;
+#pragma unroll 1
+  for (int base = 0; base < N; base += T) {
+    const int r = base + tid;
+    const int s = r < N ? (int)order[r] : -1;
+    RoundRec rec{};
+    if (s >= 0) rec = Wk.rec[s];
+    const bool jet = s >= 0 && rec.a < 0;
+    const unsigned ball = __ballot_sync(kFull, jet);
+    if (lane == 0) S.scan_tmp[warp] = __popc(ball);
+    __syncthreads();
+    int pre = 0, total = 0;
+    for (int k = 0; k < W; ++k) {
+      if (k < warp) pre += S.scan_tmp[k];
+      total += S.scan_tmp[k];
+    }
+    if (s >= 0) {
+      if (A.history) A.history[off + r] = jet ? StepRec{s, -1, rec.d} : StepRec{rec.a, s, rec.d};
+      int par = rec.a;
+      if (jet) {
+        const int k = jets + pre + __popc(ball & ((1u << lane) - 1));
+        double* jo = A.jets + (off + k) * 4;
+        jo[0] = g.at(kPx, s);
+        jo[1] = g.at(kPy, s);
+        jo[2] = g.at(kPz, s);
+        jo[3] = g.at(kE, s);
+        A.jet_label[off + k] = s;
+        par = -(k + 1);
+      }
+      parent[s] = par;
+    }
+    jets += total;
+    __syncthreads();
+  }
+  if (tid == 0) A.n_jets[e] = jets;
+  if (A.owner) {
+#pragma unroll 1
+    for (int s = tid; s < N; s += T) {
+      int v = parent[s];
+#pragma unroll 1
+      for (int guard = 0; v >= 0 && guard < N; ++guard) v = parent[v];
+      A.owner[off + s] = v < 0 ? -v - 1 : -1;
+    }
+  }
+  __syncthreads();
+  FJG_PH(mark(kPhROut); ph[kPhREvents - kPhRSetup] = 1;
+         if (A.phase && tid == 0) for (int k = kPhRSetup; k < kPhSlots; ++k)
+           atomicAdd(A.phase + k, (unsigned long long)ph[k - kPhRSetup]);)
+  return true;
+}
+
+}  // namespace fjg

@@ -41,12 +41,14 @@ struct DeviceBuffer {
 // FP64 workspace and the tiled kernel's workspace, with their buffers.
 struct ScratchSet {
   Scratch sc{};
-  DeviceBuffer lists, ws, large;
+  DeviceBuffer lists, ws, large, rounds;
   cudaError_t reserve_lists(int n_events);         // order/counts/queues/status/hist (+ offsets1)
   cudaError_t reserve_ws(int64_t particles);       // kWsFields doubles per particle
   cudaError_t reserve_large(int64_t particles);    // only when particles > kSmemMaxN
+  void reserve_rounds(int64_t particles);          // without it (no memory) the step-by-step kernels run
   void release() {
     lists.release();
+    rounds.release();
     ws.release();
     large.release();
     sc = Scratch{};
@@ -74,9 +76,9 @@ struct fjg_ctx {
   int device = 0;
   int num_sms = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side[fjg::kNumQueues] = {};
+  cudaStream_t side[fjg::kNumSide] = {};
   cudaEvent_t ev_fork = nullptr;
-  cudaEvent_t ev_join[fjg::kNumQueues] = {};
+  cudaEvent_t ev_join[fjg::kNumSide] = {};
   fjg::ScratchSet scratch;  // the context's own launches
   fjg::DeviceBuffer io;     // device copies for the host-memory entry points
   fjg::DeviceBuffer single; // outputs of fjg_cluster_pseudojets

@@ -16,6 +16,10 @@ __global__ void __launch_bounds__(kTiledT, 1) k_cluster_tiled(BatchArgs A) {
     __syncthreads();
     const int e = S.event;
     if (e < 0) break;
+    if (rounds_event(A, e)) {
+      __syncthreads();  // everyone has read S.event
+      continue;
+    }
     if (refused_event(A, e)) continue;  // ends with a barrier
     cluster_event_tiled(S, A, A.large_ws, e);  // ends with a barrier
     if (threadIdx.x == 0) signal_done(A, e);
@@ -295,8 +299,8 @@ static int check_grid() {
 static cudaError_t launch_sort(const BatchArgs& base, const Scratch& sc, int n_events, cudaStream_t stream) {
   cudaError_t err;
   if ((err = cudaMemsetAsync(sc.hist, 0, sizeof(int32_t) * kHistBins, stream)) != cudaSuccess) return err;
-  if ((err = cudaMemsetAsync(sc.queues, 0, sizeof(int) * kNumQueues, stream)) != cudaSuccess) return err;
-  if ((err = cudaMemsetAsync(sc.counts + kLargeQueue, 0, sizeof(int32_t), stream)) != cudaSuccess) return err;
+  if ((err = cudaMemsetAsync(sc.queues, 0, sizeof(int) * (sc.round_ws ? kNumLists + kNumQueues : kNumQueues), stream)) != cudaSuccess) return err;
+  if ((err = cudaMemsetAsync(sc.counts + kLargeQueue, 0, sizeof(int32_t) * (sc.round_ws ? 3 : 1), stream)) != cudaSuccess) return err;
   const int grid = (n_events + 255) / 256 < 1 ? 1 : ((n_events + 255) / 256 > 1024 ? 1024 : (n_events + 255) / 256);
   const int64_t limit = base.particles < sc.ws_stride ? base.particles : sc.ws_stride;
   k_check_args<<<grid, 256, 0, stream>>>(base.offsets, n_events, base.n_jets, limit, base.algo, base.radius);
@@ -388,96 +392,144 @@ static int bucket_grid(const Tuning& tune, int b, int num_sms, int n_events) {
   return grid < 1 ? 1 : grid;
 }
 
-cudaError_t launch_batch(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
+// Whether the rounds kernel takes some, and all, of list q's events, as far as
+// the host knows (per-event algorithms and radii are the device's).
+static void rounds_share(const BatchArgs& A, int q, bool* some, bool* all) {
+  *some = A.rounds_mode != kRoundsNone;
+  *all = false;
+  if (!*some || A.algo || A.radius) return;
+  const int lo = q == 0 ? 1 : (128 << q) + 1, hi = q == kLargeQueue ? kLargeMaxN : 256 << q;
+  const bool at_lo = rounds_take(A.rounds_mode, lo, A.algo_all, A.r_all);
+  const bool at_hi = rounds_take(A.rounds_mode, hi, A.algo_all, A.r_all);
+  *some = at_lo || at_hi;  // the rule changes at most once inside a list's range
+  *all = at_lo && at_hi;
+}
+
+// List q (a bucket, or kLargeQueue) of a batch: the rounds kernel for its
+// events, or the step-by-step kernel for the others.
+static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, int n_events, int num_sms,
+                               const Tuning& tune, bool rounds, cudaStream_t s) {
+  BatchArgs A = base;
+  A.order = sc.order + q * sc.cap_events;
+  A.n_order = sc.counts + q;
+  A.queue = sc.queues + q;
+  A.ws = sc.ws;
+  A.ws_stride = sc.ws_stride;
+  if (rounds) {
+    const int r = q == kLargeQueue ? kRetryLargeQueue : kRetryQueue;
+    A.queue = sc.queues + kNumLists + q;
+    A.round_ws = sc.round_ws;
+    A.retry = sc.order + r * sc.cap_events;
+    A.n_retry = sc.counts + r;
+    const int grid = num_sms * rounds_occupancy(q);
+    return launch_rounds(q, A, grid > n_events ? n_events : grid, s);
+  }
+  if (q == kLargeQueue) return launch_large(base, sc, n_events, num_sms, tune, s);
+  return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
+}
+
+// The events the rounds kernels left: almost always none, then both launches
+// end at once.
+static cudaError_t launch_retries(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms,
+                                  cudaStream_t s) {
+  if (base.rounds_mode == kRoundsNone) return cudaSuccess;
+  BatchArgs A = base;
+  A.rounds_mode = kRoundsNone;
+  A.order = sc.order + kRetryQueue * sc.cap_events;
+  A.n_order = sc.counts + kRetryQueue;
+  A.queue = sc.queues + kRetryQueue;
+  A.ws = sc.ws;
+  A.ws_stride = sc.ws_stride;
+  const int grid = n_events < num_sms ? n_events : num_sms;
+  cudaError_t err = launch_variant(kRetryVariant, A, grid, 1, s);
+  if (err != cudaSuccess || !sc.large_ws) return err;
+  A.order = sc.order + kRetryLargeQueue * sc.cap_events;
+  A.n_order = sc.counts + kRetryLargeQueue;
+  A.queue = sc.queues + kRetryLargeQueue;
+  A.large_ws = sc.large_ws;
+  A.tile_factor = 1.0;
+  return launch_tiled(A, grid, s);
+}
+
+// Few events: each has an SM (two CTAs of the rounds kernel) to itself.
+static int rounds_mode_of(const Scratch& sc, int n_events, int num_sms) {
+  return !sc.round_ws ? kRoundsNone : n_events <= 2 * num_sms ? kRoundsFew : kRoundsMany;
+}
+
+cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
                          cudaStream_t stream, cudaStream_t* side, cudaEvent_t* ev_fork, cudaEvent_t* ev_join) {
+  BatchArgs base = args;
+  base.rounds_mode = rounds_mode_of(sc, n_events, num_sms);
   cudaError_t err = launch_sort(base, sc, n_events, stream);
   if (err != cudaSuccess) return err;
   if ((err = cudaEventRecord(*ev_fork, stream)) != cudaSuccess) return err;
-  // largest events first: their list is launched first
-  {
-    cudaStream_t s = side ? side[kLargeQueue] : stream;
-    if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) return err;
-    if ((err = launch_large(base, sc, n_events, num_sms, tune, s)) != cudaSuccess) return err;
-    if (side) {
-      if ((err = cudaEventRecord(ev_join[kLargeQueue], s)) != cudaSuccess) return err;
-      if ((err = cudaStreamWaitEvent(stream, ev_join[kLargeQueue], 0)) != cudaSuccess) return err;
+  // largest events first: their list is launched first.  A list that both
+  // kernels work on has them side by side (the rounds kernel's streams come
+  // first).
+  for (int q = kLargeQueue; q >= 0; --q) {
+    if (q == kLargeQueue && !sc.large_ws) continue;
+    bool some, all;
+    rounds_share(base, q, &some, &all);
+    for (int k = 0; k < 2; ++k) {
+      if (k == 0 ? !some : all) continue;
+      const int i = q + (k ? kNumQueues : 0);
+      cudaStream_t s = side ? side[i] : stream;
+      if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) return err;
+      if ((err = launch_list(base, sc, q, n_events, num_sms, tune, k == 0, s)) != cudaSuccess) return err;
+      if (side) {
+        if ((err = cudaEventRecord(ev_join[i], s)) != cudaSuccess) return err;
+        if ((err = cudaStreamWaitEvent(stream, ev_join[i], 0)) != cudaSuccess) return err;
+      }
     }
   }
-  for (int b = kNumBuckets - 1; b >= 0; --b) {
-    cudaStream_t s = side ? side[b] : stream;
-    if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) return err;
-    BatchArgs A = base;
-    A.order = sc.order + b * sc.cap_events;
-    A.n_order = sc.counts + b;
-    A.queue = sc.queues + b;
-    A.ws = sc.ws;
-    A.ws_stride = sc.ws_stride;
-    if ((err = launch_variant(tune.bucket[b].variant, A, bucket_grid(tune, b, num_sms, n_events),
-                              bucket_per_sm(tune, b), s)) != cudaSuccess)
-      return err;
-    if (side) {
-      if ((err = cudaEventRecord(ev_join[b], s)) != cudaSuccess) return err;
-      if ((err = cudaStreamWaitEvent(stream, ev_join[b], 0)) != cudaSuccess) return err;
-    }
-  }
-  return cudaSuccess;
+  return launch_retries(base, sc, n_events, num_sms, stream);
 }
 
-cudaError_t launch_batch_on_stream(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms,
+cudaError_t launch_batch_on_stream(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms,
                                    const Tuning& tune, cudaStream_t stream) {
+  BatchArgs base = args;
+  base.rounds_mode = rounds_mode_of(sc, n_events, num_sms);
   cudaError_t err = launch_sort(base, sc, n_events, stream);
   if (err != cudaSuccess) return err;
-  if ((err = launch_large(base, sc, n_events, num_sms, tune, stream)) != cudaSuccess) return err;
-  for (int b = kNumBuckets - 1; b >= 0; --b) {
-    BatchArgs A = base;
-    A.order = sc.order + b * sc.cap_events;
-    A.n_order = sc.counts + b;
-    A.queue = sc.queues + b;
-    A.ws = sc.ws;
-    A.ws_stride = sc.ws_stride;
-    if ((err = launch_variant(tune.bucket[b].variant, A, bucket_grid(tune, b, num_sms, n_events),
-                              bucket_per_sm(tune, b), stream)) != cudaSuccess)
-      return err;
+  for (int q = kLargeQueue; q >= 0; --q) {
+    if (q == kLargeQueue && !sc.large_ws) continue;
+    bool some, all;
+    rounds_share(base, q, &some, &all);
+    if (some && (err = launch_list(base, sc, q, n_events, num_sms, tune, true, stream)) != cudaSuccess) return err;
+    if (!all && (err = launch_list(base, sc, q, n_events, num_sms, tune, false, stream)) != cudaSuccess) return err;
   }
-  return cudaSuccess;
+  return launch_retries(base, sc, n_events, num_sms, stream);
 }
 
-// The single-event path's input check: an event with a non-finite momentum
-// empties every work list (nothing runs) and raises kStatusBadArg.
-__global__ void k_check_single(const double* p4, int p4_stride, int n, int32_t* counts, int32_t* n_jets,
-                               int* status) {
-  __shared__ int any_bad;
-  if (threadIdx.x == 0) any_bad = 0;
-  __syncthreads();
+// The single-event path's descriptors and input check in one launch: an event
+// with a non-finite momentum empties every work list (nothing runs) and raises
+// kStatusBadArg.
+__global__ void k_single_setup(const double* p4, int p4_stride, int n, int64_t* offsets1, int32_t* order,
+                               int32_t* counts, int* queues, int32_t* n_jets, int* status) {
   bool bad = false;
   for (int s = threadIdx.x; s < n; s += blockDim.x) {
     const double* p = p4 + (int64_t)s * p4_stride;
     bad |= !(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]) && isfinite(p[3]));
   }
-  if (bad) any_bad = 1;
-  __syncthreads();
-  if (threadIdx.x == 0 && any_bad) {
-    for (int b = 0; b < kNumQueues; ++b) counts[b] = 0;
-    n_jets[0] = 0;
-    atomicOr(status, kStatusBadArg);
-  }
-}
-
-__global__ void k_single_setup(int64_t* offsets1, int32_t* order, int32_t* counts, int* queues, int n) {
-  offsets1[0] = 0;
-  offsets1[1] = n;
-  order[0] = 0;
-  for (int b = 0; b < kNumQueues; ++b) {
-    counts[b] = 1;
-    queues[b] = 0;
+  const int any_bad = __syncthreads_or(bad);
+  const int t = threadIdx.x;
+  if (t < kNumLists) counts[t] = t < kNumQueues && !any_bad ? 1 : 0;
+  if (t < kNumLists + kNumQueues) queues[t] = 0;
+  if (t < 2) offsets1[t] = t ? n : 0;
+  if (t == 0) {
+    order[0] = 0;
+    if (any_bad) {
+      n_jets[0] = 0;
+      atomicOr(status, kStatusBadArg);
+    }
   }
 }
 
 cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const Tuning& tune, cudaStream_t stream) {
   const int b = bucket_of(n);
   if (b < 0 && (!sc.large_ws || n > sc.large_ws_particles || n > kLargeMaxN)) return cudaErrorInvalidValue;
-  k_single_setup<<<1, 1, 0, stream>>>(sc.offsets1, sc.order, sc.counts, sc.queues, n);
-  k_check_single<<<1, 256, 0, stream>>>(base.p4, base.p4_stride, n, sc.counts, base.n_jets, sc.status);
+  k_single_setup<<<1, 256, 0, stream>>>(base.p4, base.p4_stride, n, sc.offsets1, sc.order, sc.counts, sc.queues,
+                                        base.n_jets, sc.status);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
   BatchArgs A = base;
@@ -487,6 +539,18 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
   A.queue = sc.queues;
   A.ws = sc.ws;
   A.ws_stride = sc.ws_stride;
+  if (sc.round_ws && rounds_take(kRoundsFew, n, base.algo_all, base.r_all)) {
+    A.rounds_mode = kRoundsFew;
+    const int q = b < 0 ? kLargeQueue : b, r = b < 0 ? kRetryLargeQueue : kRetryQueue;
+    A.round_ws = sc.round_ws;
+    A.retry = sc.order + r * sc.cap_events;
+    A.n_retry = sc.counts + r;
+    if ((err = launch_rounds(q, A, 1, stream)) != cudaSuccess) return err;
+    A.rounds_mode = kRoundsNone;
+    A.order = A.retry;
+    A.n_order = A.n_retry;
+    A.queue = sc.queues + r;
+  }
   if (b < 0) {
     A.large_ws = sc.large_ws;
     A.tile_factor = tune.tile_factor;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include "fjg_cluster.cuh"
+#include "fjg_cluster_rounds.cuh"
 #include "fjg_cluster_tiled.cuh"
 
 namespace fjg {
@@ -18,6 +19,13 @@ constexpr int kSmemMaxN = 4096;
 // kernel (one CTA of 256 threads per event, state in the large workspace).
 constexpr int kLargeQueue = kNumBuckets;
 constexpr int kNumQueues = kNumBuckets + 1;
+// Two more lists: events that the rounds kernel left to the step-by-step
+// kernels, of up to kSmemMaxN particles and above.
+constexpr int kRetryQueue = kNumQueues;
+constexpr int kRetryLargeQueue = kNumQueues + 1;
+constexpr int kNumLists = kNumQueues + 2;
+// Side streams of a batch: per list one for each of its two kernels.
+constexpr int kNumSide = 2 * kNumQueues;
 constexpr int kLargeMaxN = 1 << 24;
 
 __host__ __device__ inline int bucket_of(int n) {
@@ -58,6 +66,7 @@ __host__ __device__ inline VariantShape variant_shape(int v) {
 // Launch configuration the autotuner chooses: per bucket a variant and the
 // CTAs per SM of its persistent grid (0: as many as fit), the CTAs per SM of
 // the tiled kernel, and its tile side in units of R (>= 1).
+constexpr int kRetryVariant = 9;  // any event of up to kSmemMaxN particles
 struct BucketConfig {
   int variant;
   int ctas_per_sm;
@@ -104,6 +113,11 @@ cudaError_t launch_tiled(const BatchArgs& A, int grid, cudaStream_t s);
 // Sets the tiled kernel's launch attributes once per device (outside a capture).
 cudaError_t configure_tiled();
 
+// The rounds kernel over the work list of A; q: the list's bucket (kLargeQueue
+// above kSmemMaxN particles), which sets threads and tiles.
+cudaError_t launch_rounds(int q, BatchArgs A, int grid, cudaStream_t s);
+int rounds_occupancy(int q);  // resident CTAs per SM (sets the launch attributes on first use)
+
 // Launch variant v (a persistent grid of `grid` CTAs); resident CTAs per SM of
 // variant v on the current device.
 cudaError_t launch_variant(int v, const BatchArgs& A, int grid, int per_sm, cudaStream_t s);
@@ -113,9 +127,9 @@ int bucket_per_sm(const Tuning& tune, int b);  // CTAs per SM that bucket b runs
 
 // Device-side batch descriptor scratch owned by a context.
 struct Scratch {
-  int32_t* order;   // [kNumQueues][cap_events]
-  int32_t* counts;  // [kNumQueues]
-  int* queues;      // [kNumQueues]
+  int32_t* order;   // [kNumLists][cap_events] (kNumQueues without a rounds workspace)
+  int32_t* counts;  // [kNumLists]
+  int* queues;      // [kNumLists + kNumQueues], the last for the rounds kernels
   int* status;      // [1]
   int64_t* offsets1;  // [2] single-event offsets {0, n}
   int cap_events;
@@ -124,13 +138,14 @@ struct Scratch {
   int32_t* hist;      // [kHistBins] events per size, then per-size positions (sorting by size)
   unsigned char* large_ws;    // kLargeWsBytesPerParticle per particle, 16 B aligned (null: large events are refused)
   int64_t large_ws_particles;  // particles the large workspace covers
+  unsigned char* round_ws;     // kRoundBytesPerParticle per particle, 16 B aligned (null: no rounds kernel)
+  int64_t round_ws_particles;
 };
 
 constexpr int kHistBins = kSmemMaxN + 1;
 
 // Launch the bucketing kernels plus one persistent kernel per work list on
-// `stream` (the lists run concurrently on the kNumQueues side streams when
-// given).
+// `stream` (they run concurrently on the kNumSide side streams when given).
 cudaError_t launch_batch(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
                          cudaStream_t stream, cudaStream_t* side, cudaEvent_t* ev_fork, cudaEvent_t* ev_join);
 

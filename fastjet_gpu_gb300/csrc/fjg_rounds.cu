@@ -1,0 +1,110 @@
+// The rounds kernel (fjg_cluster_rounds.cuh) and its launcher.
+#include "fjg_kernels.cuh"
+
+namespace fjg {
+
+// SM: the event's slots in shared memory.
+template <int T, int MINB, bool SM>
+__global__ void __launch_bounds__(T, MINB) k_cluster_rounds(BatchArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RoundShared& S = *reinterpret_cast<RoundShared*>(smem_raw);
+  if (threadIdx.x == 0) {
+    S.tiles = A.round_tiles;
+    S.cells = A.round_cells;
+    S.slots = A.round_slots;
+  }
+  const int count = *A.n_order;
+  for (;;) {
+    if (threadIdx.x == 0) {
+      const int q = atomicAdd(A.queue, 1);
+      S.event = (q < count) ? A.order[q] : -1;
+    }
+    __syncthreads();
+    const int e = S.event;
+    if (e < 0) break;
+    if (!rounds_event(A, e)) {
+      __syncthreads();  // everyone has read S.event
+      continue;
+    }
+    if (refused_event(A, e)) continue;  // ends with a barrier
+    // after a conflict once more with a wider range, which costs less than the
+    // step-by-step kernel; the largest anti-kt events begin with one
+    int64_t off;
+    int n;
+    event_range(A, e, off, n);
+    const bool wide = n > kRoundWideFrom && (A.algo ? A.algo[e] : A.algo_all) == -1;
+    bool done = false;
+#pragma unroll 1
+    for (int attempt = 0; attempt < 2 && !done; ++attempt) {
+      done = cluster_event_rounds<T, SM>(S, A, e, kRoundReach[attempt + (wide ? 1 : 0)]);
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      if (done)
+        signal_done(A, e);
+      else
+        A.retry[atomicAdd(A.n_retry, 1)] = e;
+    }
+  }
+}
+
+namespace {
+
+using Kernel = void (*)(BatchArgs);
+
+// Per list: kernel, threads, tiles (at most 1.5 per particle), tiles with their
+// frame, and slots in shared memory.
+struct RoundConfig {
+  Kernel kernel;
+  int threads, tiles, cells, slots;
+};
+
+RoundConfig config_of(int q) {
+  switch (q) {
+    case 0: return {k_cluster_rounds<128, 4, true>, 128, 384, 1024, 256};
+    case 1: return {k_cluster_rounds<128, 4, true>, 128, 768, 1536, 512};
+    case 2: return {k_cluster_rounds<256, 2, true>, 256, 1024, 1792, 1024};
+    case 3: return {k_cluster_rounds<256, 2, true>, 256, 1024, 1792, 2048};
+    case 4: return {k_cluster_rounds<512, 1, true>, 512, 1024, 1792, 4096};
+    default: return {k_cluster_rounds<512, 1, false>, 512, kRoundMaxTiles, kRoundMaxCells, 0};
+  }
+}
+
+size_t bytes_of(const RoundConfig& c) {
+  return c.slots ? round_smem_bytes<true>(c.tiles, c.cells, c.slots) : round_smem_bytes<false>(c.tiles, c.cells, 0);
+}
+
+static_assert(sizeof(RoundShared) < 10240, "fixed shared memory of a CTA");
+
+}  // namespace
+
+int rounds_occupancy(int q) {
+  static int cache[64][kNumQueues] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int* slot = (dev >= 0 && dev < 64) ? &cache[dev][q] : nullptr;
+  if (slot && *slot) return *slot;
+  const RoundConfig c = config_of(q);
+  int nb = 0;
+  // the attribute belongs to the kernel: the largest any list asks for
+  size_t most = 0;
+  for (int p = 0; p < kNumQueues; ++p)
+    if (config_of(p).kernel == c.kernel && bytes_of(config_of(p)) > most) most = bytes_of(config_of(p));
+  if (cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, c.kernel, c.threads, bytes_of(c)) != cudaSuccess || nb < 1)
+    nb = 1;
+  if (slot) *slot = nb;
+  return nb;
+}
+
+cudaError_t launch_rounds(int q, BatchArgs A, int grid, cudaStream_t s) {
+  rounds_occupancy(q);  // sets the shared-memory attribute
+  const RoundConfig c = config_of(q);
+  A.round_tiles = c.tiles;
+  A.round_cells = c.cells;
+  A.round_slots = c.slots;
+  const int level = q == kLargeQueue ? tiled_priority_level(A.serve_order) : bucket_priority_level(q, A.serve_order);
+  return launch_with_priority(c.kernel, grid, c.threads, bytes_of(c), s, level, A);
+}
+
+}  // namespace fjg

@@ -83,11 +83,15 @@ struct Lane {
   int q = -1;  // queue of the micro-batch in flight
   std::vector<Req*> batch;
   Block host{}, dev{};
-  int* d_queue = nullptr;   // work-queue head (device)
+  int* d_queue = nullptr;   // work-queue head (device), then, kLaneWords in all: the kernel status word, the
+                            // rounds kernel's queue head, the events it left and their queue head
   int* d_status = nullptr;  // kernel status word (device)
+  int32_t* d_retry = nullptr;  // [max_batch] events the rounds kernel left (device)
   int* h_status = nullptr;  // its copy (pinned), valid once ev completes
   int attributed = 0;       // status bits of the micro-batch's requests seen so far
 };
+
+constexpr int kLaneWords = 8;
 
 size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -110,6 +114,7 @@ struct fjg_server {
   void* dev_mem = nullptr;
   double* d_ws = nullptr;
   unsigned char* d_large = nullptr;
+  unsigned char* d_rounds = nullptr;  // rounds kernel's workspace and retry lists (null: not enough memory)
   int32_t* d_iota = nullptr;
   int* d_words = nullptr;
   int* h_words = nullptr;
@@ -223,7 +228,7 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
   L.attributed = 0;
   // the momenta of the micro-batch were copied at admission
   cudaError_t err = cudaStreamWaitEvent(L.stream, S->ev_copy, 0);
-  if (err == cudaSuccess) err = cudaMemsetAsync(L.d_queue, 0, 2 * sizeof(int), L.stream);  // queue head and status
+  if (err == cudaSuccess) err = cudaMemsetAsync(L.d_queue, 0, kLaneWords * sizeof(int), L.stream);
   if (err != cudaSuccess) return err;
   if (S->cfg.flags & FJG_SERVE_DEVICE_CHECK) {
     // momenta checked on the device: a request with a non-finite component
@@ -231,12 +236,34 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
     err = fjg::launch_check_pairs(S->d_p4dev, L.dev.offsets, m, L.dev.ev_status, L.stream);
     if (err != cudaSuccess) return err;
   }
-  if (q == fjg::kLargeQueue) {
-    const int grid = std::min(m, ctx->num_sms * ctx->tune.large_ctas_per_sm);
-    err = fjg::launch_tiled(A, grid, L.stream);
-  } else {
+  auto step_by_step = [&](const fjg::BatchArgs& B) {
+    if (q == fjg::kLargeQueue)
+      return fjg::launch_tiled(B, std::min(m, ctx->num_sms * ctx->tune.large_ctas_per_sm), L.stream);
     const int per_sm = fjg::bucket_per_sm(ctx->tune, q);
-    err = fjg::launch_variant(ctx->tune.bucket[q].variant, A, std::min(m, ctx->num_sms * per_sm), per_sm, L.stream);
+    return fjg::launch_variant(ctx->tune.bucket[q].variant, B, std::min(m, ctx->num_sms * per_sm), per_sm, L.stream);
+  };
+  // the rounds kernel's events (the latency rule), the others, and what the
+  // rounds kernel left
+  int taken = 0;
+  if (S->d_rounds)
+    for (Req* r : L.batch) taken += fjg::rounds_take(fjg::kRoundsFew, r->n, r->algo, r->r) ? 1 : 0;
+  if (taken) {
+    A.rounds_mode = fjg::kRoundsFew;
+    fjg::BatchArgs B = A;
+    B.queue = L.d_queue + 2;
+    B.round_ws = S->d_rounds;
+    B.retry = L.d_retry;
+    B.n_retry = L.d_queue + 3;
+    err = fjg::launch_rounds(q, B, std::min(m, ctx->num_sms * fjg::rounds_occupancy(q)), L.stream);
+    if (err != cudaSuccess) return err;
+  }
+  if (taken < m) err = step_by_step(A);
+  if (err == cudaSuccess && taken) {
+    A.rounds_mode = fjg::kRoundsNone;
+    A.order = L.d_retry;
+    A.n_order = L.d_queue + 3;
+    A.queue = L.d_queue + 4;
+    err = step_by_step(A);
   }
   if (err == cudaSuccess) ++S->launches;
   if (err == cudaSuccess) err = cudaMemcpyAsync(L.h_status, L.d_status, sizeof(int), cudaMemcpyDeviceToHost, L.stream);
@@ -399,13 +426,18 @@ fjg_status fjg_server_create(fjg_ctx* ctx, const fjg_server_config* config, fjg_
   cudaError_t err = cudaHostAlloc(&S->host_mem, b_p4 + b_jets + b_lab + b_hist + b_own + b_done,
                                   cudaHostAllocMapped | cudaHostAllocPortable);
   if (err == cudaSuccess)
-    err = cudaHostAlloc(&S->block_mem, per_block * c.streams + al(8 * (size_t)c.streams),
+    err = cudaHostAlloc(&S->block_mem, per_block * c.streams + al(4 * (size_t)kLaneWords * c.streams),
                         cudaHostAllocMapped | cudaHostAllocPortable);
   const size_t b_ws = al(sizeof(double) * fjg::kWsFields * (size_t)P);
   const size_t b_large = al((size_t)fjg::kLargeWsBytesPerParticle * (size_t)P);
-  const size_t b_iota = al(4 * (size_t)c.max_batch), b_words = al(8 * (size_t)c.streams);
+  const size_t b_iota = al(4 * (size_t)c.max_batch), b_words = al(4 * (size_t)kLaneWords * c.streams);
   const size_t b_p4dev = al(32 * (size_t)P);
   if (err == cudaSuccess) err = cudaMalloc(&S->dev_mem, b_ws + b_large + b_iota + b_words + b_p4dev);
+  const size_t b_rounds = al((size_t)fjg::kRoundBytesPerParticle * (size_t)P);
+  if (err == cudaSuccess && cudaMalloc(&S->d_rounds, b_rounds + 4 * (size_t)c.max_batch * c.streams) != cudaSuccess) {
+    cudaGetLastError();
+    S->d_rounds = nullptr;
+  }
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&S->copy_stream, cudaStreamNonBlocking);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&S->ev_copy, cudaEventDisableTiming);
   auto dev_of = [&](void* h) {
@@ -464,9 +496,10 @@ fjg_status fjg_server_create(fjg_ctx* ctx, const fjg_server_config* config, fjg_
       L.dev.n_jets = static_cast<int32_t*>(dev_of(L.host.n_jets));
       L.dev.ev_status = static_cast<int32_t*>(dev_of(L.host.ev_status));
       L.dev.count = static_cast<int32_t*>(dev_of(L.host.count));
-      L.d_queue = S->d_words + 2 * k;
-      L.d_status = S->d_words + 2 * k + 1;
-      L.h_status = S->h_words + 2 * k + 1;
+      L.d_queue = S->d_words + kLaneWords * k;
+      L.d_status = L.d_queue + 1;
+      L.h_status = S->h_words + kLaneWords * k + 1;
+      if (S->d_rounds) L.d_retry = reinterpret_cast<int32_t*>(S->d_rounds + b_rounds) + (size_t)c.max_batch * k;
       if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking);
       if (err == cudaSuccess) err = cudaEventCreateWithFlags(&L.ev, cudaEventDisableTiming);
     }
@@ -509,6 +542,7 @@ void fjg_server_destroy(fjg_server* S) {
   }
   if (S->ev_copy) cudaEventDestroy(S->ev_copy);
   if (S->dev_mem) cudaFree(S->dev_mem);
+  if (S->d_rounds) cudaFree(S->d_rounds);
   if (S->host_mem) cudaFreeHost(S->host_mem);
   if (S->block_mem) cudaFreeHost(S->block_mem);
   delete S;

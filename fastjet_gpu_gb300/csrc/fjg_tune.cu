@@ -99,11 +99,14 @@ cudaError_t time_batch(fjg_ctx* ctx, const TuneBuffers& tb, int n_events, int64_
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t err = cudaEventCreate(&e0);
   if (err == cudaSuccess) err = cudaEventCreate(&e1);
+  // the shapes under test, not the rounds kernel
+  fjg::Scratch sc = ctx->scratch.sc;
+  sc.round_ws = nullptr;
   double best = 1e30;
   for (int rep = 0; rep < 3 && err == cudaSuccess; ++rep) {
     err = cudaEventRecord(e0, ctx->stream);
     if (err == cudaSuccess)
-      err = fjg::launch_batch(A, ctx->scratch.sc, n_events, ctx->num_sms, t, ctx->stream, ctx->side, &ctx->ev_fork,
+      err = fjg::launch_batch(A, sc, n_events, ctx->num_sms, t, ctx->stream, ctx->side, &ctx->ev_fork,
                               ctx->ev_join);
     if (err == cudaSuccess) err = cudaEventRecord(e1, ctx->stream);
     if (err == cudaSuccess) err = cudaEventSynchronize(e1);
