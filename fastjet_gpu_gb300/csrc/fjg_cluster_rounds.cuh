@@ -113,8 +113,9 @@ __device__ __forceinline__ bool rounds_event(const BatchArgs& A, int e) {
 
 constexpr int kRoundSteps = 32;               // steps per round, at most (a lane each)
 constexpr int kRoundBytesPerParticle = 240;   // workspace
-constexpr int kRoundMaxDirty = 512;
-constexpr int kRoundMaxTargets = 256;
+constexpr int kRoundMaxDirty = 384;
+constexpr int kRoundMaxTargets = 128;
+constexpr int kRoundSplit = 8;                // searches of a round, up to which several warps share each
 constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, also in one row
 // range of the choice of steps, in units of R (see above): the first attempt at
 // an event, the second (the first for the largest anti-kt events), the last
@@ -171,7 +172,6 @@ struct RoundWs {
   Idx* members;   // [kRoom * N]
   float2* lxy;    // [kRoom * N] coordinates in list order, read with consecutive lanes (not SM)
   double2* pos;   // [N] rapidity, azimuth
-  float* nlo;     // [N] neighbour distance, lower bound
   float* tlo;     // [N] birth time's M, rounded down
   double* tm;     // [N] birth time M
   int2* tl;       // [N] birth time l, depth
@@ -207,10 +207,9 @@ __device__ __forceinline__ RoundWs<SM> round_ws(unsigned char* base, unsigned ch
   W.tl = reinterpret_cast<int2*>(base + 120 * n);
   W.stamp = reinterpret_cast<int2*>(base + 128 * n);
   W.dnext = reinterpret_cast<int*>(base + 136 * n);
-  W.nlo = reinterpret_cast<float*>(base + 144 * n);
-  W.tlo = W.nlo + n;
-  W.lxy = reinterpret_cast<float2*>(base + 152 * n);
-  // 184 n bytes; then, in the workspace, 52 n more
+  W.lxy = reinterpret_cast<float2*>(base + 144 * n);
+  W.tlo = reinterpret_cast<float*>(base + 176 * n);
+  // 180 n bytes, and 4 n unused; then, in the workspace, 52 n more
   unsigned char* p = SM ? smem : base + 184 * n;
   const int64_t m = SM ? cap : N;
   W.xy = reinterpret_cast<float2*>(p);
@@ -256,10 +255,14 @@ struct RoundShared {
   // slots they remove and keep, tile of the new jet
   int c[kRoundSteps], j[kRoundSteps], l[kRoundSteps], depth[kRoundSteps];
   int2 tp_b[kRoundSteps], tp_a[kRoundSteps];
+  int tile_c[kRoundSteps], tile_j[kRoundSteps];
+  float2 xy_c[kRoundSteps], xy_j[kRoundSteps], wlo[kRoundSteps];  // (weights of c and of j)
   int new_u[kRoundSteps], new_v[kRoundSteps];
   double M[kRoundSteps], key[kRoundSteps], thr_c[kRoundSteps], thr_j[kRoundSteps];
   double phi[kRoundSteps], rap[kRoundSteps], w[kRoundSteps], p4[4][kRoundSteps];
   int targets[kRoundMaxTargets];
+  Cert part[kRoundSplit][4];  // searches shared by several warps
+  int parts_done[kRoundSplit];
   unsigned short cand[kRoundMaxCand];  // tiles
   unsigned short dirty[kRoundMaxDirty];
   unsigned dirty_bits[kRoundMaxTiles / 32];
@@ -271,19 +274,19 @@ struct RoundShared {
 // columns of the frame repeat the tiles across the azimuth seam, so that a
 // neighbourhood is read without wrapping) and 5-tile row minima, then `tiles`
 // entries of the per-tile arrays, then the slots.
-__host__ __device__ __forceinline__ size_t round_tile_bytes(int tiles, int cells) {
-  return ((size_t)cells * 12 + (size_t)tiles * 20 + 16 + 15) & ~size_t(15);
+__host__ __device__ constexpr size_t round_tile_bytes(int tiles, int cells) {
+  return ((size_t)cells * 12 + (size_t)tiles * 22 + 16 + 15) & ~size_t(15);
 }
-__host__ __device__ __forceinline__ size_t round_tile_bytes_sm(int tiles, int cells) {
+__host__ __device__ constexpr size_t round_tile_bytes_sm(int tiles, int cells) {
   return ((size_t)cells * 8 + (size_t)tiles * 16 + 16 + 15) & ~size_t(15);
 }
-__host__ __device__ __forceinline__ size_t round_tiles_at() { return (sizeof(RoundShared) + 15) & ~size_t(15); }
+__host__ __device__ constexpr size_t round_tiles_at() { return (sizeof(RoundShared) + 15) & ~size_t(15); }
 template <bool SM>
-__host__ __device__ __forceinline__ size_t round_slots_at(int tiles, int cells) {
+__host__ __device__ constexpr size_t round_slots_at(int tiles, int cells) {
   return round_tiles_at() + (SM ? round_tile_bytes_sm(tiles, cells) : round_tile_bytes(tiles, cells));
 }
 template <bool SM>
-__host__ __device__ __forceinline__ size_t round_smem_bytes(int tiles, int cells, int slots) {
+__host__ __device__ constexpr size_t round_smem_bytes(int tiles, int cells, int slots) {
   return round_slots_at<SM>(tiles, cells) + (size_t)slots * kRoundSlotBytes;
 }
 
@@ -298,6 +301,7 @@ struct RoundCtx {
   int* head;       // [nt] groups of the dead
   float* head_m;   // [nt] the first one's M (0: none)
   Idx* slot;       // [nt] the slot of the minimum
+  unsigned short* beside;  // [nt] the tile of its partner, or its own (not SM)
   Idx* start;      // [nt + 1]
   RoundWs<SM> W;
 };
@@ -317,6 +321,7 @@ __device__ __forceinline__ RoundCtx<SM> round_ctx() {
   C.head_m = reinterpret_cast<float*>(C.head + tiles);
   C.slot = reinterpret_cast<typename RoundCtx<SM>::Idx*>(C.head_m + tiles);
   C.start = C.slot + tiles;
+  C.beside = reinterpret_cast<unsigned short*>(C.start + tiles + 2);
   C.W = round_ws<SM>(C.S->ws, smem_raw + round_slots_at<SM>(tiles, cells), C.S->X.N, C.S->slots);
   return C;
 }
@@ -365,37 +370,44 @@ __device__ __forceinline__ int box_tile(const RoundShared& S, const RoundBox& b,
   return ((b.u0 + du) << S.sh) + v;
 }
 
-// fn(slot, load(slot, entry)) for every list entry of the box's tiles k0 .. n-1,
-// by a group of G lanes (G = 8 or 32, the same in the whole warp; the functions
-// hold no warp collectives).  Dense lists in the workspace (G = 32): five tiles
-// at a time, a lane per member, so that five loads are in flight.  Otherwise a
-// lane per tile, two members at a time.  List lengths are bounded by the
-// tile's room.
+// fn(slot, load(slot, coordinates)) for every list entry of the box's tiles k0 ..
+// n-1 (the functions hold no warp collectives).  Lists in shared memory: a group
+// of G lanes (8 or 32, the same in the whole warp), a lane per tile, two members
+// at a time.  Lists in the workspace: a warp, `sub` lanes per tile (a power of
+// two near the mean list length, so that most lists are gone over at once) and
+// five tiles a lane, so that five loads are in flight: a window of short lists
+// costs two dependent loads, not two for every pair of members.  List lengths
+// are bounded by the tile's room.
 template <bool SM, class Load, class Fn>
-__device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox& b, int k0, int n, int G, bool dense,
+__device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox& b, int k0, int n, int G, int sub,
                                           Load load, Fn fn) {
   const RoundShared& S = *C.S;
   constexpr int kNone = RoundWs<SM>::kNone;
-  if (!SM && dense) {
+  if (!SM) {
     constexpr int B = 5;
+    const int lane = threadIdx.x & 31, first = lane & (sub - 1), per = 32 / sub;
 #pragma unroll 1
-    for (; k0 < n; k0 += B) {
+    for (k0 += lane / sub; k0 < n; k0 += B * per) {
       int st[B], ln[B], most = 0;
 #pragma unroll
       for (int q = 0; q < B; ++q) {
-        const int t = box_tile(S, b, k0 + q < n ? k0 + q : k0);
+        const int k = k0 + q * per, t = box_tile(S, b, k < n ? k : k0);
         st[q] = C.start[t];
-        ln[q] = k0 + q < n ? min(C.count[t], (int)C.start[t + 1] - st[q]) : 0;
+        ln[q] = k < n ? min(C.count[t], (int)C.start[t + 1] - st[q]) : 0;
         most = max(most, ln[q]);
       }
 #pragma unroll 1
-      for (int i = threadIdx.x & 31; i < most; i += 32) {
+      for (int i = first; i < most; i += sub) {
         int u[B];
-        decltype(load(0, 0)) d[B];
+        float2 g[B];
+        decltype(load(0, make_float2(0.0f, 0.0f))) d[B];
 #pragma unroll
-        for (int q = 0; q < B; ++q) u[q] = i < ln[q] ? (int)C.W.members[st[q] + i] : kNone;
+        for (int q = 0; q < B; ++q) {
+          u[q] = i < ln[q] ? (int)C.W.members[st[q] + i] : kNone;
+          g[q] = C.W.lxy[st[q] + (i < ln[q] ? i : 0)];
+        }
 #pragma unroll
-        for (int q = 0; q < B; ++q) d[q] = load(u[q] != kNone ? u[q] : 0, st[q] + (i < ln[q] ? i : 0));
+        for (int q = 0; q < B; ++q) d[q] = load(u[q] != kNone ? u[q] : 0, g[q]);
 #pragma unroll
         for (int q = 0; q < B; ++q)
           if (u[q] != kNone) fn(u[q], d[q]);
@@ -409,7 +421,8 @@ __device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox&
 #pragma unroll 1
       for (int i = 0; i < m; i += 2) {
         const int u0 = C.W.members[st + i], u1 = i + 1 < m ? (int)C.W.members[st + i + 1] : kNone;
-        const auto d0 = load(u0 != kNone ? u0 : 0, st + i), d1 = load(u1 != kNone ? u1 : 0, st + i + (i + 1 < m ? 1 : 0));
+        const int v0 = u0 != kNone ? u0 : 0, v1 = u1 != kNone ? u1 : v0;
+        const auto d0 = load(v0, C.W.xy[v0]), d1 = load(v1, C.W.xy[v1]);
         if (u0 != kNone) fn(u0, d0);
         if (u1 != kNone) fn(u1, d1);
       }
@@ -419,8 +432,8 @@ __device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox&
 }
 
 template <bool SM, class Load, class Fn>
-__device__ __forceinline__ void for_box(const RoundCtx<SM>& C, const RoundBox& b, int G, bool dense, Load load, Fn fn) {
-  for_tiles(C, b, 0, b.nu * b.nv, G, dense, load, fn);
+__device__ __forceinline__ void for_box(const RoundCtx<SM>& C, const RoundBox& b, int G, int sub, Load load, Fn fn) {
+  for_tiles(C, b, 0, b.nu * b.nv, G, sub, load, fn);
 }
 
 // Combination of certificates over groups of G lanes (all lanes call).
@@ -473,22 +486,26 @@ __device__ __forceinline__ bool round_first(const RoundCtx<SM>& C, int s, int ro
 
 // Slot t's neighbour nn with distance interval [lo, hi]: neighbour, key and P;
 // the tile is marked as changed.  The FP32 filter's interval is wide for close
-// pairs (its bound is absolute), which FP64 settles, so that keys compare well.
+// pairs (its bound is absolute), which FP64 settles, so that keys compare well:
+// a neighbour's interval is narrower than 2^-16 of it.  `keep`: kTarget, if the
+// other groups of this phase are to leave t alone.  What may be needed is
+// loaded at once.
 template <bool SM>
-__device__ __noinline__ void round_set(int t, int nn, float lo, float hi) {
+__device__ __noinline__ void round_set(int t, int nn, float lo, float hi, int keep) {
   using Ws_ = RoundWs<SM>;
   const RoundCtx<SM> C = round_ctx<SM>();
   const EventCtx& X = C.S->X;
-  const float w = C.W.wlo[t], tlo = C.W.tlo[t];
+  const int n = nn < 0 ? t : nn;
+  const float w = C.W.wlo[t], tlo = C.W.tlo[t], wn = C.W.wlo[n], tn = C.W.tlo[n];
+  const double2 pt = C.W.pos[t], pn = C.W.pos[n];
   round_dirty(*C.S, C.W.tile[t]);
   float klo = round_wlo(w), p = fmaxf(klo, tlo);
   int field = Ws_::kNoSlot;
   if (nn < 0) {
-    lo = hi = __int_as_float(0x7f800000);
+    hi = __int_as_float(0x7f800000);
   } else {
-    const float wn = C.W.wlo[nn], tn = C.W.tlo[nn];
     if (hi - lo > lo * 0x1p-16f) {
-      const double d = C.W.dr2(t, nn);
+      const double d = dr2_64(pt.x, pt.y, pn.x, pn.y);
       lo = __double2float_rd(d);
       hi = __double2float_ru(d);
     }
@@ -496,7 +513,7 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi) {
     int kind = key_interval(klo, round_whi(w), round_wlo(wn), round_whi(wn), lo, hi, X.ilo, X.ihi, klo, khi);
     if (kind < 0) {
       const double w64 = X.g.at(kW, t);
-      const double dp = pair_distance(w64, X.g.at(kW, nn), C.W.dr2(t, nn), X.inv_r2);
+      const double dp = pair_distance(w64, X.g.at(kW, nn), dr2_64(pt.x, pt.y, pn.x, pn.y), X.inv_r2);
       kind = dp < w64 ? 1 : 0;
       klo = __double2float_rd(kind ? dp : w64);
     }
@@ -506,10 +523,7 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi) {
   }
   C.W.key[t] = make_float2(klo, p);
   C.W.nhi[t] = hi;
-  C.W.nlo[t] = lo;
-  // the field last: a reader that sees it without the target bit sees the rest
-  __threadfence_block();
-  C.W.nn[t] = (typename Ws_::Idx)field;
+  C.W.nn[t] = (typename Ws_::Idx)(field | keep);
 }
 
 // Slot t's neighbour by the exact minimum (dR2, label) over its window (whole
@@ -523,7 +537,7 @@ __device__ __noinline__ int round_exact(int t, float u1) {
   const Bound bd = C.S->X.bd;
   unsigned long long bk = ~0ull;
   int bi = 0x7fffffff;
-  for_box(C, b, 32, false, [&](int u, int i) { return C.W.entry(u, i); },
+  for_box(C, b, 32, 8, [&](int, float2 g) { return g; },
           [&](int u, float2 gu) {
             float l, h;
             dr2_32(gt.x, gt.y, gu.x, gu.y, bd, l, h);
@@ -540,10 +554,10 @@ __device__ __noinline__ int round_exact(int t, float u1) {
 // Stores slot t's neighbour from its group's certificate (every lane calls;
 // lane `first` of the group holds the work, have: it has some).
 template <bool SM>
-__device__ __forceinline__ void round_settle(bool have, bool first, int t, const Cert& c) {
+__device__ __forceinline__ void round_settle(bool have, bool first, int t, const Cert& c, int keep) {
   const bool exact = have && first && c.i1 >= 0 && !cert_ok(c);
   unsigned todo = __ballot_sync(kFull, exact);
-  if (have && first && !exact) round_set<SM>(t, c.i1, c.m1, c.u1);
+  if (have && first && !exact) round_set<SM>(t, c.i1, c.m1, c.u1, keep);
   __syncwarp();
   while (todo) {
     const int q = __ffs(todo) - 1;
@@ -551,14 +565,31 @@ __device__ __forceinline__ void round_settle(bool have, bool first, int t, const
     const int tq = __shfl_sync(kFull, t, q);
     const int nn = round_exact<SM>(tq, __shfl_sync(kFull, c.u1, q));
     // (an empty interval: the FP64 value is taken)
-    if ((threadIdx.x & 31) == q) round_set<SM>(tq, nn, 0.0f, __int_as_float(0x7f800000));
+    if ((threadIdx.x & 31) == q) round_set<SM>(tq, nn, 0.0f, __int_as_float(0x7f800000), keep);
     __syncwarp();
   }
 }
 
-// Slot t's neighbour in its window, and its key (groups of G lanes).
+// The certificate of search `item` from its parts, each done by a warp (parts >
+// 1; every lane calls): true for the last one, which holds the whole.
+__device__ __forceinline__ bool round_join(RoundShared& S, Cert& c, int item, int part, int parts) {
+  const int lane = threadIdx.x & 31;
+  int done = 0;
+  if (lane == 0) {
+    S.part[item][part] = c;
+    __threadfence_block();
+    done = atomicAdd(&S.parts_done[item], 1);
+  }
+  if (__shfl_sync(kFull, done, 0) != parts - 1) return false;
+  __threadfence_block();
+  c = cert_warp(lane < parts ? S.part[item][lane] : cert_empty());
+  return true;
+}
+
+// Slot t's neighbour in its window, and its key (groups of G lanes; or one of
+// several warps of search `item`).
 template <bool SM>
-__device__ __noinline__ void round_search(bool have, int t, int G, bool dense) {
+__device__ __noinline__ void round_search(bool have, int t, int G, int sub, int item, int part, int parts) {
   const RoundCtx<SM> C = round_ctx<SM>();
   const int tile = have ? (int)C.W.tile[t] : 0;
   RoundBox b = round_box(*C.S, tile, tile);
@@ -566,36 +597,37 @@ __device__ __noinline__ void round_search(bool have, int t, int G, bool dense) {
   const float2 gt = C.W.xy[t];
   const Bound bd = C.S->X.bd;
   Cert x = cert_empty();
-  for_box(C, b, G, dense, [&](int u, int i) { return C.W.entry(u, i); },
+  const int nb = b.nu * b.nv;
+  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub, [&](int, float2 g) { return g; },
           [&](int u, float2 gu) {
             float lo, hi;
             dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
             if (u != t) cert_add(x, lo, hi, u);
           });
   x = cert_group(x, G);
-  round_settle<SM>(have, (threadIdx.x & (G - 1)) == 0, t, x);
+  if (parts > 1 && !round_join(*C.S, x, item, part, parts)) return;
+  round_settle<SM>(have, (threadIdx.x & (G - 1)) == 0, t, x, RoundWs<SM>::kTarget);
 }
 
-// New jet a, with FP32 distance interval [lo, hi] to slot y, may be closer to y
-// than its neighbour.  (y's neighbour field had no target bit when it was
-// read; if it has just been searched, which offered it a, nothing changes.)
+// New jet a, with FP32 distance interval [lo, hi] to slot y (no target), may be
+// closer to y than its neighbour.  Another jet may be given to y at the same
+// time: whichever of y's words are seen, what is kept is closer than before,
+// and of two that claim y the second has it searched.
 template <bool SM>
-__device__ __noinline__ void round_offer(int y, int a, float lo, float hi, int round) {
+__device__ __noinline__ void round_offer(int y, int a, float lo, float hi, float nhi, int round) {
   using Ws_ = RoundWs<SM>;
   const RoundCtx<SM> C = round_ctx<SM>();
-  __threadfence_block();
-  if (!(hi < *(volatile float*)(C.W.nlo + y))) {
+  if (!(hi < nhi * (1.0f - 0x1p-14f))) {
     const int cn = *(volatile typename Ws_::Idx*)(C.W.nn + y) & Ws_::kSlotMask;
-    const double da = C.W.dr2(y, a);
     if (cn != Ws_::kNoSlot) {
-      const double dc = C.W.dr2(y, cn);
+      const double da = C.W.dr2(y, a), dc = C.W.dr2(y, cn);
       if (!(da < dc || (da == dc && a < cn))) return;
     }
   }
   if (round_first(C, y, round, 1))
-    round_set<SM>(y, a, lo, hi);
+    round_set<SM>(y, a, lo, hi, 0);
   else
-    round_target(*C.S, y);  // another new jet was closer to it as well: a full search (phase E)
+    round_target(*C.S, y);  // (phase E)
 }
 
 // D1 in FP64 (see the header): pseudojet x of a step with time part M and
@@ -616,6 +648,14 @@ __device__ __forceinline__ void round_store_min(const RoundCtx<SM>& C, int t, un
   const int u = t >> S.sh, v = t & ((1 << S.sh) - 1);
   unsigned* row = C.tmin + (u + kRoundFrame) * S.pw + kRoundFrame;
   C.slot[t] = (typename RoundCtx<SM>::Idx)slot;
+  if (!SM) {
+    int beside = t;
+    if (slot >= 0) {
+      const int f = C.W.nn[slot];
+      if (f & RoundWs<SM>::kPair) beside = C.W.tile[f & RoundWs<SM>::kSlotMask];
+    }
+    C.beside[t] = (unsigned short)beside;
+  }
   row[v] = p;
 #pragma unroll 1
   for (int w = v - S.nphi; w >= -kRoundFrame; w -= S.nphi) row[w] = p;
@@ -879,7 +919,7 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
             }
           }
         }
-        round_settle<SM>(have, true, t, c);
+        round_settle<SM>(have, true, t, c, 0);
       }
     }
     return;
@@ -909,7 +949,7 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
       }
     }
     __syncwarp();
-    round_settle<SM>(have, true, t, c);
+    round_settle<SM>(have, true, t, c, 0);
   }
 }
 
@@ -923,7 +963,7 @@ __device__ __forceinline__ float plain_dr2(float2 a, float2 b) {
 // Phase B for the steps, by groups of G lanes: D1, and the slots whose neighbour
 // is taken.  With few steps their windows are cut in parts.
 template <bool SM>
-__device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int G, bool dense, int parts) {
+__device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int G, int sub, int parts) {
   using Ws_ = RoundWs<SM>;
   RoundShared& S = *C.S;
   const Ws_& Wk = C.W;
@@ -939,16 +979,16 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
     const int part = i % parts;  // (several parts: G = 32)
     i = G == 32 ? i / parts : i + lane / 8;
     const bool have = i < F;
-    const int c = have ? S.c[i] : 0, j = have ? S.j[i] : -1, jc = j >= 0 ? j : c;
-    const float2 gc = Wk.xy[c], gj = Wk.xy[jc];
-    const float wc = round_wlo(Wk.wlo[c]), wj = round_wlo(Wk.wlo[jc]);
+    const int at = have ? i : 0, c = S.c[at], j = have ? S.j[at] : -1;
+    const float2 gc = S.xy_c[at], gj = S.xy_j[at];
+    const float wc = S.wlo[at].x, wj = S.wlo[at].y;
     RoundBox b{0, 0, 0, 1};
     double M = 0.0, thr_c = 0.0, thr_j = 0.0;
     if (have) {
       M = S.M[i];
       thr_c = S.thr_c[i];
       thr_j = S.thr_j[i];
-      b = round_box(S, Wk.tile[c], Wk.tile[jc]);
+      b = round_box(S, S.tile_c[i], S.tile_j[i]);
     }
     const float tc_hi = __double2float_ru(thr_c), tj_hi = __double2float_ru(thr_j);
     struct Slot {
@@ -958,8 +998,8 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
     };
     bool bad = false;
     const int nb = b.nu * b.nv;
-    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, dense,
-            [&](int y, int i) { return Slot{Wk.entry(y, i), Wk.wlo[y], Wk.nn[y]}; },
+    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub,
+            [&](int y, float2 g) { return Slot{g, Wk.wlo[y], Wk.nn[y]}; },
             [&](int y, const Slot& s) {
               if (y == c || y == j) return;
               const int nn = s.nn & Ws_::kSlotMask;
@@ -988,7 +1028,8 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
 
 // Phase D for one step that made jet a (groups of G lanes): the jet's window.
 template <bool SM>
-__device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, int i, int round, int G, bool dense) {
+__device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, int i, int round, int G, int sub,
+                                              int part, int parts) {
   using Ws_ = RoundWs<SM>;
   RoundShared& S = *C.S;
   const Ws_& Wk = C.W;
@@ -998,24 +1039,27 @@ __device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, 
   const int tile = have ? (S.new_u[i] << S.sh) + S.new_v[i] : 0;
   RoundBox b = round_box(S, tile, tile);
   if (!have) b.nu = 0;
-  const float2 ga = Wk.xy[a];
+  const float2 ga = make_float2(__double2float_rn(S.rap[have ? i : 0]), __double2float_rn(S.phi[have ? i : 0]));
   struct Slot {
     float2 g;
     float nhi;
     int nn;
   };
   Cert ca = cert_empty();
-  for_box(C, b, G, dense, [&](int y, int i) { return Slot{Wk.entry(y, i), Wk.nhi[y], Wk.nn[y]}; },
+  const int nb = b.nu * b.nv;
+  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub,
+          [&](int y, float2 g) { return Slot{g, Wk.nhi[y], Wk.nn[y]}; },
           [&](int y, const Slot& s) {
             if (y == a) return;
             float lo, hi;
             dr2_32(s.g.x, s.g.y, ga.x, ga.y, bd, lo, hi);
             cert_add(ca, lo, hi, y);
             // not closer, or searched anyway?
-            if (!(lo > s.nhi) && !(s.nn & Ws_::kTarget)) round_offer<SM>(y, a, lo, hi, round);
+            if (!(lo > s.nhi) && !(s.nn & Ws_::kTarget)) round_offer<SM>(y, a, lo, hi, s.nhi, round);
           });
   ca = cert_group(ca, G);
-  round_settle<SM>(have, (lane & (G - 1)) == 0, a, ca);
+  if (parts > 1 && !round_join(S, ca, i, part, parts)) return;
+  round_settle<SM>(have, (lane & (G - 1)) == 0, a, ca, Ws_::kTarget);
 }
 
 // Records of at most 4096 slots in time order: bitonic sort in shared memory
@@ -1261,6 +1305,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
 #pragma unroll 1
   for (int round = 0; n > 0; ++round) {
     const bool dense = !SM && n >= kRoundDense * nt;
+    const int sub = n > 16 * nt ? 32 : n > 8 * nt ? 16 : n > 3 * nt ? 8 : 4;
     // A: candidates.  Smallest P of five tiles along the row, then of five
     // rows (empty tiles hold the largest value)
 #pragma unroll 1
@@ -1284,13 +1329,14 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         // a step also counts where its partner is: a hard jet's own key may
         // belong to a later step (its neighbour is younger) while an earlier
         // one takes it from the far side of its reach
-        const int f = Wk.nn[C.slot[t]];
-        const int tj = f & Ws_::kPair ? (int)Wk.tile[f & Ws_::kSlotMask] : t;
+        const int tj = C.beside[t];
         if (tj != t) {
           const int vj = tj & ((1 << sh) - 1);
           unsigned* cell = C.near + ((tj >> sh) + kRoundFrame) * pw + kRoundFrame;
-          for (int w = vj % nphi - (kRoundFrame / nphi + 1) * nphi; w < nphi + kRoundFrame; w += nphi)
-            if (w >= -kRoundFrame) atomicMin(cell + w, me);
+          atomicMin(cell + vj, me);
+          // (copies across the azimuth seam: at most one each way in the frame of ten tiles or more)
+          if (vj >= nphi - kRoundFrame && vj - nphi >= -kRoundFrame) atomicMin(cell + vj - nphi, me);
+          if (vj < kRoundFrame) atomicMin(cell + vj + nphi, me);
         }
       }
       if (me == min(min(min(C.row[k - 2 * pw], C.row[k - pw]), min(C.row[k + pw], C.row[k + 2 * pw])), C.row[k])) {
@@ -1298,6 +1344,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         if (q < kRoundMaxCand) S.cand[q] = (unsigned short)t;
       }
     }
+    if (!SM && tid < kRoundSplit) S.parts_done[tid] = 0;
     if (SM)
       for (int k = tid; k < (N + 31) / 32; k += T) S.taken[k] = S.claimed[k] = 0;
     __syncthreads();
@@ -1399,6 +1446,12 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           S.depth[i] = te.depth;
           S.thr_c[i] = thr_c;
           S.thr_j[i] = thr_j;
+          const int jn = j >= 0 ? j : c;
+          S.tile_c[i] = Wk.tile[c];
+          S.tile_j[i] = Wk.tile[jn];
+          S.xy_c[i] = Wk.xy[c];
+          S.xy_j[i] = Wk.xy[jn];
+          S.wlo[i] = make_float2(round_wlo(Wk.wlo[c]), round_wlo(Wk.wlo[jn]));
         }
       }
       __syncwarp();
@@ -1428,15 +1481,15 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         if (have) {
           b = max(c, j);
           m_hi = __double2float_ru(S.M[i]);
-          const float2 gc = Wk.xy[c];
-          dc = make_float4(gc.x, gc.y, round_wlo(Wk.wlo[c]), __double2float_ru(S.thr_c[i]));
-          const int2 tpc = make_int2(Wk.tile[c], Wk.at[c]);
+          const float2 gc = S.xy_c[i];
+          dc = make_float4(gc.x, gc.y, S.wlo[i].x, __double2float_ru(S.thr_c[i]));
+          const int2 tpc = make_int2(S.tile_c[i], Wk.at[c]);
           tile_c = tpc.x;
           S.tp_b[i] = tpc;
           if (j >= 0) {
-            const float2 gj = Wk.xy[j];
-            dj = make_float4(gj.x, gj.y, round_wlo(Wk.wlo[j]), __double2float_ru(S.thr_j[i]));
-            const int2 tpj = make_int2(Wk.tile[j], Wk.at[j]);
+            const float2 gj = S.xy_j[i];
+            dj = make_float4(gj.x, gj.y, S.wlo[i].y, __double2float_ru(S.thr_j[i]));
+            const int2 tpj = make_int2(S.tile_j[i], Wk.at[j]);
             tile_j = tpj.x;
             S.tp_b[i] = c > j ? tpc : tpj;
             S.tp_a[i] = c > j ? tpj : tpc;
@@ -1481,7 +1534,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     }
     // D1 and the targets
     FJG_PH(const long long qb = clock64();)
-    round_phase_b(C, F, G, dense, G == 32 ? max(1, (W - 3) / F) : 1);
+    round_phase_b(C, F, G, sub, G == 32 ? max(1, (W - 3) / F) : 1);
     FJG_PH(if (tid == T - 32 && A.phase) atomicAdd(A.phase + kPhRScan, (unsigned long long)(clock64() - qb));)
     __syncthreads();
     FJG_PH(mark(kPhRB);)
@@ -1547,29 +1600,29 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     }
     FJG_PH(mark(kPhRC);)
 
-    // D and E: each new jet against its window; the targets' searches (one may
-    // have been taken by another step, or be a new jet); the dead of each new
-    // jet's window (D2).  A warp takes 32 / G of a kind at a time.
+    // D: each new jet against its window; the targets' searches (one may have
+    // been taken by another step); the dead of each new jet's window (D2).  A
+    // warp takes 32 / G of a kind at a time, or a part of one.
     const int ntg = min(S.n_targets, kRoundMaxTargets);
     __syncthreads();  // D adds targets
-    const int per = 32 / G, uf = (F + per - 1) / per, ut = (ntg + per - 1) / per;
+    const int per = 32 / G;
+    const int parts = !SM && F + ntg <= kRoundSplit ? min(4, W / (F + ntg)) : 1;
+    const int uf = (F + per - 1) / per * parts, ut = (ntg + per - 1) / per * parts, ud = (F + per - 1) / per;
 #pragma unroll 1
     for (;;) {
       int u = 0;
       if (lane == 0) u = atomicAdd(&S.task[1], 1);
       u = __shfl_sync(kFull, u, 0);
-      if (u >= 2 * uf + ut) break;
+      if (u >= uf + ut + ud) break;
       FJG_PH(const long long qd = clock64();)
       const int q = G == 32 ? 0 : lane / 8;
       if (u < uf) {
-        const int i = per * u + q;
-        round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, round, G, dense);
+        const int i = per * (u / parts) + q;
+        round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, round, G, sub, u % parts, parts);
       } else if (u < uf + ut) {
-        const int k = per * (u - uf) + q;
+        const int k = per * ((u - uf) / parts) + q;
         const int t = S.targets[k < ntg ? k : 0];
-        const bool live = k < ntg && (int)Wk.tile[t] != kNone &&
-                          (Wk.nn[t] & (Ws_::kSlotMask | Ws_::kTarget)) != (Ws_::kNoSlot | Ws_::kTarget);
-        round_search<SM>(live, t, G, dense);
+        round_search<SM>(k < ntg && (int)Wk.tile[t] != kNone, t, G, sub, F + k, (u - uf) % parts, parts);
       } else {
         const int i = per * (u - uf - ut) + q;
         if (i < F && S.j[i] >= 0) {
@@ -1601,12 +1654,16 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     }
     if (ntg2 > ntg) {  // slots that two new jets wanted
 #pragma unroll 1
-      for (int k = ntg + warp; k < ntg2; k += W) round_search<SM>(true, S.targets[k], 32, dense);
+      for (int k = ntg + warp; k < ntg2; k += W) round_search<SM>(true, S.targets[k], 32, sub, 0, 0, 1);
       __syncthreads();
     }
     FJG_PH(mark(kPhRE);)
 
-    // F: changed tiles
+    // F: the target bits off; changed tiles
+    if (tid < ntg2 || (tid < F && S.j[tid] >= 0)) {
+      if (tid < ntg2) Wk.nn[S.targets[tid]] &= (Idx)~Ws_::kTarget;
+      if (tid < F && S.j[tid] >= 0) Wk.nn[min(S.c[tid], S.j[tid])] &= (Idx)~Ws_::kTarget;
+    }
     const int nd = S.n_dirty, ndt = nd <= kRoundMaxDirty ? nd : nt;
     if (dense) {
 #pragma unroll 1

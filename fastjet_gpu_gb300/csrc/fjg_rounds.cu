@@ -74,7 +74,8 @@ size_t bytes_of(const RoundConfig& c) {
   return c.slots ? round_smem_bytes<true>(c.tiles, c.cells, c.slots) : round_smem_bytes<false>(c.tiles, c.cells, 0);
 }
 
-static_assert(sizeof(RoundShared) < 10240, "fixed shared memory of a CTA");
+static_assert(round_smem_bytes<true>(1024, 1792, 2048) + 1024 <= 233472 / 2, "2048 slots: two CTAs per SM");
+static_assert(round_smem_bytes<true>(1024, 1792, 4096) <= 232448, "4096 slots: one CTA per SM");
 
 }  // namespace
 
