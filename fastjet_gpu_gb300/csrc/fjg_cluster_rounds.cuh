@@ -112,10 +112,11 @@ __device__ __forceinline__ bool rounds_event(const BatchArgs& A, int e) {
 }
 
 constexpr int kRoundSteps = 32;               // steps per round, at most (a lane each)
-constexpr int kRoundBytesPerParticle = 240;   // workspace
+constexpr int kRoundBytesPerParticle = 320;   // workspace (304, and events start at whole sectors)
 constexpr int kRoundMaxDirty = 384;
 constexpr int kRoundMaxTargets = 128;
-constexpr int kRoundSplit = 8;                // searches of a round, up to which several warps share each
+constexpr int kRoundSplit = 24;               // searches of a round, up to which several warps share each
+constexpr int kRoundParts = 5;                // warps that share one, at most
 constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, also in one row
 // range of the choice of steps, in units of R (see above): the first attempt at
 // an event, the second (the first for the largest anti-kt events), the last
@@ -126,6 +127,7 @@ constexpr int kRoundMaxCells = 3072;          // with the frame
 constexpr int kRoundFrame = 5;                // tiles around the grid: the range test's 1.5 R + R
 constexpr int kRoundDense = 4;                // live slots per tile from which a warp reads lists together
 constexpr int kRoundSmemMaxN = 4096;
+constexpr int kRoundThreadsWs = 512;          // threads per event with its slots in the workspace
 constexpr int kRoundSlotBytes = 36;           // shared memory per slot
 
 // One step, stored at the slot it removes.
@@ -150,10 +152,43 @@ __device__ __forceinline__ bool time_less(const RoundTime& x, const RoundTime& y
 
 constexpr unsigned kRoundNone = 0xffffffffu;  // a tile without slots (P as a bit pattern; P >= 0 orders as integer)
 
-// The event's state: what every round reads in shared memory (SM: events of up
-// to kRoundSmemMaxN particles, 36 bytes a slot, so that two CTAs share an SM) or
-// in the global workspace; what single slots need, the dead and the records
-// always in the workspace.
+// A slot's state in the workspace, by sectors: what windows are scanned for, what
+// a slot that gets a neighbour needs, the momentum, the rest.  (Separate arrays
+// took a cache line for each of the 17 words that a step writes: phase C of a
+// round took 14 kcycles at 50,000 particles.)
+struct alignas(16) RoundSlot {
+  float2 xy;   // rap32, phi32
+  float2 key;  // lower bounds of the key, and of its step's time (P)
+  float nhi;   // neighbour distance, upper bound
+  int nn;      // neighbour field
+  float wlo;   // weight, lower bound; negated: the upper bound is the next float up
+  int tile;    // kNone: taken
+  double2 pos;  // rapidity, azimuth
+  double tm;    // birth time M
+  int2 tl;      // birth time l, depth
+  double p[4];
+  double w;
+  float tlo;  // birth time's M, rounded down
+  int at;     // position in its tile's list
+  int parent;  // (output) what the slot was merged into, or its jet
+  int pad[3];
+};
+
+// What the step that removed a slot took: [0] c, [1] j.
+struct alignas(16) RoundDead {
+  float4 geo[2];  // rap32, phi32, wlo, threshold rounded up
+  int4 grp[2];    // groups of the dead of one tile with the same M and l: next group (by descending
+                  // M), its M rounded up (float), first member, l
+  RoundRec rec;
+  int next[2];    // next member
+  int pad[6];
+};
+static_assert(sizeof(RoundSlot) == 128 && sizeof(RoundDead) == 128, "whole sectors");
+
+// The event's state.  SM (events of up to kRoundSmemMaxN particles): what every
+// round reads is in shared memory, 36 bytes a slot, so that two CTAs share an
+// SM; what single slots need, the dead and the records are always in the
+// workspace: RoundSlot[N], RoundDead[N], then (not SM) lxy and members.
 template <bool SM>
 struct RoundWs {
   using Idx = typename std::conditional<SM, unsigned short, int>::type;  // slots, tiles, list positions
@@ -162,64 +197,66 @@ struct RoundWs {
   // neighbour field: slot, or kNoSlot; a target of this round; the key is the pair distance
   static constexpr int kSlotMask = SM ? 0x1fff : 0x1ffffff, kNoSlot = kSlotMask;
   static constexpr int kTarget = SM ? 0x4000 : 0x20000000, kPair = SM ? 0x8000 : 0x40000000;
-  float2* xy;     // [N] rap32, phi32
-  float2* key;    // [N] lower bounds of the key, and of its step's time (P)
-  float* nhi;     // [N] neighbour distance, upper bound
-  float* wlo;     // [N] weight, lower bound; negated: the upper bound is the next float up
-  Idx* nn;        // [N] neighbour field
-  Idx* tile;      // [N] kNone: taken
-  Idx* at;        // [N] position in its tile's list
-  Idx* members;   // [kRoom * N]
-  float2* lxy;    // [kRoom * N] coordinates in list order, read with consecutive lanes (not SM)
-  double2* pos;   // [N] rapidity, azimuth
-  float* tlo;     // [N] birth time's M, rounded down
-  double* tm;     // [N] birth time M
-  int2* tl;       // [N] birth time l, depth
-  int2* stamp;    // [N] round in which it was taken by a step, or given a new neighbour (SM: bits in S)
-  float4* dgeo;   // [2N] dead: rap32, phi32, wlo, threshold rounded up; 2b and 2b+1: what the step
-                  //      that removed slot b took
-  int4* dgrp;     // [2N] groups of the dead of one tile with the same M and l: next group (by descending
-                  //      M), its M rounded up (float), first member, l
-  int* dnext;     // [2N] next member
-  RoundRec* rec;  // [N]
+  RoundSlot* slots;
+  RoundDead* dead;
+  Idx* members;  // [kRoom * N]
+  float2* lxy;   // [kRoom * N] coordinates in list order, read with consecutive lanes (not SM)
+  float2 *sxy, *skey;  // (SM) the slots' state
+  float *snhi, *swlo;
+  Idx *snn, *stile, *sat;
+  __device__ __forceinline__ float2& xy(int s) const { return SM ? sxy[s] : slots[s].xy; }
+  __device__ __forceinline__ float2& key(int s) const { return SM ? skey[s] : slots[s].key; }
+  __device__ __forceinline__ float& nhi(int s) const { return SM ? snhi[s] : slots[s].nhi; }
+  __device__ __forceinline__ float& wlo(int s) const { return SM ? swlo[s] : slots[s].wlo; }
+  __device__ __forceinline__ Idx& nn(int s) const { return pick(snn, slots[s].nn, s); }
+  __device__ __forceinline__ Idx& tile(int s) const { return pick(stile, slots[s].tile, s); }
+  __device__ __forceinline__ Idx& at(int s) const { return pick(sat, slots[s].at, s); }
+  __device__ __forceinline__ double2& pos(int s) const { return slots[s].pos; }
+  __device__ __forceinline__ double& tm(int s) const { return slots[s].tm; }
+  __device__ __forceinline__ int2& tl(int s) const { return slots[s].tl; }
+  __device__ __forceinline__ float& tlo(int s) const { return slots[s].tlo; }
+  __device__ __forceinline__ double& p4(int q, int s) const { return slots[s].p[q]; }
+  __device__ __forceinline__ double& w(int s) const { return slots[s].w; }
+  // the dead: 2b and 2b+1, what the step that removed slot b took
+  __device__ __forceinline__ float4& dgeo(int i) const { return dead[i >> 1].geo[i & 1]; }
+  __device__ __forceinline__ int4& dgrp(int i) const { return dead[i >> 1].grp[i & 1]; }
+  __device__ __forceinline__ int& dnext(int i) const { return dead[i >> 1].next[i & 1]; }
+  __device__ __forceinline__ RoundRec& rec(int b) const { return dead[b].rec; }
   // coordinates of slot u, entry i of the lists
-  __device__ __forceinline__ float2 entry(int u, int i) const { return SM ? xy[u] : lxy[i]; }
+  __device__ __forceinline__ float2 entry(int u, int i) const { return SM ? sxy[u] : lxy[i]; }
   __device__ __forceinline__ void place(int i, int u, float2 g) const {
     members[i] = (Idx)u;
     if (!SM) lxy[i] = g;
   }
   __device__ __forceinline__ double dr2(int s, int t) const {
-    const double2 a = pos[s], b = pos[t];
+    const double2 a = pos(s), b = pos(t);
     return dr2_64(a.x, a.y, b.x, b.y);
   }
+
+ private:
+  __device__ static __forceinline__ unsigned short& pick(unsigned short* a, int&, int s) { return a[s]; }
+  __device__ static __forceinline__ int& pick(int*, int& x, int) { return x; }
 };
 
 template <bool SM>
 __device__ __forceinline__ RoundWs<SM> round_ws(unsigned char* base, unsigned char* smem, int N, int cap) {
-  RoundWs<SM> W;
-  using Idx = typename RoundWs<SM>::Idx;
+  RoundWs<SM> W{};
   const int64_t n = N;
-  W.dgeo = reinterpret_cast<float4*>(base);
-  W.dgrp = reinterpret_cast<int4*>(base + 32 * n);
-  W.rec = reinterpret_cast<RoundRec*>(base + 64 * n);
-  W.pos = reinterpret_cast<double2*>(base + 96 * n);
-  W.tm = reinterpret_cast<double*>(base + 112 * n);
-  W.tl = reinterpret_cast<int2*>(base + 120 * n);
-  W.stamp = reinterpret_cast<int2*>(base + 128 * n);
-  W.dnext = reinterpret_cast<int*>(base + 136 * n);
-  W.lxy = reinterpret_cast<float2*>(base + 144 * n);
-  W.tlo = reinterpret_cast<float*>(base + 176 * n);
-  // 180 n bytes, and 4 n unused; then, in the workspace, 52 n more
-  unsigned char* p = SM ? smem : base + 184 * n;
-  const int64_t m = SM ? cap : N;
-  W.xy = reinterpret_cast<float2*>(p);
-  W.key = W.xy + m;
-  W.nhi = reinterpret_cast<float*>(W.key + m);
-  W.wlo = W.nhi + m;
-  W.nn = reinterpret_cast<Idx*>(W.wlo + m);
-  W.tile = W.nn + m;
-  W.at = W.tile + m;
-  W.members = W.at + m;
+  W.slots = reinterpret_cast<RoundSlot*>(base);
+  W.dead = reinterpret_cast<RoundDead*>(base + 128 * n);
+  if (!SM) {
+    W.lxy = reinterpret_cast<float2*>(base + 256 * n);
+    W.members = reinterpret_cast<typename RoundWs<SM>::Idx*>(base + 288 * n);  // to 304 n
+    return W;
+  }
+  W.sxy = reinterpret_cast<float2*>(smem);
+  W.skey = W.sxy + cap;
+  W.snhi = reinterpret_cast<float*>(W.skey + cap);
+  W.swlo = W.snhi + cap;
+  W.snn = reinterpret_cast<typename RoundWs<SM>::Idx*>(W.swlo + cap);
+  W.stile = W.snn + cap;
+  W.sat = W.stile + cap;
+  W.members = W.sat + cap;
   return W;
 }
 
@@ -240,10 +277,11 @@ struct RoundShared {
   float r2hi;  // R^2 rounded up, a little more
   int tiles, cells, slots;  // room
   double rmin, inv_side_r, inv_side_phi;
+  float rmin32, side_r, side_phi;
   int nrap, nphi, sh, nt, pw;  // tile (u, v) is u << sh | v; nt = nrap << sh
   int lut[16];                 // 2^16 / k, rounded up
-  double red[3][16];
-  int scan_tmp[16];
+  double red[3][24];
+  int scan_tmp[24];
   int event, overflow;
   // conflict flags of a round's phases A, B and D: each is read after the
   // barrier that closes its phase and written again only a round later, so
@@ -261,19 +299,19 @@ struct RoundShared {
   double M[kRoundSteps], key[kRoundSteps], thr_c[kRoundSteps], thr_j[kRoundSteps];
   double phi[kRoundSteps], rap[kRoundSteps], w[kRoundSteps], p4[4][kRoundSteps];
   int targets[kRoundMaxTargets];
-  Cert part[kRoundSplit][4];  // searches shared by several warps
-  int parts_done[kRoundSplit];
+  int parts_done[kRoundSplit];  // searches shared by several warps
   unsigned short cand[kRoundMaxCand];  // tiles
   unsigned short dirty[kRoundMaxDirty];
   unsigned dirty_bits[kRoundMaxTiles / 32];
-  // SM: slots taken by a step of this round, and given a new neighbour
+  // slots taken by a step of this round, and given a new neighbour (round_bit)
   unsigned taken[kRoundSmemMaxN / 32], claimed[kRoundSmemMaxN / 32];
 };
 
 // After it, `cells` minima of P with the grid's frame (kRoundFrame on each side;
 // columns of the frame repeat the tiles across the azimuth seam, so that a
 // neighbourhood is read without wrapping) and 5-tile row minima, then `tiles`
-// entries of the per-tile arrays, then the slots.
+// entries of the per-tile arrays, then the slots, or (not SM) the parts
+// of shared searches and a word per thread.
 __host__ __device__ constexpr size_t round_tile_bytes(int tiles, int cells) {
   return ((size_t)cells * 12 + (size_t)tiles * 22 + 16 + 15) & ~size_t(15);
 }
@@ -287,7 +325,8 @@ __host__ __device__ constexpr size_t round_slots_at(int tiles, int cells) {
 }
 template <bool SM>
 __host__ __device__ constexpr size_t round_smem_bytes(int tiles, int cells, int slots) {
-  return round_slots_at<SM>(tiles, cells) + (size_t)slots * kRoundSlotBytes;
+  return round_slots_at<SM>(tiles, cells) +
+         (SM ? (size_t)slots * kRoundSlotBytes : sizeof(Cert) * kRoundSplit * kRoundParts + sizeof(int) * kRoundThreadsWs);
 }
 
 template <bool SM>
@@ -303,6 +342,8 @@ struct RoundCtx {
   Idx* slot;       // [nt] the slot of the minimum
   unsigned short* beside;  // [nt] the tile of its partner, or its own (not SM)
   Idx* start;      // [nt + 1]
+  Cert* part;      // [kRoundSplit * kRoundParts] (not SM)
+  int* shift;      // [threads] for_tiles (not SM)
   RoundWs<SM> W;
 };
 
@@ -322,6 +363,8 @@ __device__ __forceinline__ RoundCtx<SM> round_ctx() {
   C.slot = reinterpret_cast<typename RoundCtx<SM>::Idx*>(C.head_m + tiles);
   C.start = C.slot + tiles;
   C.beside = reinterpret_cast<unsigned short*>(C.start + tiles + 2);
+  C.part = reinterpret_cast<Cert*>(smem_raw + round_slots_at<SM>(tiles, cells));
+  C.shift = reinterpret_cast<int*>(C.part + kRoundSplit * kRoundParts);
   C.W = round_ws<SM>(C.S->ws, smem_raw + round_slots_at<SM>(tiles, cells), C.S->X.N, C.S->slots);
   return C;
 }
@@ -335,6 +378,9 @@ __device__ __forceinline__ int round_v(const RoundShared& S, double phi) {
   const int v = (int)floor(phi * S.inv_side_phi);
   return v < 0 ? 0 : (v >= S.nphi ? S.nphi - 1 : v);
 }
+
+// R^2 and more than the FP32 distances' error.
+__device__ __forceinline__ float round_far2(const RoundShared& S) { return S.r2hi * 1.001f + 1e-6f; }
 
 // A box of tiles: nu rows from u0, nv columns from v0 (wrapping; nv <= 9).
 struct RoundBox {
@@ -370,47 +416,76 @@ __device__ __forceinline__ int box_tile(const RoundShared& S, const RoundBox& b,
   return ((b.u0 + du) << S.sh) + v;
 }
 
+// Squared distance of a point to tile (u, v); the outermost rows hold what lies
+// beyond them.
+__device__ __forceinline__ float tile_d2(const RoundShared& S, float2 g, int u, int v) {
+  const float lo = S.rmin32 + u * S.side_r;
+  float dr = 0.0f;
+  if (u > 0) dr = fmaxf(dr, lo - g.x);
+  if (u < S.nrap - 1) dr = fmaxf(dr, g.x - lo - S.side_r);
+  float dp = fabsf(g.y - (v + 0.5f) * S.side_phi);
+  dp = fmaxf(fminf(dp, kTwoPiF - dp) - 0.5f * S.side_phi, 0.0f);
+  return dr * dr + dp * dp;
+}
+
 // fn(slot, load(slot, coordinates)) for every list entry of the box's tiles k0 ..
 // n-1 (the functions hold no warp collectives).  Lists in shared memory: a group
 // of G lanes (8 or 32, the same in the whole warp), a lane per tile, two members
-// at a time.  Lists in the workspace: a warp, `sub` lanes per tile (a power of
-// two near the mean list length, so that most lists are gone over at once) and
-// five tiles a lane, so that five loads are in flight: a window of short lists
-// costs two dependent loads, not two for every pair of members.  List lengths
-// are bounded by the tile's room.
+// at a time.  Lists in the workspace: a warp; a lane per tile first, which leaves
+// out the tiles further than R from p and from q and adds the lengths up; then the lists as one sequence, every lane an
+// entry of it, three at a time so that their loads are in flight together.
+// (Lanes given to tiles, 32 / length tiles at a time, ran four times the
+// instructions: lists differ in length.)  Lengths are bounded by the tile's room.
 template <bool SM, class Load, class Fn>
-__device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox& b, int k0, int n, int G, int sub,
-                                          Load load, Fn fn) {
+__device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox& b, int k0, int n, int G, float2 p,
+                                          float2 q, Load load, Fn fn) {
   const RoundShared& S = *C.S;
   constexpr int kNone = RoundWs<SM>::kNone;
   if (!SM) {
-    constexpr int B = 5;
-    const int lane = threadIdx.x & 31, first = lane & (sub - 1), per = 32 / sub;
+    constexpr int B = 3;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1, upto = below | (1u << lane);
+    const float far2 = round_far2(S);
+    int* shift = C.shift + (threadIdx.x & ~31);
 #pragma unroll 1
-    for (k0 += lane / sub; k0 < n; k0 += B * per) {
-      int st[B], ln[B], most = 0;
+    for (; k0 < n; k0 += 32) {
+      const int k = k0 + lane, t = box_tile(S, b, k < n ? k : k0), st = C.start[t];
+      const int u = t >> S.sh, v = t & ((1 << S.sh) - 1);
+      int ln = 0;
+      if (k < n && fminf(tile_d2(S, p, u, v), tile_d2(S, q, u, v)) <= far2)
+        ln = min(C.count[t], (int)C.start[t + 1] - st);
+      int end = ln;
 #pragma unroll
-      for (int q = 0; q < B; ++q) {
-        const int k = k0 + q * per, t = box_tile(S, b, k < n ? k : k0);
-        st[q] = C.start[t];
-        ln[q] = k < n ? min(C.count[t], (int)C.start[t + 1] - st[q]) : 0;
-        most = max(most, ln[q]);
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(kFull, end, o);
+        if (lane >= o) end += x;
       }
+      const int total = __shfl_sync(kFull, end, 31), begin = end - ln;
+      const unsigned some = __ballot_sync(kFull, ln > 0);
+      if (ln > 0) shift[__popc(some & below)] = st - begin;
+      __syncwarp();
+      int before = -1;  // lists that begin before this point of the sequence
 #pragma unroll 1
-      for (int i = first; i < most; i += sub) {
+      for (int base = 0; base < total; base += 32 * B) {
         int u[B];
         float2 g[B];
         decltype(load(0, make_float2(0.0f, 0.0f))) d[B];
 #pragma unroll
-        for (int q = 0; q < B; ++q) {
-          u[q] = i < ln[q] ? (int)C.W.members[st[q] + i] : kNone;
-          g[q] = C.W.lxy[st[q] + (i < ln[q] ? i : 0)];
+        for (int c = 0; c < B; ++c) {
+          const unsigned at = (unsigned)(begin - base - 32 * c);
+          const unsigned starts = __reduce_or_sync(kFull, ln > 0 && at < 32u ? 1u << at : 0u);
+          const int i = base + 32 * c + lane, r = before + __popc(starts & upto);
+          before += __popc(starts);
+          const int e = i < total ? shift[r] + i : 0;
+          u[c] = i < total ? (int)C.W.members[e] : kNone;
+          g[c] = C.W.lxy[e];
         }
 #pragma unroll
-        for (int q = 0; q < B; ++q) d[q] = load(u[q] != kNone ? u[q] : 0, g[q]);
+        for (int c = 0; c < B; ++c) d[c] = load(u[c] != kNone ? u[c] : 0, g[c]);
 #pragma unroll
-        for (int q = 0; q < B; ++q)
-          if (u[q] != kNone) fn(u[q], d[q]);
+        for (int c = 0; c < B; ++c)
+          if (u[c] != kNone) fn(u[c], d[c]);
+        __syncwarp();
       }
     }
   } else {
@@ -422,7 +497,7 @@ __device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox&
       for (int i = 0; i < m; i += 2) {
         const int u0 = C.W.members[st + i], u1 = i + 1 < m ? (int)C.W.members[st + i + 1] : kNone;
         const int v0 = u0 != kNone ? u0 : 0, v1 = u1 != kNone ? u1 : v0;
-        const auto d0 = load(v0, C.W.xy[v0]), d1 = load(v1, C.W.xy[v1]);
+        const auto d0 = load(v0, C.W.xy(v0)), d1 = load(v1, C.W.xy(v1));
         if (u0 != kNone) fn(u0, d0);
         if (u1 != kNone) fn(u1, d1);
       }
@@ -432,8 +507,8 @@ __device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox&
 }
 
 template <bool SM, class Load, class Fn>
-__device__ __forceinline__ void for_box(const RoundCtx<SM>& C, const RoundBox& b, int G, int sub, Load load, Fn fn) {
-  for_tiles(C, b, 0, b.nu * b.nv, G, sub, load, fn);
+__device__ __forceinline__ void for_box(const RoundCtx<SM>& C, const RoundBox& b, int G, float2 p, Load load, Fn fn) {
+  for_tiles(C, b, 0, b.nu * b.nv, G, p, p, load, fn);
 }
 
 // Combination of certificates over groups of G lanes (all lanes call).
@@ -469,15 +544,18 @@ __device__ __forceinline__ void round_target(RoundShared& S, int t) {
   if (k < kRoundMaxTargets) S.targets[k] = t;
 }
 
-// True for the first caller of a round: slot s is taken by a step (claim = 0),
-// or given a new neighbour (1).
+// A slot's bit of S.taken and S.claimed: its own, or (not SM) one of 4096 by a
+// hash.  A bit shared with another slot costs time, not correctness: a step waits
+// for the next round, a slot is searched.
 template <bool SM>
-__device__ __forceinline__ bool round_first(const RoundCtx<SM>& C, int s, int round, int claim) {
-  if (SM) {
-    const unsigned bit = 1u << (s & 31);
-    return !(atomicOr((claim ? C.S->claimed : C.S->taken) + (s >> 5), bit) & bit);
-  }
-  return atomicExch(claim ? &C.W.stamp[s].y : &C.W.stamp[s].x, round) != round;
+__device__ __forceinline__ int round_bit(int s) {
+  return SM ? s : (int)(((unsigned)s * 2654435761u) >> 20);
+}
+
+// True for the first caller of a round.
+__device__ __forceinline__ bool round_first(unsigned* bits, int b) {
+  const unsigned bit = 1u << (b & 31);
+  return !(atomicOr(bits + (b >> 5), bit) & bit);
 }
 
 // The routines that a round's lanes call for single slots stay out of line: the
@@ -487,7 +565,9 @@ __device__ __forceinline__ bool round_first(const RoundCtx<SM>& C, int s, int ro
 // Slot t's neighbour nn with distance interval [lo, hi]: neighbour, key and P;
 // the tile is marked as changed.  The FP32 filter's interval is wide for close
 // pairs (its bound is absolute), which FP64 settles, so that keys compare well:
-// a neighbour's interval is narrower than 2^-16 of it.  `keep`: kTarget, if the
+// a neighbour's interval is narrower than 2^-16 of it.  Beyond R there is no
+// neighbour: the lighter of such a pair is promoted before the pair's turn, and
+// all that have c as their neighbour are found within R of c.  `keep`: kTarget, if the
 // other groups of this phase are to leave t alone.  What may be needed is
 // loaded at once.
 template <bool SM>
@@ -496,24 +576,24 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi, int ke
   const RoundCtx<SM> C = round_ctx<SM>();
   const EventCtx& X = C.S->X;
   const int n = nn < 0 ? t : nn;
-  const float w = C.W.wlo[t], tlo = C.W.tlo[t], wn = C.W.wlo[n], tn = C.W.tlo[n];
-  const double2 pt = C.W.pos[t], pn = C.W.pos[n];
-  round_dirty(*C.S, C.W.tile[t]);
+  const float w = C.W.wlo(t), tlo = C.W.tlo(t), wn = C.W.wlo(n), tn = C.W.tlo(n);
+  const double2 pt = C.W.pos(t), pn = C.W.pos(n);
+  round_dirty(*C.S, C.W.tile(t));
   float klo = round_wlo(w), p = fmaxf(klo, tlo);
   int field = Ws_::kNoSlot;
-  if (nn < 0) {
-    hi = __int_as_float(0x7f800000);
+  if (nn >= 0 && hi - lo > lo * 0x1p-16f) {
+    const double d = dr2_64(pt.x, pt.y, pn.x, pn.y);
+    lo = __double2float_rd(d);
+    hi = __double2float_ru(d);
+  }
+  if (nn < 0 || lo > C.S->r2hi) {
+    hi = C.S->r2hi;
   } else {
-    if (hi - lo > lo * 0x1p-16f) {
-      const double d = dr2_64(pt.x, pt.y, pn.x, pn.y);
-      lo = __double2float_rd(d);
-      hi = __double2float_ru(d);
-    }
     float khi;
     int kind = key_interval(klo, round_whi(w), round_wlo(wn), round_whi(wn), lo, hi, X.ilo, X.ihi, klo, khi);
     if (kind < 0) {
-      const double w64 = X.g.at(kW, t);
-      const double dp = pair_distance(w64, X.g.at(kW, nn), dr2_64(pt.x, pt.y, pn.x, pn.y), X.inv_r2);
+      const double w64 = C.W.w(t);
+      const double dp = pair_distance(w64, C.W.w(nn), dr2_64(pt.x, pt.y, pn.x, pn.y), X.inv_r2);
       kind = dp < w64 ? 1 : 0;
       klo = __double2float_rd(kind ? dp : w64);
     }
@@ -521,9 +601,9 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi, int ke
     if (kind) p = fmaxf(p, tn);
     field = nn | (kind ? Ws_::kPair : 0);
   }
-  C.W.key[t] = make_float2(klo, p);
-  C.W.nhi[t] = hi;
-  C.W.nn[t] = (typename Ws_::Idx)(field | keep);
+  C.W.key(t) = make_float2(klo, p);
+  C.W.nhi(t) = hi;
+  C.W.nn(t) = (typename Ws_::Idx)(field | keep);
 }
 
 // Slot t's neighbour by the exact minimum (dR2, label) over its window (whole
@@ -531,13 +611,13 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi, int ke
 template <bool SM>
 __device__ __noinline__ int round_exact(int t, float u1) {
   const RoundCtx<SM> C = round_ctx<SM>();
-  const int tile = C.W.tile[t];
+  const int tile = C.W.tile(t);
   const RoundBox b = round_box(*C.S, tile, tile);
-  const float2 gt = C.W.xy[t];
+  const float2 gt = C.W.xy(t);
   const Bound bd = C.S->X.bd;
   unsigned long long bk = ~0ull;
   int bi = 0x7fffffff;
-  for_box(C, b, 32, 8, [&](int, float2 g) { return g; },
+  for_box(C, b, 32, gt, [&](int, float2 g) { return g; },
           [&](int u, float2 gu) {
             float l, h;
             dr2_32(gt.x, gt.y, gu.x, gu.y, bd, l, h);
@@ -572,40 +652,42 @@ __device__ __forceinline__ void round_settle(bool have, bool first, int t, const
 
 // The certificate of search `item` from its parts, each done by a warp (parts >
 // 1; every lane calls): true for the last one, which holds the whole.
-__device__ __forceinline__ bool round_join(RoundShared& S, Cert& c, int item, int part, int parts) {
+template <bool SM>
+__device__ __forceinline__ bool round_join(const RoundCtx<SM>& C, Cert& c, int item, int part, int parts) {
+  Cert* all = C.part + item * kRoundParts;
   const int lane = threadIdx.x & 31;
   int done = 0;
   if (lane == 0) {
-    S.part[item][part] = c;
+    all[part] = c;
     __threadfence_block();
-    done = atomicAdd(&S.parts_done[item], 1);
+    done = atomicAdd(&C.S->parts_done[item], 1);
   }
   if (__shfl_sync(kFull, done, 0) != parts - 1) return false;
   __threadfence_block();
-  c = cert_warp(lane < parts ? S.part[item][lane] : cert_empty());
+  c = cert_warp(lane < parts ? all[lane] : cert_empty());
   return true;
 }
 
 // Slot t's neighbour in its window, and its key (groups of G lanes; or one of
 // several warps of search `item`).
 template <bool SM>
-__device__ __noinline__ void round_search(bool have, int t, int G, int sub, int item, int part, int parts) {
+__device__ __noinline__ void round_search(bool have, int t, int G, int item, int part, int parts) {
   const RoundCtx<SM> C = round_ctx<SM>();
-  const int tile = have ? (int)C.W.tile[t] : 0;
+  const int tile = have ? (int)C.W.tile(t) : 0;
   RoundBox b = round_box(*C.S, tile, tile);
   if (!have) b.nu = 0;
-  const float2 gt = C.W.xy[t];
+  const float2 gt = C.W.xy(t);
   const Bound bd = C.S->X.bd;
   Cert x = cert_empty();
   const int nb = b.nu * b.nv;
-  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub, [&](int, float2 g) { return g; },
+  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, gt, gt, [&](int, float2 g) { return g; },
           [&](int u, float2 gu) {
             float lo, hi;
             dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
             if (u != t) cert_add(x, lo, hi, u);
           });
   x = cert_group(x, G);
-  if (parts > 1 && !round_join(*C.S, x, item, part, parts)) return;
+  if (parts > 1 && !round_join(C, x, item, part, parts)) return;
   round_settle<SM>(have, (threadIdx.x & (G - 1)) == 0, t, x, RoundWs<SM>::kTarget);
 }
 
@@ -614,17 +696,17 @@ __device__ __noinline__ void round_search(bool have, int t, int G, int sub, int 
 // time: whichever of y's words are seen, what is kept is closer than before,
 // and of two that claim y the second has it searched.
 template <bool SM>
-__device__ __noinline__ void round_offer(int y, int a, float lo, float hi, float nhi, int round) {
+__device__ __noinline__ void round_offer(int y, int a, float lo, float hi, float nhi) {
   using Ws_ = RoundWs<SM>;
   const RoundCtx<SM> C = round_ctx<SM>();
   if (!(hi < nhi * (1.0f - 0x1p-14f))) {
-    const int cn = *(volatile typename Ws_::Idx*)(C.W.nn + y) & Ws_::kSlotMask;
+    const int cn = *(volatile typename Ws_::Idx*)&C.W.nn(y) & Ws_::kSlotMask;
     if (cn != Ws_::kNoSlot) {
       const double da = C.W.dr2(y, a), dc = C.W.dr2(y, cn);
       if (!(da < dc || (da == dc && a < cn))) return;
     }
   }
-  if (round_first(C, y, round, 1))
+  if (round_first(C.S->claimed, round_bit<SM>(y)))
     round_set<SM>(y, a, lo, hi, 0);
   else
     round_target(*C.S, y);  // (phase E)
@@ -636,24 +718,22 @@ template <bool SM>
 __device__ __noinline__ bool round_d1_exact(int x, int y, double thr, double M) {
   const RoundCtx<SM> C = round_ctx<SM>();
   const EventCtx& X = C.S->X;
-  const double wx = X.g.at(kW, x), wy = X.g.at(kW, y), ty = C.W.tm[y];
+  const double wx = C.W.w(x), wy = C.W.w(y), ty = C.W.tm(y);
   const double d = pair_distance(wx, wy, C.W.dr2(x, y), X.inv_r2);
   return d <= thr && d <= fmin(wx, wy) && !(ty > M);
 }
 
-// The minimum of tile t into its cell and the frame's copies of it.
+// The minimum of tile t (slot: P, neighbour field) into its cell and the frame's
+// copies of it.
 template <bool SM>
-__device__ __forceinline__ void round_store_min(const RoundCtx<SM>& C, int t, unsigned p, int slot) {
+__device__ __forceinline__ void round_store_min(const RoundCtx<SM>& C, int t, unsigned p, int slot, int nn) {
   const RoundShared& S = *C.S;
   const int u = t >> S.sh, v = t & ((1 << S.sh) - 1);
   unsigned* row = C.tmin + (u + kRoundFrame) * S.pw + kRoundFrame;
   C.slot[t] = (typename RoundCtx<SM>::Idx)slot;
   if (!SM) {
     int beside = t;
-    if (slot >= 0) {
-      const int f = C.W.nn[slot];
-      if (f & RoundWs<SM>::kPair) beside = C.W.tile[f & RoundWs<SM>::kSlotMask];
-    }
+    if (slot >= 0 && (nn & RoundWs<SM>::kPair)) beside = C.W.tile(nn & RoundWs<SM>::kSlotMask);
     C.beside[t] = (unsigned short)beside;
   }
   row[v] = p;
@@ -678,7 +758,7 @@ __device__ __noinline__ void round_summary_warp(int t) {
   const int lane = threadIdx.x & 31;
   const int st = C.start[t], m = min(C.count[t], (int)C.start[t + 1] - st);
   float2 best = make_float2(0.0f, 0.0f);
-  int slot = -1, out = 0;
+  int slot = -1, nn = 0, out = 0;
 #pragma unroll 1
   for (int i0 = 0; i0 < m; i0 += 32) {
     const int i = i0 + lane;
@@ -689,12 +769,14 @@ __device__ __noinline__ void round_summary_warp(int t) {
       const int p = out + __popc(ball & ((1u << lane) - 1));
       if (p != i) {
         C.W.place(st + p, u, gu);
-        C.W.at[u] = (Idx)p;
+        C.W.at(u) = (Idx)p;
       }
-      const float2 k = C.W.key[u];
+      const float2 k = C.W.key(u);
+      const int f = C.W.nn(u);
       if (round_before(k, u, best, slot)) {
         best = k;
         slot = u;
+        nn = f;
       }
     }
     out += __popc(ball);
@@ -705,8 +787,9 @@ __device__ __noinline__ void round_summary_warp(int t) {
   const unsigned k = slot >= 0 && p == pb ? __float_as_uint(best.x) : kRoundNone;
   const unsigned kb = __reduce_min_sync(kFull, k);
   const unsigned sb = __reduce_min_sync(kFull, slot >= 0 && p == pb && k == kb ? (unsigned)slot : kRoundNone);
-  if (lane == 0) {
-    round_store_min(C, t, pb, (int)sb);
+  const unsigned win = __ballot_sync(kFull, slot >= 0 && (unsigned)slot == sb);
+  if (lane == (win ? __ffs(win) - 1 : 0)) {
+    round_store_min(C, t, pb, (int)sb, nn);
     C.count[t] = out;
   }
 }
@@ -725,16 +808,16 @@ __device__ __noinline__ void round_summary_thread(int t) {
     if (u == RoundWs<SM>::kNone) continue;
     if (out != i) {
       C.W.place(st + out, u, C.W.entry(0, st + i));
-      C.W.at[u] = (Idx)out;
+      C.W.at(u) = (Idx)out;
     }
     ++out;
-    const float2 k = C.W.key[u];
+    const float2 k = C.W.key(u);
     if (round_before(k, u, best, slot)) {
       best = k;
       slot = u;
     }
   }
-  round_store_min(C, t, slot >= 0 ? __float_as_uint(best.y) : kRoundNone, slot);
+  round_store_min(C, t, slot >= 0 ? __float_as_uint(best.y) : kRoundNone, slot, slot >= 0 ? (int)C.W.nn(slot) : 0);
   C.count[t] = out;
 }
 
@@ -753,8 +836,8 @@ __device__ __noinline__ void round_lists(int n) {
   __syncthreads();
 #pragma unroll 1
   for (int s = tid; s < N; s += T) {
-    const int t = C.W.tile[s];
-    if (t != kNone) C.W.at[s] = (Idx)atomicAdd(&C.count[t], 1);
+    const int t = C.W.tile(s);
+    if (t != kNone) C.W.at(s) = (Idx)atomicAdd(&C.count[t], 1);
   }
   __syncthreads();
   int carry = 0;
@@ -784,8 +867,8 @@ __device__ __noinline__ void round_lists(int n) {
   __syncthreads();
 #pragma unroll 1
   for (int s = tid; s < N; s += T) {
-    const int t = C.W.tile[s];
-    if (t != kNone) C.W.place(C.start[t] + C.W.at[s], s, C.W.xy[s]);
+    const int t = C.W.tile(s);
+    if (t != kNone) C.W.place(C.start[t] + C.W.at(s), s, C.W.xy(s));
   }
   __syncthreads();
 }
@@ -806,12 +889,12 @@ __device__ __noinline__ void round_bury(bool have, int tile, int idx, float4 g, 
     const unsigned same = __match_any_sync(kFull, todo ? tile : -1 - (int)(threadIdx.x & 31));
     if (todo && (threadIdx.x & 31) == (unsigned)(__ffs(same) - 1)) {
       todo = false;
-      C.W.dgeo[idx] = g;
+      C.W.dgeo(idx) = g;
       int prev = -1, x = C.head[tile];
       float xm = C.head_m[tile];
 #pragma unroll 1
       for (int guard = 0; x >= 0 && xm > m_hi && guard < most; ++guard) {
-        const int4 r = C.W.dgrp[x];
+        const int4 r = C.W.dgrp(x);
         prev = x;
         x = r.x;
         xm = __int_as_float(r.y);
@@ -821,23 +904,23 @@ __device__ __noinline__ void round_bury(bool have, int tile, int idx, float4 g, 
       bool found = false;
 #pragma unroll 1
       for (int guard = 0; q >= 0 && qm == m_hi && !found && guard < most; ++guard) {
-        const int4 r = C.W.dgrp[q];
+        const int4 r = C.W.dgrp(q);
         if (r.w == l) {
-          C.W.dnext[idx] = r.z;
-          C.W.dgrp[q].z = idx;
+          C.W.dnext(idx) = r.z;
+          C.W.dgrp(q).z = idx;
           found = true;
         }
         q = r.x;
         qm = __int_as_float(r.y);
       }
       if (!found) {
-        C.W.dnext[idx] = -1;
-        C.W.dgrp[idx] = make_int4(x, __float_as_int(xm), idx, l);
+        C.W.dnext(idx) = -1;
+        C.W.dgrp(idx) = make_int4(x, __float_as_int(xm), idx, l);
         if (prev < 0) {
           C.head[tile] = idx;
           C.head_m[tile] = m_hi;
         } else {
-          *reinterpret_cast<int2*>(C.W.dgrp + prev) = make_int2(idx, __float_as_int(m_hi));
+          *reinterpret_cast<int2*>(&C.W.dgrp(prev)) = make_int2(idx, __float_as_int(m_hi));
         }
       }
     }
@@ -852,26 +935,26 @@ template <bool SM>
 __device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) {
   const RoundCtx<SM> C = round_ctx<SM>();
   const EventCtx& X = C.S->X;
-  const float m_lo = __double2float_rd(M), wa = round_wlo(C.W.wlo[a]), r2hi = C.S->r2hi, ilo = X.ilo;
-  const float2 ga = C.W.xy[a];
+  const float m_lo = __double2float_rd(M), wa = round_wlo(C.W.wlo(a)), r2hi = C.S->r2hi, ilo = X.ilo;
+  const float2 ga = C.W.xy(a);
   const Bound bd = X.bd;
   bool bad = false;
 #pragma unroll 1
   for (int guard = 0; x >= 0 && guard < 2 * X.N; ++guard) {
-    const int4 r = C.W.dgrp[x];
+    const int4 r = C.W.dgrp(x);
     if (r.w != l) {
       int y = r.z;
 #pragma unroll 1
       for (int g2 = 0; y >= 0 && g2 < 2 * X.N; ++g2) {
-        const float4 dg = C.W.dgeo[y];
+        const float4 dg = C.W.dgeo(y);
         float lo, hi;
         dr2_32(dg.x, dg.y, ga.x, ga.y, bd, lo, hi);
         const float plo = __fmul_rd(__fmul_rd(__fmul_rd(fminf(wa, dg.z), lo), ilo), 0.99999976158142089844f);
         if (lo <= r2hi && !(plo > dg.w)) {
-          const RoundRec q = C.W.rec[y >> 1];
+          const RoundRec q = C.W.rec(y >> 1);
           bad |= time_less(RoundTime{M, l, depth}, RoundTime{q.M, q.l, q.depth});
         }
-        y = C.W.dnext[y];
+        y = C.W.dnext(y);
       }
     }
     if (__int_as_float(r.y) < m_lo) break;
@@ -898,7 +981,7 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
       for (int i0 = 0; i0 < m0; i0 += 32) {
         const bool have = i0 + lane < m0;
         const int t = C.W.members[st0 + (have ? i0 + lane : i0)];
-        const float2 gt = C.W.xy[t];
+        const float2 gt = C.W.xy(t);
         Cert c = cert_empty();
 #pragma unroll 1
         for (int k = 0; k < nb; ++k) {
@@ -930,10 +1013,10 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
     const bool have = t < N;
     Cert c = cert_empty();
     if (have) {
-      const int tile = C.W.tile[t];
+      const int tile = C.W.tile(t);
       const RoundBox b = round_box(S, tile, tile);
       const int nb = b.nu * b.nv;
-      const float2 gt = C.W.xy[t];
+      const float2 gt = C.W.xy(t);
 #pragma unroll 1
       for (int k = 0; k < nb; ++k) {
         const int tt = box_tile(S, b, k);
@@ -963,13 +1046,13 @@ __device__ __forceinline__ float plain_dr2(float2 a, float2 b) {
 // Phase B for the steps, by groups of G lanes: D1, and the slots whose neighbour
 // is taken.  With few steps their windows are cut in parts.
 template <bool SM>
-__device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int G, int sub, int parts) {
+__device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int G, int parts) {
   using Ws_ = RoundWs<SM>;
   RoundShared& S = *C.S;
   const Ws_& Wk = C.W;
   const int lane = threadIdx.x & 31;
   const Bound bd = S.X.bd;
-  const float ilo = S.X.ilo, r2hi = S.r2hi, far2 = r2hi * 1.001f + 1e-6f;
+  const float ilo = S.X.ilo, r2hi = S.r2hi, far2 = round_far2(S);
 #pragma unroll 1
   for (;;) {
     int i = 0;
@@ -998,13 +1081,13 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
     };
     bool bad = false;
     const int nb = b.nu * b.nv;
-    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub,
-            [&](int y, float2 g) { return Slot{g, Wk.wlo[y], Wk.nn[y]}; },
+    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, gc, gj,
+            [&](int y, float2 g) { return Slot{g, Wk.wlo(y), Wk.nn(y)}; },
             [&](int y, const Slot& s) {
               if (y == c || y == j) return;
               const int nn = s.nn & Ws_::kSlotMask;
               if (nn == c || (j >= 0 && nn == j)) {
-                Wk.nn[y] = (typename Ws_::Idx)(s.nn | Ws_::kTarget);
+                Wk.nn(y) = (typename Ws_::Idx)(s.nn | Ws_::kTarget);
                 round_target(S, y);
               }
               // beyond R of c and of j (the FP32 distance is good to 1e-5 there)?
@@ -1028,7 +1111,7 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
 
 // Phase D for one step that made jet a (groups of G lanes): the jet's window.
 template <bool SM>
-__device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, int i, int round, int G, int sub,
+__device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, int i, int G,
                                               int part, int parts) {
   using Ws_ = RoundWs<SM>;
   RoundShared& S = *C.S;
@@ -1047,18 +1130,18 @@ __device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, 
   };
   Cert ca = cert_empty();
   const int nb = b.nu * b.nv;
-  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, sub,
-          [&](int y, float2 g) { return Slot{g, Wk.nhi[y], Wk.nn[y]}; },
+  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, ga, ga,
+          [&](int y, float2 g) { return Slot{g, Wk.nhi(y), Wk.nn(y)}; },
           [&](int y, const Slot& s) {
             if (y == a) return;
             float lo, hi;
             dr2_32(s.g.x, s.g.y, ga.x, ga.y, bd, lo, hi);
             cert_add(ca, lo, hi, y);
             // not closer, or searched anyway?
-            if (!(lo > s.nhi) && !(s.nn & Ws_::kTarget)) round_offer<SM>(y, a, lo, hi, s.nhi, round);
+            if (!(lo > s.nhi) && !(s.nn & Ws_::kTarget)) round_offer<SM>(y, a, lo, hi, s.nhi);
           });
   ca = cert_group(ca, G);
-  if (parts > 1 && !round_join(S, ca, i, part, parts)) return;
+  if (parts > 1 && !round_join(C, ca, i, part, parts)) return;
   round_settle<SM>(have, (lane & (G - 1)) == 0, a, ca, Ws_::kTarget);
 }
 
@@ -1080,7 +1163,7 @@ __device__ __forceinline__ void round_sort_smem(const RoundCtx<SM>& C, int N, in
     sec[s] = kRoundNone;
     id[s] = (unsigned short)s;
     if (s < N) {
-      const RoundRec r = C.W.rec[s];
+      const RoundRec r = C.W.rec(s);
       M[s] = dbits(r.M);  // non-negative: ordered as integers
       sec[s] = ((unsigned)r.l << 12) | (unsigned)r.depth;
     }
@@ -1134,8 +1217,8 @@ __device__ __forceinline__ void round_sort(const RoundCtx<SM>& C, int N, int n2,
         const int lo = base + r, hi = flip ? base + 2 * stride - 1 - r : lo + stride;
         if (hi < N) {
           const Idx x = order[lo], y = order[hi];
-          const RoundRec& rx = C.W.rec[x];
-          const RoundRec& ry = C.W.rec[y];
+          const RoundRec& rx = C.W.rec(x);
+          const RoundRec& ry = C.W.rec(y);
           if (time_less(RoundTime{ry.M, ry.l, ry.depth}, RoundTime{rx.M, rx.l, rx.depth})) {
             order[lo] = y;
             order[hi] = x;
@@ -1165,16 +1248,12 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   event_range(A, e, off, N);
   const int algo = A.algo ? A.algo[e] : A.algo_all;
   const double R = A.radius ? A.radius[e] : A.r_all;
-  Ws g;
-  g.base = A.ws + off;
-  g.stride = A.ws_stride;
   if (tid == 0) {
     S.X.N = N;
     S.X.algo = algo;
     S.X.inv_r2 = 1.0 / (R * R);
     S.X.ilo = __double2float_rd(S.X.inv_r2);
     S.X.ihi = __double2float_ru(S.X.inv_r2);
-    S.X.g = g;
     S.ws = A.round_ws + off * kRoundBytesPerParticle;
     S.r2hi = __double2float_ru(R * R) * 1.0001f;
   }
@@ -1190,18 +1269,17 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     const double* p = A.p4 + (off + s) * A.p4_stride;
     const double px = p[0], py = p[1], pz = p[2], E = p[3];
     const Kin kin = kinematics(px, py, pz, E, algo);
-    g.at(kPx, s) = px;
-    g.at(kPy, s) = py;
-    g.at(kPz, s) = pz;
-    g.at(kE, s) = E;
-    g.at(kW, s) = kin.w;
-    Wk.pos[s] = make_double2(kin.rap, kin.phi);
-    Wk.xy[s] = make_float2(__double2float_rn(kin.rap), __double2float_rn(kin.phi));
-    Wk.wlo[s] = round_weight(kin.w);
-    Wk.tlo[s] = 0.0f;
-    Wk.tm[s] = -1.0;
-    Wk.tl[s] = make_int2(-1, 0);
-    if (!SM) Wk.stamp[s] = make_int2(-1, -1);
+    Wk.p4(0, s) = px;
+    Wk.p4(1, s) = py;
+    Wk.p4(2, s) = pz;
+    Wk.p4(3, s) = E;
+    Wk.w(s) = kin.w;
+    Wk.pos(s) = make_double2(kin.rap, kin.phi);
+    Wk.xy(s) = make_float2(__double2float_rn(kin.rap), __double2float_rn(kin.phi));
+    Wk.wlo(s) = round_weight(kin.w);
+    Wk.tlo(s) = 0.0f;
+    Wk.tm(s) = -1.0;
+    Wk.tl(s) = make_int2(-1, 0);
     rlo = fmin(rlo, kin.rap);
     rhi = fmax(rhi, kin.rap);
     amax = fmax(amax, fabs(kin.rap));
@@ -1268,6 +1346,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     S.rmin = lo;
     S.inv_side_r = (double)nrap / fmax(hi - lo, side);
     S.inv_side_phi = (double)nphi / 6.283185307179586;
+    S.rmin32 = (float)lo;
+    S.side_r = (float)(1.0 / S.inv_side_r);
+    S.side_phi = (float)(1.0 / S.inv_side_phi);
     S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
     S.overflow = 0;
     S.n_cand = S.n_fire = S.n_targets = S.n_dirty = 0;
@@ -1283,8 +1364,8 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   for (int t = tid; t < (S.nrap + 2 * kRoundFrame) * pw; t += T) C.tmin[t] = C.row[t] = kRoundNone;
 #pragma unroll 1
   for (int s = tid; s < N; s += T) {
-    const double2 p = Wk.pos[s];
-    Wk.tile[s] = (Idx)((round_u(S, p.x) << sh) + round_v(S, p.y));
+    const double2 p = Wk.pos(s);
+    Wk.tile(s) = (Idx)((round_u(S, p.x) << sh) + round_v(S, p.y));
   }
   __syncthreads();
   round_lists<SM>(N);
@@ -1300,15 +1381,14 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
 
   // ---- rounds
   int n = N;
-  const float side_r = (float)(1.0 / S.inv_side_r), side_phi = (float)(1.0 / S.inv_side_phi);
-  const float range = reach * (float)R, rmin = (float)S.rmin, inv_side = 1.0f / fminf(side_r, side_phi);
+  const float side_r = S.side_r, side_phi = S.side_phi;
+  const float range = reach * (float)R, rmin = S.rmin32, inv_side = 1.0f / fminf(side_r, side_phi);
 #pragma unroll 1
-  for (int round = 0; n > 0; ++round) {
+  while (n > 0) {
     const bool dense = !SM && n >= kRoundDense * nt;
-    const int sub = n > 16 * nt ? 32 : n > 8 * nt ? 16 : n > 3 * nt ? 8 : 4;
     // A: candidates.  Smallest P of five tiles along the row, then of five
     // rows (empty tiles hold the largest value)
-#pragma unroll 1
+#pragma unroll (SM ? 1 : 4)
     for (int t = tid; t < nt; t += T) {
       const int u = t >> sh, v = t & ((1 << sh) - 1);
       if (v >= nphi) continue;
@@ -1345,8 +1425,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       }
     }
     if (!SM && tid < kRoundSplit) S.parts_done[tid] = 0;
-    if (SM)
-      for (int k = tid; k < (N + 31) / 32; k += T) S.taken[k] = S.claimed[k] = 0;
+    for (int k = tid; k < (SM ? (N + 31) / 32 : kRoundSmemMaxN / 32); k += T) S.taken[k] = S.claimed[k] = 0;
     __syncthreads();
     FJG_PH(mark(kPhRCand);)
     const int nc = min(S.n_cand, kRoundMaxCand);
@@ -1360,23 +1439,41 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       const int cell = (u + kRoundFrame) * pw + kRoundFrame + v;
       const unsigned me = C.tmin[cell];
       int c = C.slot[t];
-      const int fc = Wk.nn[c];
+      const int fc = Wk.nn(c);
       int j = fc & Ws_::kPair ? fc & Ws_::kSlotMask : -1;
-      const float2 gc = Wk.xy[c];
-      const float ckey = Wk.key[c].x;
+      const float2 gc = Wk.xy(c);
+      const float ckey = Wk.key(c).x;
       // distance within which an earlier step could matter: to c, or to its
       // partner as far from c as that is
-      const float beside = j >= 0 ? sqrtf(Wk.nhi[c]) : 0.0f, lim = range + beside;
+      const float beside = j >= 0 ? sqrtf(Wk.nhi(c)) : 0.0f, lim = range + beside;
       float near2 = lim * lim;
       if (algo != -1) {
-        float w = round_wlo(Wk.wlo[c]);
-        if (j >= 0) w = fminf(w, round_wlo(Wk.wlo[j]));
+        float w = round_wlo(Wk.wlo(c));
+        if (j >= 0) w = fminf(w, round_wlo(Wk.wlo(j)));
         const float l = range * sqrtf(fminf(1.0f, __uint_as_float(me) / (0.7f * w))) + beside;
         near2 = l * l;
       }
       const float fu = (gc.x - rmin) - u * side_r, fv = gc.y - v * side_phi;  // within its tile
       const float lim2 = lim * lim;
       const int far = min((int)(lim * inv_side) + 1, kRoundFrame), side = 2 * far + 1, lut = S.lut[side];
+      // what a step that passes needs (in the workspace: loaded meanwhile)
+      const int jc = j >= 0 ? j : c;
+      int fj;
+      double wc, wj, mc, mj;
+      double2 pc, pj;
+      int2 lc, lj;
+      auto load = [&]() {
+        fj = Wk.nn(jc);
+        wc = Wk.w(c);
+        wj = Wk.w(jc);
+        mc = Wk.tm(c);
+        mj = Wk.tm(jc);
+        lc = Wk.tl(c);
+        lj = Wk.tl(jc);
+        pc = Wk.pos(c);
+        pj = Wk.pos(jc);
+      };
+      if (!SM) load();
       bool blocked = false;
 #pragma unroll 1
       for (int i = lane & 7; i < side * side; i += 8) {
@@ -1393,32 +1490,29 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           if (o == me || ov < 0 || ov >= nphi) continue;
           const int so = C.slot[((u + du) << sh) + ov];
           if (so == kNone) continue;  // (a step counted at its partner)
-          const float l = range * sqrtf(fminf(1.0f, __uint_as_float(me) / (0.7f * round_wlo(Wk.wlo[so])))) + beside;
+          const float l = range * sqrtf(fminf(1.0f, __uint_as_float(me) / (0.7f * round_wlo(Wk.wlo(so))))) + beside;
           blocked |= d2 <= l * l;
         } else if (o < me) {
           blocked = true;
         } else if (SM || o == C.tmin[cell + du * pw + dv]) {  // equal P: the smaller key goes first
-          if (ov >= 0 && ov < nphi) blocked |= Wk.key[C.slot[((u + du) << sh) + ov]].x < ckey;
+          if (ov >= 0 && ov < nphi) blocked |= Wk.key(C.slot[((u + du) << sh) + ov]).x < ckey;
         }
       }
       const unsigned ball = __ballot_sync(kFull, blocked);
       if (k < nc && (lane & 7) == 0 && !((ball >> (lane & 24)) & 0xffu)) {
-        // two steps never share a slot: the lower slot is claimed first, so of
+        // two steps never share a slot: the lower bit is claimed first, so of
         // several that want the same ones, one gets both of its own
-        const int jc = j >= 0 ? j : c;
-        bool ok = round_first(C, min(c, jc), round, 0);
-        if (ok && j >= 0) ok = round_first(C, max(c, j), round, 0);
+        const int bc = round_bit<SM>(c), bj = round_bit<SM>(jc);
+        bool ok = round_first(S.taken, min(bc, bj));
+        if (ok && bc != bj) ok = round_first(S.taken, max(bc, bj));
         const int i = ok ? atomicAdd(&S.n_fire, 1) : kRoundSteps;
         if (i < kRoundSteps) {
-          const int fj = Wk.nn[jc];
+          if (SM) load();
           const bool mutual = j >= 0 && (fj & Ws_::kPair) && (fj & Ws_::kSlotMask) == c;
-          const double wc = g.at(kW, c), wj = g.at(kW, jc);
-          const double mc = Wk.tm[c], mj = Wk.tm[jc];
-          const int2 lc = Wk.tl[c], lj = Wk.tl[jc];
           double key = wc;
           RoundTime tc{mc, lc.x, lc.y}, tj{-2.0, -1, 0};
           if (j >= 0) {
-            key = pair_distance(wc, wj, Wk.dr2(c, j), S.X.inv_r2);
+            key = pair_distance(wc, wj, dr2_64(pc.x, pc.y, pj.x, pj.y), S.X.inv_r2);
             tj = RoundTime{mj, lj.x, lj.y};
             if (wj <= key && wj < wc) {
               // a partner at R, up to FP32: its promotion goes first
@@ -1447,11 +1541,11 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           S.thr_c[i] = thr_c;
           S.thr_j[i] = thr_j;
           const int jn = j >= 0 ? j : c;
-          S.tile_c[i] = Wk.tile[c];
-          S.tile_j[i] = Wk.tile[jn];
-          S.xy_c[i] = Wk.xy[c];
-          S.xy_j[i] = Wk.xy[jn];
-          S.wlo[i] = make_float2(round_wlo(Wk.wlo[c]), round_wlo(Wk.wlo[jn]));
+          S.tile_c[i] = Wk.tile(c);
+          S.tile_j[i] = Wk.tile(jn);
+          S.xy_c[i] = Wk.xy(c);
+          S.xy_j[i] = Wk.xy(jn);
+          S.wlo[i] = make_float2(round_wlo(Wk.wlo(c)), round_wlo(Wk.wlo(jn)));
         }
       }
       __syncwarp();
@@ -1483,18 +1577,18 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           m_hi = __double2float_ru(S.M[i]);
           const float2 gc = S.xy_c[i];
           dc = make_float4(gc.x, gc.y, S.wlo[i].x, __double2float_ru(S.thr_c[i]));
-          const int2 tpc = make_int2(S.tile_c[i], Wk.at[c]);
+          const int2 tpc = make_int2(S.tile_c[i], Wk.at(c));
           tile_c = tpc.x;
           S.tp_b[i] = tpc;
           if (j >= 0) {
             const float2 gj = S.xy_j[i];
             dj = make_float4(gj.x, gj.y, S.wlo[i].y, __double2float_ru(S.thr_j[i]));
-            const int2 tpj = make_int2(S.tile_j[i], Wk.at[j]);
+            const int2 tpj = make_int2(S.tile_j[i], Wk.at(j));
             tile_j = tpj.x;
             S.tp_b[i] = c > j ? tpc : tpj;
             S.tp_a[i] = c > j ? tpj : tpc;
             const double w =
-                fjk_weight(__dadd_rn(g.at(kPx, c), g.at(kPx, j)), __dadd_rn(g.at(kPy, c), g.at(kPy, j)), algo);
+                fjk_weight(__dadd_rn(Wk.p4(0, c), Wk.p4(0, j)), __dadd_rn(Wk.p4(1, c), Wk.p4(1, j)), algo);
             S.w[i] = w;
             if (!(w > 0.0)) S.conflict[1] = 1;
           }
@@ -1505,7 +1599,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           r.depth = S.depth[i];
           r.a = j >= 0 ? min(c, j) : -1;
           r.pad = 0;
-          Wk.rec[b] = r;
+          Wk.rec(b) = r;
         }
         __syncwarp();
 #pragma unroll 1
@@ -1513,13 +1607,13 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           round_bury<SM>(have && (!q || j >= 0), q ? tile_j : tile_c, 2 * b + q, q ? dj : dc, m_hi,
                          have ? S.l[i] : 0);
       } else if (have && j >= 0) {
-        const double px = __dadd_rn(g.at(kPx, c), g.at(kPx, j)), py = __dadd_rn(g.at(kPy, c), g.at(kPy, j));
+        const double px = __dadd_rn(Wk.p4(0, c), Wk.p4(0, j)), py = __dadd_rn(Wk.p4(1, c), Wk.p4(1, j));
         if (role == 0) {
           const double phi = fjk_phi(px, py);
           S.phi[i] = phi;
           S.new_v[i] = round_v(S, phi);
         } else {
-          const double pz = __dadd_rn(g.at(kPz, c), g.at(kPz, j)), E = __dadd_rn(g.at(kE, c), g.at(kE, j));
+          const double pz = __dadd_rn(Wk.p4(2, c), Wk.p4(2, j)), E = __dadd_rn(Wk.p4(3, c), Wk.p4(3, j));
           const double rap = fjk_rap(px, py, pz, E);
           S.p4[0][i] = px;
           S.p4[1][i] = py;
@@ -1534,7 +1628,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     }
     // D1 and the targets
     FJG_PH(const long long qb = clock64();)
-    round_phase_b(C, F, G, sub, G == 32 ? max(1, (W - 3) / F) : 1);
+    round_phase_b(C, F, G, G == 32 ? max(1, (SM ? W - 3 : 2 * (W - 3)) / F) : 1);
     FJG_PH(if (tid == T - 32 && A.phase) atomicAdd(A.phase + kPhRScan, (unsigned long long)(clock64() - qb));)
     __syncthreads();
     FJG_PH(mark(kPhRB);)
@@ -1547,7 +1641,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         const int b = max(c, j);
         const int2 tb = S.tp_b[i];
         Wk.members[C.start[tb.x] + tb.y] = (Idx)kNone;
-        Wk.tile[b] = (Idx)kNone;
+        Wk.tile(b) = (Idx)kNone;
         round_dirty(S, tb.x);
         if (j >= 0) {
           const int a = min(c, j);
@@ -1561,8 +1655,8 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
               Wk.place(C.start[t] + p, a, make_float2(__double2float_rn(S.rap[i]), __double2float_rn(S.phi[i])));
             else
               S.overflow = 1;
-            Wk.tile[a] = (Idx)t;
-            Wk.at[a] = (Idx)p;
+            Wk.tile(a) = (Idx)t;
+            Wk.at(a) = (Idx)p;
           } else if (!SM) {
             Wk.place(C.start[t] + ta.y, a, make_float2(__double2float_rn(S.rap[i]), __double2float_rn(S.phi[i])));
           }
@@ -1578,16 +1672,16 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         const int a = min(S.c[i], S.j[i]);
         const double rap = S.rap[i], phi = S.phi[i], w = S.w[i];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) g.at(kPx + q, a) = S.p4[q][i];
-        g.at(kW, a) = w;
-        Wk.pos[a] = make_double2(rap, phi);
-        Wk.xy[a] = make_float2(__double2float_rn(rap), __double2float_rn(phi));
-        Wk.nhi[a] = inf;
-        Wk.wlo[a] = round_weight(w);
-        Wk.tlo[a] = fmaxf(__double2float_rd(S.M[i]), 0.0f);
-        Wk.tm[a] = S.M[i];
-        Wk.tl[a] = make_int2(S.l[i], S.depth[i]);
-        Wk.nn[a] = (Idx)(Ws_::kNoSlot | Ws_::kTarget);  // its own group searches its neighbour
+        for (int q = 0; q < 4; ++q) Wk.p4(q, a) = S.p4[q][i];
+        Wk.w(a) = w;
+        Wk.pos(a) = make_double2(rap, phi);
+        Wk.xy(a) = make_float2(__double2float_rn(rap), __double2float_rn(phi));
+        Wk.nhi(a) = inf;
+        Wk.wlo(a) = round_weight(w);
+        Wk.tlo(a) = fmaxf(__double2float_rd(S.M[i]), 0.0f);
+        Wk.tm(a) = S.M[i];
+        Wk.tl(a) = make_int2(S.l[i], S.depth[i]);
+        Wk.nn(a) = (Idx)(Ws_::kNoSlot | Ws_::kTarget);  // its own group searches its neighbour
       }
     }
     __syncthreads();
@@ -1606,7 +1700,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     const int ntg = min(S.n_targets, kRoundMaxTargets);
     __syncthreads();  // D adds targets
     const int per = 32 / G;
-    const int parts = !SM && F + ntg <= kRoundSplit ? min(4, W / (F + ntg)) : 1;
+    const int parts = !SM && F + ntg <= kRoundSplit ? max(1, min(kRoundParts, W / (F + ntg))) : 1;
     const int uf = (F + per - 1) / per * parts, ut = (ntg + per - 1) / per * parts, ud = (F + per - 1) / per;
 #pragma unroll 1
     for (;;) {
@@ -1618,11 +1712,11 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       const int q = G == 32 ? 0 : lane / 8;
       if (u < uf) {
         const int i = per * (u / parts) + q;
-        round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, round, G, sub, u % parts, parts);
+        round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, G, u % parts, parts);
       } else if (u < uf + ut) {
         const int k = per * ((u - uf) / parts) + q;
         const int t = S.targets[k < ntg ? k : 0];
-        round_search<SM>(k < ntg && (int)Wk.tile[t] != kNone, t, G, sub, F + k, (u - uf) % parts, parts);
+        round_search<SM>(k < ntg && (int)Wk.tile(t) != kNone, t, G, F + k, (u - uf) % parts, parts);
       } else {
         const int i = per * (u - uf - ut) + q;
         if (i < F && S.j[i] >= 0) {
@@ -1654,15 +1748,15 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     }
     if (ntg2 > ntg) {  // slots that two new jets wanted
 #pragma unroll 1
-      for (int k = ntg + warp; k < ntg2; k += W) round_search<SM>(true, S.targets[k], 32, sub, 0, 0, 1);
+      for (int k = ntg + warp; k < ntg2; k += W) round_search<SM>(true, S.targets[k], 32, 0, 0, 1);
       __syncthreads();
     }
     FJG_PH(mark(kPhRE);)
 
     // F: the target bits off; changed tiles
     if (tid < ntg2 || (tid < F && S.j[tid] >= 0)) {
-      if (tid < ntg2) Wk.nn[S.targets[tid]] &= (Idx)~Ws_::kTarget;
-      if (tid < F && S.j[tid] >= 0) Wk.nn[min(S.c[tid], S.j[tid])] &= (Idx)~Ws_::kTarget;
+      if (tid < ntg2) Wk.nn(S.targets[tid]) &= (Idx)~Ws_::kTarget;
+      if (tid < F && S.j[tid] >= 0) Wk.nn(min(S.c[tid], S.j[tid])) &= (Idx)~Ws_::kTarget;
     }
     const int nd = S.n_dirty, ndt = nd <= kRoundMaxDirty ? nd : nt;
     if (dense) {
@@ -1701,14 +1795,13 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     round_sort<SM>(C, N, n2, order);
   FJG_PH(mark(kPhRSort);)
   // ---- outputs
-  int* parent = Wk.dnext;  // [N] of 2N
   int jets = 0;
 #pragma unroll 1
   for (int base = 0; base < N; base += T) {
     const int r = base + tid;
     const int s = r < N ? (int)order[r] : -1;
     RoundRec rec{};
-    if (s >= 0) rec = Wk.rec[s];
+    if (s >= 0) rec = Wk.rec(s);
     const bool jet = s >= 0 && rec.a < 0;
     const unsigned ball = __ballot_sync(kFull, jet);
     if (lane == 0) S.scan_tmp[warp] = __popc(ball);
@@ -1724,14 +1817,14 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       if (jet) {
         const int k = jets + pre + __popc(ball & ((1u << lane) - 1));
         double* jo = A.jets + (off + k) * 4;
-        jo[0] = g.at(kPx, s);
-        jo[1] = g.at(kPy, s);
-        jo[2] = g.at(kPz, s);
-        jo[3] = g.at(kE, s);
+        jo[0] = Wk.p4(0, s);
+        jo[1] = Wk.p4(1, s);
+        jo[2] = Wk.p4(2, s);
+        jo[3] = Wk.p4(3, s);
         A.jet_label[off + k] = s;
         par = -(k + 1);
       }
-      parent[s] = par;
+      Wk.slots[s].parent = par;
     }
     jets += total;
     __syncthreads();
@@ -1740,9 +1833,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   if (A.owner) {
 #pragma unroll 1
     for (int s = tid; s < N; s += T) {
-      int v = parent[s];
+      int v = Wk.slots[s].parent;
 #pragma unroll 1
-      for (int guard = 0; v >= 0 && guard < N; ++guard) v = parent[v];
+      for (int guard = 0; v >= 0 && guard < N; ++guard) v = Wk.slots[v].parent;
       A.owner[off + s] = v < 0 ? -v - 1 : -1;
     }
   }

@@ -138,7 +138,7 @@ struct Scratch {
   int32_t* hist;      // [kHistBins] events per size, then per-size positions (sorting by size)
   unsigned char* large_ws;    // kLargeWsBytesPerParticle per particle, 16 B aligned (null: large events are refused)
   int64_t large_ws_particles;  // particles the large workspace covers
-  unsigned char* round_ws;     // kRoundBytesPerParticle per particle, 16 B aligned (null: no rounds kernel)
+  unsigned char* round_ws;     // kRoundBytesPerParticle per particle, 64 B aligned (null: no rounds kernel)
   int64_t round_ws_particles;
 };
 

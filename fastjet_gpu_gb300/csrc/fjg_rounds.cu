@@ -66,7 +66,7 @@ RoundConfig config_of(int q) {
     case 2: return {k_cluster_rounds<256, 2, true>, 256, 1024, 1792, 1024};
     case 3: return {k_cluster_rounds<256, 2, true>, 256, 1024, 1792, 2048};
     case 4: return {k_cluster_rounds<512, 1, true>, 512, 1024, 1792, 4096};
-    default: return {k_cluster_rounds<512, 1, false>, 512, kRoundMaxTiles, kRoundMaxCells, 0};
+    default: return {k_cluster_rounds<kRoundThreadsWs, 1, false>, kRoundThreadsWs, kRoundMaxTiles, kRoundMaxCells, 0};
   }
 }
 
