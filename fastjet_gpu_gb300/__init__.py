@@ -236,10 +236,10 @@ class Context:
               "t_s3c_summaries", "t_kin_rapidity", "t_detect_s2", "t_steps", "t_events", "exact_key", "exact_nn",
               "t_targets", "t_target_steps", "t_list_update", "t_targets_warp1", "t_window_thread0",
               "t_resolve_new_jet", "t_summary_new_jet_tile", "t_summaries_warp1",
-              "r_setup", "r_candidates", "r_range", "r_keys", "r_b", "r_c", "r_d", "r_e", "r_f", "r_sort", "r_outputs",
+              "r_setup", "r_candidates", "r_range", "r_backs", "r_b", "r_c", "r_d", "r_e", "r_f", "r_sort", "r_outputs",
               "r_rounds", "r_steps", "r_events", "r_retries", "r_cands",
               "r_conflict_a", "r_conflict_b", "r_conflict_d", "r_targets", "r_kin",
-              "r_role0", "r_role1", "r_role2", "r_scan", "r_new_jet", "r_search", "r_dead", "r_overflows")
+              "r_role0", "r_role1", "r_role2", "r_scan", "r_new_jet", "r_search", "r_dead", "r_overflows", "r_undone")
 
     def phase_clocks(self, reset=False):
         """Per-step phase counters of the clustering kernels (only in the

@@ -68,14 +68,14 @@ enum PhaseSlot {
   // targets, thread 0's share of the window pass; warp 0's resolution of the
   // new jet's neighbour and its tile's summary, warp 1's other summaries
   kPhTListUpd = 26, kPhTTargetsW1, kPhTWindowT0, kPhTResolveA, kPhTSumA, kPhTSumW1,
-  // the rounds kernel: set-up, the phases A (candidates; range test; keys), B to
+  // the rounds kernel: set-up, the phases A (candidates; range test), B to
   // F of a round, sort, outputs; rounds, steps, events, events left to the
   // step-by-step kernels
-  kPhRSetup = 32, kPhRCand, kPhRRange, kPhRKeys, kPhRB, kPhRC, kPhRD, kPhRE, kPhRF, kPhRSort, kPhROut, kPhRRounds,
+  kPhRSetup = 32, kPhRCand, kPhRRange, kPhRBacks, kPhRB, kPhRC, kPhRD, kPhRE, kPhRF, kPhRSort, kPhROut, kPhRRounds,
   kPhRSteps, kPhREvents, kPhRRetries, kPhRCands,
   kPhRConflictA, kPhRConflictB, kPhRConflictD, kPhRTargets, kPhRKin,
-  kPhRRole0, kPhRRole1, kPhRRole2, kPhRScan, kPhRNewJet, kPhRSearch, kPhRDead, kPhROverflows,
-  kPhSlots = 61
+  kPhRRole0, kPhRRole1, kPhRRole2, kPhRScan, kPhRNewJet, kPhRSearch, kPhRDead, kPhROverflows, kPhRUndone,
+  kPhSlots = 62
 };
 #ifdef FJG_PHASE_CLOCKS
 #define FJG_PH(...) __VA_ARGS__

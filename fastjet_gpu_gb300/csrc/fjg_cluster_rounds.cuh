@@ -35,9 +35,13 @@
 // T(x, y) >= d_xy, so with thr = k for the one whose own time sets a chained
 // T(E) and thr = T(E)'s key part for the other, a pair is a conflict only if
 // d_xy <= thr (an exact tie counts), d_xy is at most both weights and the other
-// is not younger than E.  An event with a conflict is handed to the
-// step-by-step kernel (retry list) and this kernel's work on it is dropped, so
-// the rule that picks the steps of a round only has to be good, not proven.
+// is not younger than E.  After a conflict the steps from the one that
+// came too early on are taken back (round_undo) and its slot is held until the
+// other step's time; where that is not enough, a wider range follows, and rounds
+// of the one earliest step, which cannot conflict but for exact ties.  Those, and
+// events with too many conflicts, are handed to the step-by-step kernel (retry
+// list) and this kernel's work is dropped.  So the rule that picks the steps of a
+// round only has to be good, not proven.
 //
 // Choice of a round's steps.  Tiles of side >= R/2; per tile the slot with the
 // smallest (P, key), P being the FP32 lower bound of its step's time.  A tile
@@ -47,17 +51,20 @@
 // in a merge, the range shrinks to that of pairs with d below the candidate's
 // P.  Steps a round on the benchmark's kind of events: anti-kt R = 0.4 4 at 200
 // particles, 10 at 1500, 8 to 6 at 8000 to 40,000 dense ones, R = 0.8 3; kt R =
-// 0.6 12 at 1000, 14 at 20,000; C/A R = 0.8 8 at 1000.  Conflicts: none in 1100
-// events of up to 4000 particles (anti-kt R = 0.4, kt, C/A), in about 2 % of
-// anti-kt R = 0.8 events of 3000, in 2 to 6 % of dense anti-kt R = 0.4 events of
-// 8000 to 15,000 and in half of those of 30,000 and more, where a hard jet's
-// chain of steps reaches further; those begin with a range of 2 R (none in 120
-// events).
+// 0.6 12 at 1000, 14 at 20,000; C/A R = 0.8 8 at 1000.  Conflicts with a range of
+// 1.5 R: none in 1100 events of up to 4000 particles (anti-kt R = 0.4, kt, C/A),
+// in about 2 % of anti-kt R = 0.8 events of 3000 and in 2 to 8 % of dense anti-kt
+// R = 0.4 events of 8000 to 15,000; those of 40,000 and more, where a hard jet's
+// chain of steps reaches further, have one or several.  A conflict there costs
+// 100 to 4000 rounds, so events above 20,000 begin with 1.8 R: 64 events of
+// 10,000 to 60,000 particles have 3 to 11 conflicts (10 samples) and take 314 to
+// 330 ms, 333 to 345 with 2.0 R, 308 to 434 with 1.5 R.
 //
 // A round (F steps), eight warps or so:
 //   A   candidates (a thread per tile); range test (eight lanes per candidate),
 //       and the keys, times and thresholds of the steps that pass.
-//   B   new jets' azimuth, rapidity and weight: three warps, a lane per step;
+//   B   new jets' azimuth, rapidity and weight, and what takes the steps back:
+//       four warps, a lane per step;
 //       meanwhile the other warps go over the windows of c and j: D1, and the
 //       slots whose neighbour is taken ("targets").
 //   C   the new jets' state and the tile lists (a lane per step).
@@ -91,7 +98,7 @@ namespace fjg {
 //                R 0.6: 1000 of 600-1000 11.1 -> 9.3, 600 of 1100-2000 17.8 -> 17.9
 //                kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
 //                kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
-//   above 4096   R 0.4: 9000 93 -> 31;  R 0.6: 92 -> 54;  R 0.8: 97 -> 74, where later steps conflict more often
+//   above 4096   R 0.4: 12,000 123 -> 31, 58,000 700 -> 285;  R 0.6: 92 -> 54;  R 0.8: 97 -> 74, where later steps conflict more often
 enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsFew = 2 };
 
 __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
@@ -112,19 +119,22 @@ __device__ __forceinline__ bool rounds_event(const BatchArgs& A, int e) {
 }
 
 constexpr int kRoundSteps = 32;               // steps per round, at most (a lane each)
-constexpr int kRoundBytesPerParticle = 320;   // workspace (304, and events start at whole sectors)
+constexpr int kRoundBytesPerParticle = 384;   // workspace (368, and events start at whole sectors)
 constexpr int kRoundMaxDirty = 384;
 constexpr int kRoundMaxTargets = 128;
 constexpr int kRoundSplit = 24;               // searches of a round, up to which several warps share each
 constexpr int kRoundParts = 5;                // warps that share one, at most
 constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, also in one row
-// range of the choice of steps, in units of R (see above): the first attempt at
-// an event, the second (the first for the largest anti-kt events), the last
-__constant__ const float kRoundReach[3] = {1.5f, 2.0f, 2.5f};
-constexpr int kRoundWideFrom = 20000;
+// range of the choice of steps, in units of R (see above): at first, and after a
+// conflict
+constexpr float kRoundReach = 1.5f, kRoundReachLarge = 1.8f, kRoundReachWide = 2.25f;
+constexpr int kRoundLargeFrom = 20000;
+constexpr int kRoundCareRounds = 64;          // rounds that take care, more than twice those taken back
+constexpr int kRoundMaxBacks = 8;             // conflicts of an event, and one more per 2048 particles
 constexpr int kRoundMaxTiles = 2048;
 constexpr int kRoundMaxCells = 3072;          // with the frame
 constexpr int kRoundFrame = 5;                // tiles around the grid: the range test's 1.5 R + R
+constexpr int kRoundCrowded = 6;              // live slots per tile from which a search begins with the tiles around
 constexpr int kRoundDense = 4;                // live slots per tile from which a warp reads lists together
 constexpr int kRoundSmemMaxN = 4096;
 constexpr int kRoundThreadsWs = 512;          // threads per event with its slots in the workspace
@@ -136,7 +146,7 @@ struct alignas(16) RoundRec {
   double d;   // recorded distance
   int l, depth;
   int a;      // merged into slot a, or -1 (promotion)
-  int pad;
+  int round;  // in which it was fired
 };
 
 struct RoundTime {
@@ -171,7 +181,8 @@ struct alignas(16) RoundSlot {
   float tlo;  // birth time's M, rounded down
   int at;     // position in its tile's list
   int parent;  // (output) what the slot was merged into, or its jet
-  int pad[3];
+  float hold;  // a step of this slot with P from here on waits until all P are
+  int pad[2];
 };
 
 // What the step that removed a slot took: [0] c, [1] j.
@@ -181,9 +192,12 @@ struct alignas(16) RoundDead {
                   // M), its M rounded up (float), first member, l
   RoundRec rec;
   int next[2];    // next member
-  int pad[6];
+  int2 tl;        // slot a before the step, to take it back: as in RoundSlot
+  double p[4], w, tm;
+  double2 pos;
+  int pad[4];
 };
-static_assert(sizeof(RoundSlot) == 128 && sizeof(RoundDead) == 128, "whole sectors");
+static_assert(sizeof(RoundSlot) == 128 && sizeof(RoundDead) == 192, "whole sectors");
 
 // The event's state.  SM (events of up to kRoundSmemMaxN particles): what every
 // round reads is in shared memory, 36 bytes a slot, so that two CTAs share an
@@ -245,8 +259,8 @@ __device__ __forceinline__ RoundWs<SM> round_ws(unsigned char* base, unsigned ch
   W.slots = reinterpret_cast<RoundSlot*>(base);
   W.dead = reinterpret_cast<RoundDead*>(base + 128 * n);
   if (!SM) {
-    W.lxy = reinterpret_cast<float2*>(base + 256 * n);
-    W.members = reinterpret_cast<typename RoundWs<SM>::Idx*>(base + 288 * n);  // to 304 n
+    W.lxy = reinterpret_cast<float2*>(base + 320 * n);
+    W.members = reinterpret_cast<typename RoundWs<SM>::Idx*>(base + 352 * n);  // to 368 n
     return W;
   }
   W.sxy = reinterpret_cast<float2*>(smem);
@@ -287,6 +301,13 @@ struct RoundShared {
   // barrier that closes its phase and written again only a round later, so
   // every thread of the CTA takes the same way
   int conflict[3];
+  int back;  // round to go back to
+  int hopeless, alive, backs;
+  // rounds before `care_until` take care: 1: the wide range; 2: one step, that
+  // with the earliest time
+  int care, care_until;
+  unsigned p_min;
+  float reach;
   int n_cand, n_fire, n_targets, n_dirty;
   int task[2];
   // the round's steps: c, j (-1: promotion), tile and list position of the
@@ -669,7 +690,7 @@ __device__ __forceinline__ bool round_join(const RoundCtx<SM>& C, Cert& c, int i
 }
 
 // Slot t's neighbour in its window, and its key (groups of G lanes; or one of
-// several warps of search `item`).
+// several warps of search `item`; parts = 0: the tiles around first).
 template <bool SM>
 __device__ __noinline__ void round_search(bool have, int t, int G, int item, int part, int parts) {
   const RoundCtx<SM> C = round_ctx<SM>();
@@ -679,14 +700,37 @@ __device__ __noinline__ void round_search(bool have, int t, int G, int item, int
   const float2 gt = C.W.xy(t);
   const Bound bd = C.S->X.bd;
   Cert x = cert_empty();
-  const int nb = b.nu * b.nv;
-  for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, gt, gt, [&](int, float2 g) { return g; },
-          [&](int u, float2 gu) {
-            float lo, hi;
-            dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
-            if (u != t) cert_add(x, lo, hi, u);
-          });
-  x = cert_group(x, G);
+  bool near = false;
+  if (!SM && parts == 0) {
+    // many slots per tile: the tiles next to its own, beyond which all is further
+    // than the smaller side
+    if (have) {
+      const int u = tile >> C.S->sh, v = tile & ((1 << C.S->sh) - 1);
+      b.u0 = max(u - 1, 0);
+      b.nu = min(u + 1, C.S->nrap - 1) - b.u0 + 1;
+      b.v0 = v ? v - 1 : C.S->nphi - 1;
+      b.nv = 3;
+    }
+    near = true;
+    parts = 1;
+  }
+#pragma unroll 1
+  for (;;) {
+    const int nb = b.nu * b.nv;
+    for_tiles(C, b, nb * part / parts, nb * (part + 1) / parts, G, gt, gt, [&](int, float2 g) { return g; },
+            [&](int u, float2 gu) {
+              float lo, hi;
+              dr2_32(gt.x, gt.y, gu.x, gu.y, bd, lo, hi);
+              if (u != t) cert_add(x, lo, hi, u);
+            });
+    x = cert_group(x, G);
+    if (!near) break;
+    near = false;
+    const float side = fminf(C.S->side_r, C.S->side_phi) * 0.999f;
+    if (!have || (x.i1 >= 0 && x.u1 <= side * side)) break;
+    x = cert_empty();
+    b = round_box(*C.S, tile, tile);
+  }
   if (parts > 1 && !round_join(C, x, item, part, parts)) return;
   round_settle<SM>(have, (threadIdx.x & (G - 1)) == 0, t, x, RoundWs<SM>::kTarget);
 }
@@ -952,7 +996,12 @@ __device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) 
         const float plo = __fmul_rd(__fmul_rd(__fmul_rd(fminf(wa, dg.z), lo), ilo), 0.99999976158142089844f);
         if (lo <= r2hi && !(plo > dg.w)) {
           const RoundRec q = C.W.rec(y >> 1);
-          bad |= time_less(RoundTime{M, l, depth}, RoundTime{q.M, q.l, q.depth});
+          if (time_less(RoundTime{M, l, depth}, RoundTime{q.M, q.l, q.depth})) {
+            bad = true;
+            atomicMin(&C.S->back, q.round);
+            // (both positive: ordered as integers)
+            atomicMax(reinterpret_cast<int*>(&C.W.slots[y >> 1].hold), __float_as_int(m_lo * (1.0f - 0x1p-13f)));
+          }
         }
         y = C.W.dnext(y);
       }
@@ -961,6 +1010,203 @@ __device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) 
     x = r.x;
   }
   return bad;
+}
+
+// What the time of a step is made of: of c and of its partner j.
+struct RoundPair {
+  double wc, wj, mc, mj;
+  double2 pc, pj;
+  int2 lc, lj;
+  int fj;
+  float hold;
+};
+
+template <bool SM>
+__device__ __forceinline__ RoundPair round_pair(const RoundWs<SM>& W, int c, int j) {
+  return RoundPair{W.w(c), W.w(j), W.tm(c), W.tm(j), W.pos(c), W.pos(j), W.tl(c), W.tl(j), (int)W.nn(j),
+                   fmaxf(W.slots[c].hold, W.slots[j].hold)};
+}
+
+// The step of slot c with partner j (-1: none): its key, its time and whether it
+// follows that of c or of j.
+struct RoundStep {
+  int c, j;
+  double key;
+  RoundTime t;
+  bool chained, from_j;
+};
+
+template <bool SM>
+__device__ __forceinline__ RoundStep round_step(int c, int j, const RoundPair& p, double inv_r2) {
+  const bool mutual = j >= 0 && (p.fj & RoundWs<SM>::kPair) && (p.fj & RoundWs<SM>::kSlotMask) == c;
+  RoundStep s{c, j, p.wc, {}, false, false};
+  RoundTime tc{p.mc, p.lc.x, p.lc.y}, tj{-2.0, -1, 0};
+  if (j >= 0) {
+    s.key = pair_distance(p.wc, p.wj, dr2_64(p.pc.x, p.pc.y, p.pj.x, p.pj.y), inv_r2);
+    tj = RoundTime{p.mj, p.lj.x, p.lj.y};
+    if (p.wj <= s.key && p.wj < p.wc) {
+      // a partner at R, up to FP32: its promotion goes first
+      s.c = j;
+      s.j = -1;
+      s.key = p.wj;
+      tc = tj;
+      tj = RoundTime{-2.0, -1, 0};
+    }
+  }
+  s.from_j = time_less(tc, tj);
+  const RoundTime tp = s.from_j ? tj : tc;
+  s.t = RoundTime{s.key, mutual && s.j >= 0 ? min(c, j) : s.c, 0};
+  s.chained = s.t.M < tp.M || (s.t.M == tp.M && s.t.l <= tp.l);
+  if (s.chained) s.t = RoundTime{tp.M, tp.l, tp.depth + 1};
+  return s;
+}
+
+// The order of steps: those of the same time follow the same one, the smallest
+// key first.
+__device__ __forceinline__ bool round_earlier(const RoundTime& x, double kx, int cx, const RoundTime& y, double ky,
+                                              int cy) {
+  if (time_less(x, y)) return true;
+  if (time_less(y, x)) return false;
+  return kx < ky || (kx == ky && cx < cy);
+}
+
+// A slot with the earliest step of all, per warp, into S.targets (whole CTA); P
+// is within 2^-15 of the time's M.
+template <bool SM>
+__device__ __noinline__ void round_pick() {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  RoundShared& S = *C.S;
+  using Ws_ = RoundWs<SM>;
+  const float lim = __uint_as_float(S.p_min) * (1.0f + 0x1p-13f);
+  RoundStep best{};
+  int slot = -1;
+#pragma unroll 1
+  for (int s = threadIdx.x; s < S.X.N; s += blockDim.x) {
+    if (C.W.tile(s) == (typename Ws_::Idx)Ws_::kNone || !(C.W.key(s).y <= lim)) continue;
+    const int f = C.W.nn(s), j = f & Ws_::kPair ? f & Ws_::kSlotMask : -1;
+    const RoundStep q = round_step<SM>(s, j, round_pair(C.W, s, j >= 0 ? j : s), S.X.inv_r2);
+    if (slot < 0 || round_earlier(q.t, q.key, s, best.t, best.key, slot)) {
+      best = q;
+      slot = s;
+    }
+  }
+#pragma unroll 1
+  for (int o = 16; o; o >>= 1) {
+    RoundTime t;
+    t.M = __shfl_xor_sync(kFull, best.t.M, o);
+    t.l = __shfl_xor_sync(kFull, best.t.l, o);
+    t.depth = __shfl_xor_sync(kFull, best.t.depth, o);
+    const double key = __shfl_xor_sync(kFull, best.key, o);
+    const int other = __shfl_xor_sync(kFull, slot, o);
+    if (other >= 0 && (slot < 0 || round_earlier(t, key, other, best.t, best.key, slot))) {
+      best.t = t;
+      best.key = key;
+      slot = other;
+    }
+  }
+  if ((threadIdx.x & 31) == 0 && slot >= 0) round_target(S, slot);
+}
+
+// Of the round's steps only the earliest stays (one thread).
+template <bool SM>
+__device__ __noinline__ void round_earliest() {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  RoundShared& S = *C.S;
+  int b = 0;
+#pragma unroll 1
+  for (int i = 1; i < min(S.n_fire, kRoundSteps); ++i)
+    if (round_earlier(RoundTime{S.M[i], S.l[i], S.depth[i]}, S.key[i], S.c[i],
+                      RoundTime{S.M[b], S.l[b], S.depth[b]}, S.key[b], S.c[b]))
+      b = i;
+  if (S.new_u[b]) S.conflict[0] = 1;
+  S.c[0] = S.c[b];
+  S.j[0] = S.j[b];
+  S.key[0] = S.key[b];
+  S.M[0] = S.M[b];
+  S.l[0] = S.l[b];
+  S.depth[0] = S.depth[b];
+  S.thr_c[0] = S.thr_c[b];
+  S.thr_j[0] = S.thr_j[b];
+  S.tile_c[0] = S.tile_c[b];
+  S.tile_j[0] = S.tile_j[b];
+  S.xy_c[0] = S.xy_c[b];
+  S.xy_j[0] = S.xy_j[b];
+  S.wlo[0] = S.wlo[b];
+  S.n_fire = min(S.n_fire, 1);
+  S.n_targets = 0;
+}
+
+// Takes back the steps of rounds r0 and later (whole CTA): the slots they removed
+// return, those they merged into get back what the first such step saved, and the
+// groups of the dead are made again from the others' (a warp per 1 / W of the
+// tiles).  Lists, neighbours and minima are to be made again.  Leaves the number
+// of live slots in S.alive.
+template <bool SM>
+__device__ __noinline__ void round_undo(int r0) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  RoundShared& S = *C.S;
+  using Idx = typename RoundWs<SM>::Idx;
+  constexpr int kNone = RoundWs<SM>::kNone;
+  const int N = S.X.N, T = blockDim.x, W = T / 32, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto undone = [&](int s) { return C.W.tile(s) == kNone && C.W.rec(s).round >= r0 && C.W.rec(s).a >= 0; };
+  for (int s = tid; s < N; s += T) C.W.slots[s].parent = 0x7fffffff;
+  for (int t = tid; t < S.nt; t += T) {
+    C.head[t] = -1;
+    C.head_m[t] = 0.0f;
+  }
+  if (tid == 0) S.alive = 0;
+  __syncthreads();
+#pragma unroll 1
+  for (int s = tid; s < N; s += T)
+    if (undone(s)) atomicMin(&C.W.slots[C.W.rec(s).a].parent, C.W.rec(s).round);
+  __syncthreads();
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    if (!undone(s)) continue;
+    const int a = C.W.rec(s).a;
+    if (C.W.slots[a].parent != C.W.rec(s).round) continue;
+    const RoundDead& D = C.W.dead[s];
+    for (int q = 0; q < 4; ++q) C.W.p4(q, a) = D.p[q];
+    C.W.w(a) = D.w;
+    C.W.pos(a) = D.pos;
+    C.W.tm(a) = D.tm;
+    C.W.tl(a) = D.tl;
+    C.W.tlo(a) = fmaxf(__double2float_rd(D.tm), 0.0f);
+    C.W.xy(a) = make_float2(__double2float_rn(D.pos.x), __double2float_rn(D.pos.y));
+    C.W.wlo(a) = round_weight(D.w);
+  }
+  __syncthreads();
+  int alive = 0;
+#pragma unroll 1
+  for (int s = tid; s < N; s += T) {
+    if (C.W.tile(s) == kNone && C.W.rec(s).round < r0) continue;
+    const double2 p = C.W.pos(s);
+    C.W.tile(s) = (Idx)((round_u(S, p.x) << S.sh) + round_v(S, p.y));
+    ++alive;
+  }
+  alive = __reduce_add_sync(kFull, alive);
+  if (lane == 0) atomicAdd(&S.alive, alive);
+  __syncthreads();
+#pragma unroll 1
+  for (int s0 = 0; s0 < N; s0 += 32) {
+    const int s = s0 + lane;
+    const bool dead = s < N && C.W.tile(s) == kNone;
+    const RoundRec r = C.W.rec(dead ? s : s0);
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+      const float4 g = C.W.dgeo(2 * (dead ? s : s0) + q);
+      const int t = dead && (!q || r.a >= 0) ? (round_u(S, g.x) << S.sh) + round_v(S, g.y) : -1;
+      const bool mine = t >= 0 && t % W == warp;
+      if (__any_sync(kFull, mine)) round_bury<SM>(mine, mine ? t : 0, 2 * s + q, g, __double2float_ru(r.M), r.l);
+    }
+  }
+  if (tid == 0) {
+    S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
+    S.n_cand = S.n_fire = S.n_targets = S.overflow = 0;
+    S.p_min = kRoundNone;
+    S.task[0] = S.task[1] = 0;
+  }
+  __syncthreads();
 }
 
 // Initial neighbours: a thread per slot, or (dense) a warp per tile -- a lane per
@@ -983,9 +1229,14 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
         const int t = C.W.members[st0 + (have ? i0 + lane : i0)];
         const float2 gt = C.W.xy(t);
         Cert c = cert_empty();
+        // its own tile, then those that can hold something closer for a lane
 #pragma unroll 1
-        for (int k = 0; k < nb; ++k) {
-          const int tt = box_tile(S, b, k);
+        for (int k = -1; k < nb; ++k) {
+          const int tt = k < 0 ? tile : box_tile(S, b, k);
+          if (k >= 0) {
+            const float d = tile_d2(S, gt, tt >> S.sh, tt & ((1 << S.sh) - 1)) * 0.999f - 1e-6f;
+            if (tt == tile || !__any_sync(kFull, have && d <= c.u1)) continue;
+          }
           const int st = C.start[tt], m = C.count[tt];
 #pragma unroll 1
           for (int q0 = 0; q0 < m; q0 += 32) {
@@ -1010,10 +1261,10 @@ __device__ __forceinline__ void round_init(const RoundCtx<SM>& C, bool dense) {
 #pragma unroll 1
   for (int s0 = threadIdx.x & ~31; s0 < N; s0 += blockDim.x) {
     const int t = s0 + lane;
-    const bool have = t < N;
+    const int tile = t < N ? C.W.tile(t) : (typename RoundWs<SM>::Idx)RoundWs<SM>::kNone;
+    const bool have = t < N && tile != RoundWs<SM>::kNone;
     Cert c = cert_empty();
     if (have) {
-      const int tile = C.W.tile(t);
       const RoundBox b = round_box(S, tile, tile);
       const int nb = b.nu * b.nv;
       const float2 gt = C.W.xy(t);
@@ -1231,10 +1482,9 @@ __device__ __forceinline__ void round_sort(const RoundCtx<SM>& C, int N, int n2,
 }
 
 // Clusters event e; false: a conflict (nothing of the event's outputs was
-// written).  S.tiles, cells and slots are set; reach: the range of the choice
-// of steps, in units of R.
+// written).  S.tiles, cells and slots are set.
 template <int T, bool SM>
-__device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const BatchArgs& A, int e, float reach) {
+__device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const BatchArgs& A, int e) {
   constexpr int W = T / 32;
   using Ws_ = RoundWs<SM>;
   using Idx = typename Ws_::Idx;
@@ -1279,6 +1529,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     Wk.wlo(s) = round_weight(kin.w);
     Wk.tlo(s) = 0.0f;
     Wk.tm(s) = -1.0;
+    Wk.slots[s].hold = 0.0f;
     Wk.tl(s) = make_int2(-1, 0);
     rlo = fmin(rlo, kin.rap);
     rhi = fmax(rhi, kin.rap);
@@ -1350,7 +1601,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     S.side_r = (float)(1.0 / S.inv_side_r);
     S.side_phi = (float)(1.0 / S.inv_side_phi);
     S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
-    S.overflow = 0;
+    S.overflow = S.hopeless = S.backs = S.care = S.care_until = 0;
+    S.p_min = kRoundNone;
+    S.reach = algo == -1 && N > kRoundLargeFrom ? kRoundReachLarge : kRoundReach;
     S.n_cand = S.n_fire = S.n_targets = S.n_dirty = 0;
     S.task[0] = S.task[1] = 0;
   }
@@ -1368,24 +1621,30 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     Wk.tile(s) = (Idx)((round_u(S, p.x) << sh) + round_v(S, p.y));
   }
   __syncthreads();
-  round_lists<SM>(N);
 
-  // ---- initial neighbours (round_set marks tiles as changed: cleared after)
-  round_init(C, N >= kRoundDense * nt);
+  int n = N, round = 0;
+#pragma unroll 1
+  for (;;) {
+  round_lists<SM>(n);
+  // ---- neighbours (round_set marks tiles as changed: cleared after)
+  round_init(C, n >= kRoundDense * nt);
   __syncthreads();
   for (int t = tid; t < nt; t += T) round_summary_thread<SM>(t);
   for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
   __syncthreads();
-  if (tid == 0) S.n_dirty = 0;
+  if (tid == 0) {
+    S.n_dirty = 0;
+    S.back = 0x7fffffff;
+  }
   FJG_PH(mark(kPhRSetup);)
 
   // ---- rounds
-  int n = N;
   const float side_r = S.side_r, side_phi = S.side_phi;
-  const float range = reach * (float)R, rmin = S.rmin32, inv_side = 1.0f / fminf(side_r, side_phi);
+  const float rmin = S.rmin32, inv_side = 1.0f / fminf(side_r, side_phi);
 #pragma unroll 1
-  while (n > 0) {
+  for (; n > 0; ++round) {
     const bool dense = !SM && n >= kRoundDense * nt;
+    const int care = round < S.care_until ? S.care : 0;
     // A: candidates.  Smallest P of five tiles along the row, then of five
     // rows (empty tiles hold the largest value)
 #pragma unroll (SM ? 1 : 4)
@@ -1405,6 +1664,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       const int k = (u + kRoundFrame) * pw + kRoundFrame + v;
       const unsigned me = C.tmin[k];
       if (me == kRoundNone) continue;
+      if (S.backs) atomicMin(&S.p_min, me);
       if (!SM) {
         // a step also counts where its partner is: a hard jet's own key may
         // belong to a later step (its neighbour is younger) while an earlier
@@ -1428,17 +1688,22 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     for (int k = tid; k < (SM ? (N + 31) / 32 : kRoundSmemMaxN / 32); k += T) S.taken[k] = S.claimed[k] = 0;
     __syncthreads();
     FJG_PH(mark(kPhRCand);)
-    const int nc = min(S.n_cand, kRoundMaxCand);
+    if (care == 2) {
+      round_pick<SM>();
+      __syncthreads();
+    }
+    const int nc = care == 2 ? min(S.n_targets, kRoundSteps) : min(S.n_cand, kRoundMaxCand);
+    const float range = (care ? kRoundReachWide : S.reach) * (float)R;
     // range test, eight lanes per candidate, and the keys, times and thresholds
     // of the steps that pass
 #pragma unroll 1
     for (int k0 = 4 * warp; k0 < nc; k0 += 4 * W) {
       const int k = k0 + lane / 8;
-      const int t = k < nc ? S.cand[k] : S.cand[k0];
+      const int kk = k < nc ? k : k0, t = care == 2 ? (int)Wk.tile(S.targets[kk]) : S.cand[kk];
       const int u = t >> sh, v = t & ((1 << sh) - 1);
       const int cell = (u + kRoundFrame) * pw + kRoundFrame + v;
       const unsigned me = C.tmin[cell];
-      int c = C.slot[t];
+      int c = care == 2 ? S.targets[kk] : (int)C.slot[t];
       const int fc = Wk.nn(c);
       int j = fc & Ws_::kPair ? fc & Ws_::kSlotMask : -1;
       const float2 gc = Wk.xy(c);
@@ -1458,25 +1723,11 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       const int far = min((int)(lim * inv_side) + 1, kRoundFrame), side = 2 * far + 1, lut = S.lut[side];
       // what a step that passes needs (in the workspace: loaded meanwhile)
       const int jc = j >= 0 ? j : c;
-      int fj;
-      double wc, wj, mc, mj;
-      double2 pc, pj;
-      int2 lc, lj;
-      auto load = [&]() {
-        fj = Wk.nn(jc);
-        wc = Wk.w(c);
-        wj = Wk.w(jc);
-        mc = Wk.tm(c);
-        mj = Wk.tm(jc);
-        lc = Wk.tl(c);
-        lj = Wk.tl(jc);
-        pc = Wk.pos(c);
-        pj = Wk.pos(jc);
-      };
-      if (!SM) load();
+      RoundPair pair;
+      if (!SM) pair = round_pair(Wk, c, jc);
       bool blocked = false;
 #pragma unroll 1
-      for (int i = lane & 7; i < side * side; i += 8) {
+      for (int i = lane & 7; i < side * side && care != 2; i += 8) {
         const int row = (i * lut) >> 16, du = row - far, dv = i - side * row - far;
         const unsigned o = C.near[cell + du * pw + dv];
         if (o > me) continue;
@@ -1503,35 +1754,25 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         // two steps never share a slot: the lower bit is claimed first, so of
         // several that want the same ones, one gets both of its own
         const int bc = round_bit<SM>(c), bj = round_bit<SM>(jc);
-        bool ok = round_first(S.taken, min(bc, bj));
-        if (ok && bc != bj) ok = round_first(S.taken, max(bc, bj));
+        bool ok = care == 2;
+        if (SM) pair = round_pair(Wk, c, jc);
+        if (!ok && !(__uint_as_float(me) >= pair.hold && __uint_as_float(S.p_min) < pair.hold)) {
+          ok = round_first(S.taken, min(bc, bj));
+          if (ok && bc != bj) ok = round_first(S.taken, max(bc, bj));
+        }
         const int i = ok ? atomicAdd(&S.n_fire, 1) : kRoundSteps;
         if (i < kRoundSteps) {
-          if (SM) load();
-          const bool mutual = j >= 0 && (fj & Ws_::kPair) && (fj & Ws_::kSlotMask) == c;
-          double key = wc;
-          RoundTime tc{mc, lc.x, lc.y}, tj{-2.0, -1, 0};
-          if (j >= 0) {
-            key = pair_distance(wc, wj, dr2_64(pc.x, pc.y, pj.x, pj.y), S.X.inv_r2);
-            tj = RoundTime{mj, lj.x, lj.y};
-            if (wj <= key && wj < wc) {
-              // a partner at R, up to FP32: its promotion goes first
-              c = j;
-              j = -1;
-              key = wj;
-              tc = tj;
-              tj = RoundTime{-2.0, -1, 0};
-            }
-          }
-          const bool from_j = time_less(tc, tj);
-          const RoundTime tp = from_j ? tj : tc;
-          RoundTime te{key, mutual && j >= 0 ? min(c, j) : c, 0};
-          const bool chained = te.M < tp.M || (te.M == tp.M && te.l <= tp.l);
-          if (chained) te = RoundTime{tp.M, tp.l, tp.depth + 1};
-          const double thr_c = chained && !from_j ? key : te.M;
-          const double thr_j = chained && from_j ? key : te.M;
+          const RoundStep st = round_step<SM>(c, j, pair, S.X.inv_r2);
+          c = st.c;
+          j = st.j;
+          const RoundTime te = st.t;
+          const double key = st.key, wc = pair.wc, wj = pair.wj;
+          const double thr_c = st.chained && !st.from_j ? key : te.M;
+          const double thr_j = st.chained && st.from_j ? key : te.M;
           // the promotions of c and j come later
-          if (j >= 0 && (wc <= thr_c || wj <= thr_j)) S.conflict[0] = 1;
+          const bool late = j >= 0 && (wc <= thr_c || wj <= thr_j);
+          if (late && care != 2) S.conflict[0] = 1;
+          S.new_u[i] = late;
           S.c[i] = c;
           S.j[i] = j;
           S.key[i] = key;
@@ -1551,6 +1792,10 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       __syncwarp();
     }
     __syncthreads();
+    if (care == 2) {
+      if (tid == 0) round_earliest<SM>();
+      __syncthreads();
+    }
     const int F = min(S.n_fire, kRoundSteps);
     if (!F || S.conflict[0]) {  // (F = 0: cannot happen)
       if (tid == 0) S.conflict[1] = 1;
@@ -1562,7 +1807,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
 
     // B: kinematics of the new jets, a lane per step
 #pragma unroll 1
-    for (int role = warp; role < 3; role += W) {
+    for (int role = warp; role < 4; role += W) {
       FJG_PH(const long long q0 = clock64();)
       const int i = lane;
       const bool have = i < F;
@@ -1590,7 +1835,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
             const double w =
                 fjk_weight(__dadd_rn(Wk.p4(0, c), Wk.p4(0, j)), __dadd_rn(Wk.p4(1, c), Wk.p4(1, j)), algo);
             S.w[i] = w;
-            if (!(w > 0.0)) S.conflict[1] = 1;
+            if (!(w > 0.0)) S.conflict[1] = S.hopeless = 1;
           }
           RoundRec r;
           r.M = S.M[i];
@@ -1598,7 +1843,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
           r.l = S.l[i];
           r.depth = S.depth[i];
           r.a = j >= 0 ? min(c, j) : -1;
-          r.pad = 0;
+          r.round = round;
           Wk.rec(b) = r;
         }
         __syncwarp();
@@ -1606,6 +1851,17 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         for (int q = 0; q < 2; ++q)
           round_bury<SM>(have && (!q || j >= 0), q ? tile_j : tile_c, 2 * b + q, q ? dj : dc, m_hi,
                          have ? S.l[i] : 0);
+      } else if (role == 3) {
+        if (have && j >= 0) {  // slot a as it was, to take the step back
+          RoundDead& D = Wk.dead[max(c, j)];
+          const RoundSlot& a = Wk.slots[min(c, j)];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) D.p[q] = a.p[q];
+          D.w = a.w;
+          D.tm = a.tm;
+          D.tl = a.tl;
+          D.pos = a.pos;
+        }
       } else if (have && j >= 0) {
         const double px = __dadd_rn(Wk.p4(0, c), Wk.p4(0, j)), py = __dadd_rn(Wk.p4(1, c), Wk.p4(1, j));
         if (role == 0) {
@@ -1624,7 +1880,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         }
       }
       __syncwarp();
-      FJG_PH(if (lane == 0 && A.phase) atomicAdd(A.phase + kPhRRole0 + role, (unsigned long long)(clock64() - q0));)
+      FJG_PH(if (lane == 0 && A.phase && role < 3) atomicAdd(A.phase + kPhRRole0 + role, (unsigned long long)(clock64() - q0));)
     }
     // D1 and the targets
     FJG_PH(const long long qb = clock64();)
@@ -1664,6 +1920,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       }
       if (lane == 0) {
         S.n_cand = 0;
+        S.p_min = kRoundNone;
         S.task[0] = 0;
       }
     } else if (warp == 1) {
@@ -1701,7 +1958,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     __syncthreads();  // D adds targets
     const int per = 32 / G;
     const int parts = !SM && F + ntg <= kRoundSplit ? max(1, min(kRoundParts, W / (F + ntg))) : 1;
-    const int uf = (F + per - 1) / per * parts, ut = (ntg + per - 1) / per * parts, ud = (F + per - 1) / per;
+    // (parts of the targets' searches)
+    const int pt = !SM && n >= kRoundCrowded * nt && nphi >= 5 ? 0 : parts, pts = pt ? pt : 1;
+    const int uf = (F + per - 1) / per * parts, ut = (ntg + per - 1) / per * pts, ud = (F + per - 1) / per;
 #pragma unroll 1
     for (;;) {
       int u = 0;
@@ -1714,9 +1973,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         const int i = per * (u / parts) + q;
         round_new_jet(C, i < F && S.j[i < F ? i : 0] >= 0, i < F ? i : 0, G, u % parts, parts);
       } else if (u < uf + ut) {
-        const int k = per * ((u - uf) / parts) + q;
+        const int k = per * ((u - uf) / pts) + q;
         const int t = S.targets[k < ntg ? k : 0];
-        round_search<SM>(k < ntg && (int)Wk.tile(t) != kNone, t, G, F + k, (u - uf) % parts, parts);
+        round_search<SM>(k < ntg && (int)Wk.tile(t) != kNone, t, G, F + k, (u - uf) % pts, pt);
       } else {
         const int i = per * (u - uf - ut) + q;
         if (i < F && S.j[i] >= 0) {
@@ -1776,12 +2035,29 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     // (the next writers of these follow the next barriers)
   }
   __syncthreads();
-  if (S.conflict[0] | S.conflict[1] | S.conflict[2]) {
-    FJG_PH(if (A.phase && tid == 0) {
-      atomicAdd(A.phase + kPhRRetries, 1ull);
-      for (int k = 0; k < 3; ++k) atomicAdd(A.phase + kPhRConflictA + k, (unsigned long long)(S.conflict[k] != 0));
-    })
-    return false;
+  if (!(S.conflict[0] | S.conflict[1] | S.conflict[2])) break;
+  // back to before the step that came too early (D1, and D2 within a round: this
+  // round's), and from there with more care
+  const int r0 = min(S.back, round);
+  const bool again = round < S.care_until;
+  const int care = !S.conflict[2] ? 2 : !again ? 0 : round - r0 <= 4 * kRoundCareRounds ? 2 : 1;
+  const bool hopeless = S.hopeless || S.backs >= kRoundMaxBacks + N / 2048 || (again && S.care == 2 && r0 == round);
+  FJG_PH(ph[kPhRBacks - kPhRSetup] += 1; if (A.phase && tid == 0) {
+    atomicAdd(A.phase + kPhRRetries, (unsigned long long)hopeless);
+    for (int k = 0; k < 3; ++k) atomicAdd(A.phase + kPhRConflictA + k, (unsigned long long)(S.conflict[k] != 0));
+    atomicAdd(A.phase + kPhRUndone, (unsigned long long)(round - r0));
+  })
+  __syncthreads();
+  if (hopeless) return false;
+  round_undo<SM>(r0);
+  if (tid == 0) {
+    ++S.backs;
+    S.care = care;
+    S.care_until = round + (care < 2 ? 2 * (round - r0) + kRoundCareRounds : max(S.alive - n, 0) + kRoundCareRounds / 4);
+  }
+  n = S.alive;
+  ++round;
+  FJG_PH(mark(kPhRSetup);)
   }
 
   // ---- records in sequential order

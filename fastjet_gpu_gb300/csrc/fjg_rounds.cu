@@ -27,18 +27,8 @@ __global__ void __launch_bounds__(T, MINB) k_cluster_rounds(BatchArgs A) {
       continue;
     }
     if (refused_event(A, e)) continue;  // ends with a barrier
-    // after a conflict once more with a wider range, which costs less than the
-    // step-by-step kernel; the largest anti-kt events begin with one
-    int64_t off;
-    int n;
-    event_range(A, e, off, n);
-    const bool wide = n > kRoundWideFrom && (A.algo ? A.algo[e] : A.algo_all) == -1;
-    bool done = false;
-#pragma unroll 1
-    for (int attempt = 0; attempt < 2 && !done; ++attempt) {
-      done = cluster_event_rounds<T, SM>(S, A, e, kRoundReach[attempt + (wide ? 1 : 0)]);
-      __syncthreads();
-    }
+    const bool done = cluster_event_rounds<T, SM>(S, A, e);
+    __syncthreads();
     if (threadIdx.x == 0) {
       if (done)
         signal_done(A, e);

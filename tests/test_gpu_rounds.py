@@ -95,3 +95,13 @@ def test_many_events_mixed_rules(ctx):
     out = {k: v.cpu().numpy() for k, v in g.out.items() if k != "history"}
     out["history"] = F.history_records(g.out["history"])
     U.same_results(out, res, off)
+
+
+def test_steps_taken_back(ctx):
+    """Events in which a step is found to have come too early (dense, R = 0.6 and
+    0.8; above 4096 particles the slots' state is in the workspace): the steps
+    since are taken back, and the result is the step-by-step one."""
+    for n, radius, seeds in ((3000, 0.8, 12), (6000, 0.6, 3), (30000, 0.4, 1)):
+        for s in range(seeds):
+            p4 = E.single_event(n, 2 + s % 5, 1000 * n + s, **({} if n == 3000 else {"soft_mean": 0.6, "soft_eta": 4.0}))
+            _check_event(ctx, p4, -1, radius, f"n {n} R {radius} seed {s}")
