@@ -87,11 +87,15 @@ namespace fjg {
 
 // Which events the rounds kernel takes.  Its gain is the number of steps a round
 // holds, which falls with R^2 (the area a step keeps to itself), and a round
-// costs about three steps of the step-by-step kernels.  kRoundsFew: an SM or
-// more per event, the event's latency counts; kRoundsMany: the SMs are shared,
+// costs about three steps of the step-by-step kernels.  kRoundsFew: an SM per
+// event, both kernels run it with their widest CTA; kRoundsSome: half an SM or
+// more, the event's latency counts; kRoundsMany: the SMs are shared,
 // instructions count, of which a round's fixed part is many for small events.
 // Measured (GB300; step by step -> rounds, anti-kt unless noted):
-//   one event    R 0.4: 80 particles 0.44 -> 0.50 ms, 120 0.56 -> 0.53, 250 1.18 -> 0.67, 3000 14.6 -> 4.5
+//   one event    R 0.4: 200 particles 0.60 -> 0.67 ms, 256 0.76 -> 0.64, 500 1.62 -> 0.87, 2000 8.4 -> 2.9
+//   (Few)        R 0.8: 400 1.43 -> 1.52, 500 1.81 -> 1.77, 2000 8.7 -> 7.8
+//                kt R 0.6: 150 0.52 -> 0.61, 200 0.68 -> 0.65, 2000 9.0 -> 2.7;  C/A R 0.8: 200 0.74 -> 0.71
+//   Some         R 0.4 (64 x 4 threads x slots to 512 x 8): 80 0.44 -> 0.50, 120 0.56 -> 0.53, 250 1.18 -> 0.67
 //                R 0.8: 300 1.87 -> 1.31, 3000 15.3 -> 12.4;  R 1.0: 800 4.2 -> 3.3, 1500 6.8 -> 7.9
 //                C/A R 1.2: 300 1.95 -> 1.23, 3000 16.3 -> 10.4
 //   batches      R 0.4: 2000 of 260-512 6.9 -> 6.3, 1000 of 600-1000 11.1 -> 5.9, 600 of 1100-2000 18.0 -> 6.9
@@ -99,12 +103,16 @@ namespace fjg {
 //                kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
 //                kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
 //   above 4096   R 0.4: 12,000 123 -> 31, 58,000 700 -> 285;  R 0.6: 92 -> 54;  R 0.8: 97 -> 74, where later steps conflict more often
-enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsFew = 2 };
+enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsSome = 2, kRoundsFew = 3 };
 
 __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
   if (mode == kRoundsNone) return false;
   if (n > 4096) return algo == -1 ? R <= 0.65 : R <= 1.5;
-  if (mode == kRoundsFew) return n >= 112 && (algo == -1 ? R <= 0.85 || (R <= 1.05 && n <= 1024) : R <= 1.5);
+  if (mode == kRoundsFew) {
+    if (algo == -1) return R <= 0.45 ? n >= 224 : R <= 0.65 ? n >= 320 : R <= 0.85 && n > 512;
+    return R <= 0.8 ? n >= 200 : R <= 1.2 ? n >= 320 : R <= 1.5 && n > 512;
+  }
+  if (mode == kRoundsSome) return n >= 112 && (algo == -1 ? R <= 0.85 || (R <= 1.05 && n <= 1024) : R <= 1.5);
   if (n <= 512) return n >= 400 && R <= (algo == -1 ? 0.42 : 0.6);
   return R <= (algo == -1 ? 0.55 : n <= 1024 ? 1.0 : 1.3);
 }

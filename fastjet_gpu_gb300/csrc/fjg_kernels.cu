@@ -392,6 +392,17 @@ static int bucket_grid(const Tuning& tune, int b, int num_sms, int n_events) {
   return grid < 1 ? 1 : grid;
 }
 
+// Shape of the step-by-step kernel where an event has an SM to itself: its
+// latency counts, so the widest CTA that holds the bucket's slots, two to eight a
+// thread (the configured shapes are those with the most events per second: one to
+// four merge warps, many CTAs per SM).  One event, GB300, 64 x 4 to 256 x 8 -> 256
+// x 2 to 512 x 4: 50 particles 0.33 -> 0.24 ms, 111 0.55 -> 0.38; anti-kt R = 1.2,
+// 500 3.6 -> 1.9, 1000 5.7 -> 4.2, 2000 10.1 -> 8.7.
+static int lone_variant(int b) {
+  constexpr int v[kNumBuckets] = {4, 4, 6, 8, 9};
+  return v[b];
+}
+
 // Whether the rounds kernel takes some, and all, of list q's events, as far as
 // the host knows (per-event algorithms and radii are the device's).
 static void rounds_share(const BatchArgs& A, int q, bool* some, bool* all) {
@@ -425,6 +436,7 @@ static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, 
     return launch_rounds(q, A, grid > n_events ? n_events : grid, s);
   }
   if (q == kLargeQueue) return launch_large(base, sc, n_events, num_sms, tune, s);
+  if (n_events <= num_sms) return launch_variant(lone_variant(q), A, n_events, 1, s);
   return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
 }
 
@@ -451,9 +463,10 @@ static cudaError_t launch_retries(const BatchArgs& base, const Scratch& sc, int 
   return launch_tiled(A, grid, s);
 }
 
-// Few events: each has an SM (two CTAs of the rounds kernel) to itself.
+// Few events: each has an SM to itself; some: two CTAs of the rounds kernel share
+// one.
 static int rounds_mode_of(const Scratch& sc, int n_events, int num_sms) {
-  return !sc.round_ws ? kRoundsNone : n_events <= 2 * num_sms ? kRoundsFew : kRoundsMany;
+  return !sc.round_ws ? kRoundsNone : n_events <= num_sms ? kRoundsFew : n_events <= 2 * num_sms ? kRoundsSome : kRoundsMany;
 }
 
 cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
@@ -558,7 +571,7 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
     k_cluster_tiled<<<1, kTiledT, 0, stream>>>(A);
     return cudaGetLastError();
   }
-  return launch_variant(tune.bucket[b].variant, A, 1, 1, stream);
+  return launch_variant(lone_variant(b), A, 1, 1, stream);
 }
 
 __global__ void k_kinematics(const double* p4, int n, int algo, double* rap, double* phi, double* w) {

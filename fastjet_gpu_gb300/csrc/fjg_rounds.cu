@@ -49,6 +49,12 @@ struct RoundConfig {
   int threads, tiles, cells, slots;
 };
 
+//
+// An event with an SM to itself (kRoundsFew) has the widest: one event, anti-kt R
+// = 0.4, 128 / 256 -> 512 threads: 300 particles 0.90 -> 0.71 ms, 500 1.27 -> 0.87,
+// 1000 1.61 -> 1.44, 2000 3.41 -> 2.91.
+constexpr int kWidest = 4;
+
 RoundConfig config_of(int q) {
   switch (q) {
     case 0: return {k_cluster_rounds<128, 4, true>, 128, 384, 1024, 256};
@@ -89,8 +95,9 @@ int rounds_occupancy(int q) {
 }
 
 cudaError_t launch_rounds(int q, BatchArgs A, int grid, cudaStream_t s) {
-  rounds_occupancy(q);  // sets the shared-memory attribute
-  const RoundConfig c = config_of(q);
+  const int shape = A.rounds_mode == kRoundsFew && q != kLargeQueue ? kWidest : q;
+  rounds_occupancy(shape);  // sets the shared-memory attribute
+  const RoundConfig c = config_of(shape);
   A.round_tiles = c.tiles;
   A.round_cells = c.cells;
   A.round_slots = c.slots;

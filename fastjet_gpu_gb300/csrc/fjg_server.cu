@@ -246,9 +246,9 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
   // rounds kernel left
   int taken = 0;
   if (S->d_rounds)
-    for (Req* r : L.batch) taken += fjg::rounds_take(fjg::kRoundsFew, r->n, r->algo, r->r) ? 1 : 0;
+    for (Req* r : L.batch) taken += fjg::rounds_take(fjg::kRoundsSome, r->n, r->algo, r->r) ? 1 : 0;
   if (taken) {
-    A.rounds_mode = fjg::kRoundsFew;
+    A.rounds_mode = fjg::kRoundsSome;
     fjg::BatchArgs B = A;
     B.queue = L.d_queue + 2;
     B.round_ws = S->d_rounds;

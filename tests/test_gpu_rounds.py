@@ -29,9 +29,9 @@ def _check_event(ctx, p4, algo, radius, tag):
                     out["jet_label"].cpu().numpy(), tag)
 
 
-# lists of 256 << b particles, the smallest event the kernel takes alone (112),
-# the end of the shared-memory slots (4096), an odd size above it
-SIZES = [111, 112, 255, 257, 512, 513, 1023, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 6001]
+# lists of 256 << b particles, the smallest events the kernel takes alone (224, kt
+# and C/A 200) or among some (112), the end of the shared-memory slots (4096), an odd size above it
+SIZES = [111, 112, 199, 200, 223, 224, 255, 257, 512, 513, 1023, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 6001]
 
 
 @pytest.mark.parametrize("n", SIZES)
@@ -72,11 +72,13 @@ def test_ties_go_to_the_step_by_step_kernels(ctx):
             _check_event(ctx, np.ascontiguousarray(p4), algo, 0.4, f"{name} algo {algo}")
 
 
-def test_many_events_mixed_rules(ctx):
-    """More events than share the GPU one to an SM: the other rule, per event
-    (algorithm and R from arrays), both kernels on one list; and the same batch
-    through a captured graph."""
+@pytest.mark.parametrize("count", [40, 200, 320])
+def test_many_events_mixed_rules(ctx, count):
+    """Events that have an SM each, that share one by two, and more: a rule each,
+    per event (algorithm and R from arrays), both kernels on one list; and the same
+    batch through a captured graph."""
     sizes = [5000, 3000, 2100, 1500, 1100, 900, 700, 600, 513, 512, 450, 400, 399] + [20 + i % 60 for i in range(307)]
+    sizes = sizes[:count - 8] + [250, 230, 210, 200, 190, 150, 113, 100]
     evs = [E.single_event(n, 1 + i % 4, 900 + i) for i, n in enumerate(sizes)]
     off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
     p4 = np.ascontiguousarray(np.concatenate(evs))
