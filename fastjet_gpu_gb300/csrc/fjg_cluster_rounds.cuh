@@ -48,9 +48,11 @@
 // whose minimum is the smallest of its 5x5 tiles is a candidate; it fires if
 // no tile closer to c than 1.5 R and the distance of c and j (from the point to
 // the tile) has an earlier minimum.  For kt and C/A, whose weights do not fall
-// in a merge, the range shrinks to that of pairs with d below the candidate's
-// P.  Steps a round on the benchmark's kind of events: anti-kt R = 0.4 4 at 200
-// particles, 10 at 1500, 8 to 6 at 8000 to 40,000 dense ones, R = 0.8 3; kt R =
+// in a merge, it is R and shrinks to that of pairs with d below the candidate's P
+// (48 kt events of 8000: 17.1 ms with 1.5 R, 16.0 with R; 600 events of 1500, 5.9
+// and 5.4, C/A 7.6 and 7.1; with 0.7 R conflicts come: kt 21.2 and 15.2).  Steps a
+// round on the benchmark's kind of events: anti-kt R = 0.4 4 at 200 particles, 10
+// at 1500, 8 to 6 at 8000 to 40,000 dense ones, R = 0.8 3; with 1.5 R kt R =
 // 0.6 12 at 1000, 14 at 20,000; C/A R = 0.8 8 at 1000.  Conflicts with a range of
 // 1.5 R: none in 1100 events of up to 4000 particles (anti-kt R = 0.4, kt, C/A),
 // in about 2 % of anti-kt R = 0.8 events of 3000 and in 2 to 8 % of dense anti-kt
@@ -133,9 +135,9 @@ constexpr int kRoundMaxTargets = 128;
 constexpr int kRoundSplit = 24;               // searches of a round, up to which several warps share each
 constexpr int kRoundParts = 5;                // warps that share one, at most
 constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, also in one row
-// range of the choice of steps, in units of R (see above): at first, and after a
-// conflict
-constexpr float kRoundReach = 1.5f, kRoundReachLarge = 1.8f, kRoundReachWide = 2.25f;
+// range of the choice of steps, in units of R (see above): at first (anti-kt, its
+// largest events, kt and C/A), and after a conflict
+constexpr float kRoundReach = 1.5f, kRoundReachLarge = 1.8f, kRoundReachKt = 1.0f, kRoundReachWide = 2.25f;
 constexpr int kRoundLargeFrom = 20000;
 constexpr int kRoundCareRounds = 64;          // rounds that take care, more than twice those taken back
 constexpr int kRoundMaxBacks = 8;             // conflicts of an event, and one more per 2048 particles
@@ -1405,7 +1407,9 @@ __device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, 
 }
 
 // Records of at most 4096 slots in time order: bitonic sort in shared memory
-// (the tile arrays' room).  Labels and depths are below 4096.
+// (the room of the tile arrays and of the slots' state up to `members`, which
+// takes the order).  Labels and depths are below 4096.  4000 particles: 0.55 M
+// cycles in the workspace, where the tile arrays alone were too small, now 0.2 M.
 constexpr int kRoundSortMax = 4096;
 constexpr size_t kRoundSortBytes = 14;  // per record, of a power of two
 
@@ -1611,7 +1615,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
     S.overflow = S.hopeless = S.backs = S.care = S.care_until = 0;
     S.p_min = kRoundNone;
-    S.reach = algo == -1 && N > kRoundLargeFrom ? kRoundReachLarge : kRoundReach;
+    S.reach = algo != -1 ? kRoundReachKt : N > kRoundLargeFrom ? kRoundReachLarge : kRoundReach;
     S.n_cand = S.n_fire = S.n_targets = S.n_dirty = 0;
     S.task[0] = S.task[1] = 0;
   }
@@ -2073,7 +2077,8 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   int n2 = 1;
   while (n2 < N) n2 <<= 1;
   if (n2 <= kRoundSortMax &&
-      n2 * kRoundSortBytes <= (SM ? round_tile_bytes_sm(S.tiles, S.cells) : round_tile_bytes(S.tiles, S.cells)))
+      n2 * kRoundSortBytes <= (SM ? round_tile_bytes_sm(S.tiles, S.cells) + 30 * (size_t)S.slots
+                                  : round_tile_bytes(S.tiles, S.cells)))
     round_sort_smem<SM>(C, N, n2, order);
   else
     round_sort<SM>(C, N, n2, order);
