@@ -1,4 +1,4 @@
-"""Per-step phase breakdown of the shared-memory clustering kernel on the GPU.
+"""Phase breakdown of the clustering kernels on the GPU.
 
     python -m fastjet_gpu_gb300.phases [--sizes 200,500,1000,2000,4000] [--batch 1024]
 
@@ -7,10 +7,12 @@ fastjet_gpu_gb300/_lib_phases/; the product build is untouched) and loads it
 in place of the product library.  It then clusters lone events of the given
 sizes, one event per launch (anti-kt R=0.4; the plain path, where a step's
 latency is the event's critical path; above 4096 particles pile-up-like
-events on the tiled kernel), and one batch of mixed events of 50-2000
+events), and one batch of mixed events of 50-2000
 particles (several CTAs per SM, the throughput path).  For each it prints the
-clock cycles per merge step of each phase, as counted by the kernels'
-clock64() phase counters.  Shared-memory kernel:
+clock cycles of each phase, as counted by the kernels' clock64() phase
+counters: per round for the events that the rounds kernel takes, per merge step
+for the others.  Rounds kernel (csrc/fjg_cluster_rounds.cuh names the phases):
+r_candidates and r_range (A), r_b .. r_f.  Step-by-step kernels, shared memory:
 
   s1_argmin      argmin of the keys, up to its decision (barrier B1)
   s2_merge       the merge: new jet's kinematics || target scans, up to B2
@@ -23,7 +25,7 @@ clock64() phase counters.  Shared-memory kernel:
                  closer-than-its-neighbour test, a key's pair-or-beam choice,
                  a neighbour search whose certificate failed
 
-Tiled kernel: t_rebuild (tile-list rebuilds, per step), t_s1_argmin (over the
+Step-by-step, tiled: t_rebuild (tile-list rebuilds, per step), t_s1_argmin (over the
 tile summaries), t_s2_merge_detect (merge || target detection and scans),
 t_s3_lists_targets_window (list update, targets, the new jet against its
 window), t_s3_overflow (targets beyond the listed ones, flags), t_s3c_summaries (changed tiles, the new jet's neighbour); inside t_s2:
@@ -64,6 +66,9 @@ def main():
     tiled = ["t_rebuild", "t_s1_argmin", "t_s2_merge_detect", "t_s3_lists_targets_window", "t_s3_overflow",
              "t_s3c_summaries", "t_kin_rapidity", "t_detect_s2", "t_list_update", "t_targets_warp1",
              "t_window_thread0", "t_resolve_new_jet", "t_summary_new_jet_tile", "t_summaries_warp1"]
+    # (a mark's clock is read before the barrier in front of it has opened: part of
+    # the wait for a phase's slowest warp counts in the next phase)
+    rounds = ["r_candidates", "r_range", "r_b", "r_c", "r_d", "r_e", "r_f"]
     rows = []
 
     def report(tag, c):
@@ -88,6 +93,15 @@ def main():
             print(f"{tag:>28}: " + "  ".join(f"{k} {row[k]:8.0f}" for k in tiled + ["t_step_total"]) +
                   f"  targets per step {row['t_targets_per_step']:.2f}, steps with targets "
                   f"{row['t_steps_with_targets']:.2f}", flush=True)
+        if c["r_rounds"]:
+            n = c["r_rounds"]
+            row.update({"r_rounds": n, "r_events": c["r_events"], "r_steps_per_round": c["r_steps"] / n})
+            row.update({k: c[k] / n for k in rounds})
+            row["r_round_total"] = sum(row[k] for k in rounds)
+            row.update({k: c[k] for k in ("r_setup", "r_sort", "r_outputs", "r_backs", "r_retries")})
+            print(f"{tag:>28}: " + "  ".join(f"{k} {row[k]:8.0f}" for k in rounds + ["r_round_total"]) +
+                  f"  rounds {n}, steps per round {row['r_steps_per_round']:.2f}, set-up {c['r_setup']}, sort "
+                  f"{c['r_sort']}, conflicts {c['r_backs']}, left to the other kernels {c['r_retries']}", flush=True)
         rows.append(row)
 
     for n in [int(x) for x in args.sizes.split(",") if x]:

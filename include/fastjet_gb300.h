@@ -46,7 +46,8 @@ typedef enum {
 
 /* Largest event the library clusters (particles per event); larger events
  * are refused with FJG_ETOOBIG.  Events above 4096 particles also need the
- * tiled kernel's workspace (96 bytes per particle of the batch). */
+ * tiled kernel's workspace (96 bytes per particle of the batch); the rounds
+ * kernel's (384 bytes per particle) is used where it can be allocated. */
 #define FJG_MAX_EVENT_PARTICLES 16777216
 
 /* I/O record of the reference (PseudoJet.h:4-11): 40 bytes, px at offset 8. */
@@ -210,7 +211,10 @@ void fjg_graph_destroy(fjg_graph* graph);
  * fit); events above 4096 particles run on the tiled kernel with a grid of
  * large_ctas_per_sm CTAs per SM (one is resident per SM) and rapidity-azimuth
  * tiles of side at least tile_factor * R (tile_factor >= 1), larger where an
- * event is sparse (about 32 particles per tile).  Every choice gives identical
+ * event is sparse (about 32 particles per tile).  The choice concerns events
+ * that are clustered step by step in calls of more events than the GPU has SMs:
+ * in smaller calls each event has the widest CTA, and the events that the rounds
+ * kernel takes have shapes of their own.  Every choice gives identical
  * results; only the speed differs. */
 #define FJG_NUM_BUCKETS 5
 typedef struct {
