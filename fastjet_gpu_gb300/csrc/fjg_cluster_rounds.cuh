@@ -104,12 +104,15 @@ namespace fjg {
 //                R 0.6: 1000 of 600-1000 11.1 -> 9.3, 600 of 1100-2000 17.8 -> 17.9
 //                kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
 //                kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
-//   above 4096   R 0.4: 12,000 123 -> 31, 58,000 700 -> 285;  R 0.6: 92 -> 54;  R 0.8: 97 -> 74, where later steps conflict more often
+//   above 4096   R 0.4: 12,000 123 -> 31, 58,000 700 -> 285, 250,000 6760 -> 3190;  R 0.6: 100,000 2350 -> 1610
+//                R 0.8: 4500 44.5 -> 26, 12,000 141 -> 89, 30,000 528 -> 394;  R 1.0: 44.7 -> 36, 165 -> 124, 658 -> 546
+//                R 1.2: 46 -> 40 to 46, 187 -> 150 to 199 (conflicts), 804 -> 694
+//                kt R 1.8: 63.7 -> 40, 310 -> 178, 1498 -> 869;  C/A R 2.0: 72.6 -> 45.5, 376 -> 209, 1895 -> 1045
 enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsSome = 2, kRoundsFew = 3 };
 
 __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
   if (mode == kRoundsNone) return false;
-  if (n > 4096) return algo == -1 ? R <= 0.65 : R <= 1.5;
+  if (n > 4096) return R <= (algo == -1 ? 1.05 : 2.0);
   if (mode == kRoundsFew) {
     if (algo == -1) return R <= 0.45 ? n >= 224 : R <= 0.65 ? n >= 320 : R <= 0.85 && n > 512;
     return R <= 0.8 ? n >= 200 : R <= 1.2 ? n >= 320 : R <= 1.5 && n > 512;

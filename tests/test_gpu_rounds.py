@@ -107,3 +107,10 @@ def test_steps_taken_back(ctx):
         for s in range(seeds):
             p4 = E.single_event(n, 2 + s % 5, 1000 * n + s, **({} if n == 3000 else {"soft_mean": 0.6, "soft_eta": 4.0}))
             _check_event(ctx, p4, -1, radius, f"n {n} R {radius} seed {s}")
+
+
+@pytest.mark.parametrize("algo,radius", [(-1, 1.05), (-1, 1.06), (1, 1.8), (0, 2.0), (0, 2.01)])
+def test_large_radii_above_4096(ctx, algo, radius):
+    """Few tiles around in azimuth (six at R = 2), and both sides of the rule's
+    largest radii for events above 4096 particles."""
+    _check_event(ctx, E.single_event(4200, 4, 11, soft_mean=0.6, soft_eta=4.0), algo, radius, f"algo {algo} R {radius}")
