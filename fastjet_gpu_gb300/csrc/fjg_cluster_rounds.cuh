@@ -302,6 +302,7 @@ struct RoundShared {
   EventCtx X;
   unsigned char* ws;
   float r2hi;  // R^2 rounded up, a little more
+  float far2;  // two slots whose FP32 coordinates are further apart (squared) are beyond R
   int tiles, cells, slots;  // room
   double rmin, inv_side_r, inv_side_phi;
   float rmin32, side_r, side_phi;
@@ -413,8 +414,14 @@ __device__ __forceinline__ int round_v(const RoundShared& S, double phi) {
   return v < 0 ? 0 : (v >= S.nphi ? S.nphi - 1 : v);
 }
 
-// R^2 and more than the FP32 distances' error.
-__device__ __forceinline__ float round_far2(const RoundShared& S) { return S.r2hi * 1.001f + 1e-6f; }
+// S.far2 for an event with |rapidity| up to rmax.  An FP32 coordinate is off by
+// 2^-24 of itself (a rapidity of 1e5, of a particle on the beam line, by 0.004),
+// so two slots within R can be 2^-23 (rmax + 4 pi) further apart in FP32; twice
+// that, and 1e-3 and 1e-6 for the rounding of the distance and of the tiles' edges.
+__device__ __forceinline__ float round_far2(float r2hi, double rmax) {
+  const double d = sqrt((double)r2hi) + 0x1p-22 * (rmax + 12.6);
+  return __double2float_ru(d * d * 1.001 + 1e-6);
+}
 
 // A box of tiles: nu rows from u0, nv columns from v0 (wrapping; nv <= 9).
 struct RoundBox {
@@ -479,7 +486,7 @@ __device__ __forceinline__ void for_tiles(const RoundCtx<SM>& C, const RoundBox&
     constexpr int B = 3;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1, upto = below | (1u << lane);
-    const float far2 = round_far2(S);
+    const float far2 = S.far2;
     int* shift = C.shift + (threadIdx.x & ~31);
 #pragma unroll 1
     for (; k0 < n; k0 += 32) {
@@ -1316,7 +1323,7 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
   const Ws_& Wk = C.W;
   const int lane = threadIdx.x & 31;
   const Bound bd = S.X.bd;
-  const float ilo = S.X.ilo, r2hi = S.r2hi, far2 = round_far2(S);
+  const float ilo = S.X.ilo, r2hi = S.r2hi, far2 = S.far2;
 #pragma unroll 1
   for (;;) {
     int i = 0;
@@ -1354,7 +1361,7 @@ __device__ __forceinline__ void round_phase_b(const RoundCtx<SM>& C, int F, int 
                 Wk.nn(y) = (typename Ws_::Idx)(s.nn | Ws_::kTarget);
                 round_target(S, y);
               }
-              // beyond R of c and of j (the FP32 distance is good to 1e-5 there)?
+              // beyond R of c and of j (round_far2)?
               if (fminf(plain_dr2(gc, s.g), plain_dr2(gj, s.g)) > far2) return;
               const float w = round_wlo(s.w);
 #pragma unroll 1
@@ -1575,6 +1582,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
       rmax = fmax(rmax, S.red[2][k]);
     }
     S.X.bd = make_bound(rmax);
+    S.far2 = round_far2(S.r2hi, rmax);
     lo = fmax(lo, -15.0);
     hi = fmin(hi, 15.0);
     if (!(hi >= lo)) hi = lo;

@@ -1,0 +1,45 @@
+"""The rounds kernel (csrc/fjg_cluster_rounds.cuh) on inputs at the ends of the
+number range, against the CPU oracle bit for bit."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not torch.cuda.is_available(), reason="needs a GPU")]
+
+import fastjet_gpu_gb300 as F  # noqa: E402
+import gpu_util as U  # noqa: E402
+from fastjet_gpu_gb300 import events as E  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return F.Context(0)
+
+
+def _check_event(ctx, p4, algo, radius, tag):
+    out = ctx.cluster_event(torch.from_numpy(p4).cuda(), algo, radius, history=True, owner=True)
+    U.compare_event(p4, algo, radius, out["jets"].cpu().numpy(), int(out["n_jets"][0]),
+                    F.history_records(out["history"]), out["owner"].cpu().numpy(),
+                    out["jet_label"].cpu().numpy(), tag)
+
+
+def _on_the_beam(pz):
+    """Particles without pT and mass: their rapidity is 1e5 + |pz|."""
+    pz = np.asarray(pz, np.float64)
+    return np.stack([0 * pz, 0 * pz, pz, np.abs(pz)], 1)
+
+
+# the smallest event alone that the kernel takes, slots in shared memory and in the workspace
+@pytest.mark.parametrize("n", [224, 600, 4200])
+def test_particles_on_the_beam_line(ctx, n):
+    """Rapidities of 1e5, where FP32 coordinates are 2^-7 apart: particles just
+    within R of one another, whose weights are all the same 1e300."""
+    base = E.single_event(n, 3, 91 + n)
+    rng = np.random.default_rng(n)
+    chains = [[10.8019, 10.4024, 10.0038]]
+    chains += [rng.uniform(1, 50) + np.cumsum(rng.uniform(0.37, 0.402, 7)) * rng.choice([-1, 1]) for _ in range(6)]
+    for i, pz in enumerate(chains):
+        pz = np.asarray(pz) * (1 if i % 2 == 0 else -1)
+        for algo in (-1, 0, 1):
+            _check_event(ctx, np.concatenate([_on_the_beam(pz), base]), algo, 0.4, f"n {n} chain {i} algo {algo}")
