@@ -297,7 +297,8 @@ __device__ __forceinline__ double exact_key(SmemLayout<T, SPT>& S, const EventCt
 // certificate: returns the slot (or -1) and the dR2 interval.  All 32 lanes of
 // the calling warp call.  When the certificate fails (near-tie), every
 // candidate whose lower bound does not exceed the best upper bound is
-// evaluated in FP64 and the exact minimum (dR2, label) wins.
+// evaluated in FP64 and the exact minimum (dR2, label) wins; a NaN upper bound
+// (two slots of infinite rapidity) excludes none, so one is always found.
 template <int T, int SPT>
 __device__ __forceinline__ int resolve_nn(SmemLayout<T, SPT>& S, const EventCtx& X, int t, int n, const Cert& c,
                                           float& lo_out, float& hi_out) {
@@ -319,7 +320,7 @@ __device__ __forceinline__ int resolve_nn(SmemLayout<T, SPT>& S, const EventCtx&
     if (u == t) continue;
     float lo, hi;
     dr2_32(rt, pt, S.rap32[u], S.phi32[u], X.bd, lo, hi);
-    if (lo <= c.u1) {
+    if (!(lo > c.u1)) {
       const unsigned long long k = dbits(dr2_slots(X.g, t, u));
       if (arg_less(k, S.label[u], bk, bl)) {
         bk = k;
@@ -518,7 +519,7 @@ __device__ void cluster_event_smem(SmemLayout<T, SPT>& S, const BatchArgs& A, in
         if (u == t) continue;
         float lo, hi;
         dr2_32(rt, pt, S.rap32[u], S.phi32[u], X.bd, lo, hi);
-        if (lo <= c.u1) {
+        if (!(lo > c.u1)) {
           const unsigned long long du = dbits(dr2_slots(g, t, u));
           if (arg_less(du, S.label[u], bk, bl)) {
             bk = du;

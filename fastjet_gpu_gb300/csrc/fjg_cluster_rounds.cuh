@@ -414,6 +414,14 @@ __device__ __forceinline__ int round_v(const RoundShared& S, double phi) {
   return v < 0 ? 0 : (v >= S.nphi ? S.nphi - 1 : v);
 }
 
+// What this kernel leaves to the step-by-step kernels.  A weight of 0 (kt without
+// pT: a pair distance of 0 at any distance) or one that overflowed; a rapidity that
+// did (no pT and E < |pz| gives +-infinity, sums beyond 1e154 NaN), or whose FP32
+// distances could: a NaN bound certifies no neighbour, and the FP64 search that
+// follows would find none within it.  Below 1e30 bounds may be infinite, never NaN.
+__device__ __forceinline__ bool round_refuses(double w) { return !(w > 0.0 && w <= 1.7976931348623157e308); }
+__device__ __forceinline__ bool round_refuses_rap(double rap) { return !(fabs(rap) < 1e30); }
+
 // S.far2 for an event with |rapidity| up to rmax.  An FP32 coordinate is off by
 // 2^-24 of itself (a rapidity of 1e5, of a particle on the beam line, by 0.004),
 // so two slots within R can be 2^-23 (rmax + 4 pi) further apart in FP32; twice
@@ -662,7 +670,7 @@ __device__ __noinline__ int round_exact(int t, float u1) {
           [&](int u, float2 gu) {
             float l, h;
             dr2_32(gt.x, gt.y, gu.x, gu.y, bd, l, h);
-            if (u == t || !(l <= u1)) return;
+            if (u == t || l > u1) return;
             const unsigned long long k = dbits(C.W.dr2(t, u));
             if (arg_less(k, u, bk, bi)) {
               bk = k;
@@ -1535,7 +1543,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
 
   // ---- load and kinematics
   double rlo = 1e300, rhi = -1e300, amax = 0.0;
-  bool weightless = false;  // a pair distance of 0 at any distance (kt, no pT): left to the other kernels
+  bool refused = false;  // left to the other kernels (round_refuses)
 #pragma unroll 1
   for (int s = tid; s < N; s += T) {
     const double* p = A.p4 + (off + s) * A.p4_stride;
@@ -1556,7 +1564,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     rlo = fmin(rlo, kin.rap);
     rhi = fmax(rhi, kin.rap);
     amax = fmax(amax, fabs(kin.rap));
-    weightless |= !(kin.w > 0.0);
+    refused |= round_refuses(kin.w) || round_refuses_rap(kin.rap);
   }
 #pragma unroll 1
   for (int o = 16; o; o >>= 1) {
@@ -1572,7 +1580,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
   for (int k = tid; k < kRoundSmemMaxN / 32; k += T) S.taken[k] = S.claimed[k] = 0;
   if (tid < 16) S.lut[tid] = tid ? (65536 + tid - 1) / tid : 0;
-  if (__syncthreads_or(weightless)) return false;
+  if (__syncthreads_or(refused)) return false;
   if (tid == 0) {
     double lo = 1e300, hi = -1e300, rmax = 0.0;
 #pragma unroll 1
@@ -1858,7 +1866,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
             const double w =
                 fjk_weight(__dadd_rn(Wk.p4(0, c), Wk.p4(0, j)), __dadd_rn(Wk.p4(1, c), Wk.p4(1, j)), algo);
             S.w[i] = w;
-            if (!(w > 0.0)) S.conflict[1] = S.hopeless = 1;
+            if (round_refuses(w)) S.conflict[1] = S.hopeless = 1;
           }
           RoundRec r;
           r.M = S.M[i];
@@ -1894,6 +1902,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         } else {
           const double pz = __dadd_rn(Wk.p4(2, c), Wk.p4(2, j)), E = __dadd_rn(Wk.p4(3, c), Wk.p4(3, j));
           const double rap = fjk_rap(px, py, pz, E);
+          if (round_refuses_rap(rap)) S.conflict[1] = S.hopeless = 1;
           S.p4[0][i] = px;
           S.p4[1][i] = py;
           S.p4[2][i] = pz;

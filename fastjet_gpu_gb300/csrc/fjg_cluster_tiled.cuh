@@ -472,7 +472,7 @@ __device__ __forceinline__ int resolve_large(const TiledShared& S, const LargeWs
   auto consider = [&](int u) {
     float lo, hi;
     dr2_32(rt, pt, L.rap32[u], L.phi32[u], X.bd, lo, hi);
-    if (lo <= c.u1) {
+    if (!(lo > c.u1)) {  // (a NaN bound excludes none)
       const unsigned long long k = dbits(dr2_ws(X.g, t, u));
       if (arg_less(k, u, bk, bi)) {
         bk = k;
@@ -806,7 +806,7 @@ __device__ inline void cluster_event_tiled(TiledShared& S, const BatchArgs& A, u
           if (u < 0 || u == t) continue;
           float lo, hi;
           dr2_32(rt, pt, L.rap32[u], L.phi32[u], X.bd, lo, hi);
-          if (lo <= c.u1) {
+          if (!(lo > c.u1)) {  // (a NaN bound excludes none)
             const unsigned long long du = dbits(dr2_ws(g, t, u));
             if (arg_less(du, u, bk, bi)) {
               bk = du;

@@ -43,3 +43,33 @@ def test_particles_on_the_beam_line(ctx, n):
         pz = np.asarray(pz) * (1 if i % 2 == 0 else -1)
         for algo in (-1, 0, 1):
             _check_event(ctx, np.concatenate([_on_the_beam(pz), base]), algo, 0.4, f"n {n} chain {i} algo {algo}")
+
+
+# (alone: the rounds kernel's sizes, which hands such an event on; 100 and R = 3: the step-by-step kernels at once)
+@pytest.mark.parametrize("n,radius", [(100, 0.4), (300, 0.4), (1500, 3.0), (4200, 0.4), (4200, 3.0)])
+def test_infinite_rapidity(ctx, n, radius):
+    """No pT and E below |pz| (rounded input): the rapidity is infinite, and so is
+    the distance to everything; two of them are a NaN apart.  Every neighbour
+    search has to find some slot all the same."""
+    p4 = E.single_event(n, 3, 17 + n)
+    beam = _on_the_beam([20.0, 30.0, -7.0, -8.0, 3.0])
+    beam[:, 3] *= 1.0 - 2.0 ** -40
+    for at in (0, n // 2, n):
+        p = np.concatenate([p4[:at], beam, p4[at:]])
+        for algo in (-1, 0):
+            _check_event(ctx, p, algo, radius, f"n {n} R {radius} at {at} algo {algo}")
+
+
+def test_sums_that_overflow(ctx):
+    """A merged jet's pT^2 or E that is beyond the number range: its rapidity is
+    infinite or NaN.  Such an event gives some result or an error, and the next
+    one is clustered as ever."""
+    base = E.single_event(400, 3, 23)
+    for scale in (1e153, 1e154, 1e200):
+        for algo in (-1, 0, 1):
+            try:
+                out = ctx.cluster_event(torch.from_numpy(base * scale).cuda(), algo, 0.4)
+                assert 0 <= int(out["n_jets"][0]) <= base.shape[0]
+            except F.FjgError:
+                pass
+    _check_event(ctx, base, -1, 0.4, "after")
