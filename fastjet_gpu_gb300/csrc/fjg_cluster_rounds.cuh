@@ -35,13 +35,13 @@
 // T(x, y) >= d_xy, so with thr = k for the one whose own time sets a chained
 // T(E) and thr = T(E)'s key part for the other, a pair is a conflict only if
 // d_xy <= thr (an exact tie counts), d_xy is at most both weights and the other
-// is not younger than E.  After a conflict the steps from the one that
-// came too early on are taken back (round_undo) and its slot is held until the
-// other step's time; where that is not enough, a wider range follows, and rounds
-// of the one earliest step, which cannot conflict but for exact ties.  Those, and
-// events with too many conflicts, are handed to the step-by-step kernel (retry
-// list) and this kernel's work is dropped.  So the rule that picks the steps of a
-// round only has to be good, not proven.
+// is not younger than E.  After a conflict the line of steps that came too
+// early (round_line) and all that was fired since are taken back (round_undo), and
+// its slots are held until the other step's time; where that is not enough, a wider
+// range follows, and rounds of the one earliest step, which cannot conflict but for
+// exact ties.  Those, and events with too many conflicts, are handed to the
+// step-by-step kernel (retry list) and this kernel's work is dropped.  So the rule
+// that picks the steps of a round only has to be good, not proven.
 //
 // Choice of a round's steps.  Tiles of side >= R/2; per tile the slot with the
 // smallest (P, key), P being the FP32 lower bound of its step's time.  A tile
@@ -57,8 +57,8 @@
 // 1.5 R: none in 1100 events of up to 4000 particles (anti-kt R = 0.4, kt, C/A),
 // in about 2 % of anti-kt R = 0.8 events of 3000 and in 2 to 8 % of dense anti-kt
 // R = 0.4 events of 8000 to 15,000; those of 40,000 and more, where a hard jet's
-// chain of steps reaches further, have one or several.  A conflict there costs
-// 100 to 4000 rounds, so events above 20,000 begin with 1.8 R: 64 events of
+// chain of steps reaches further, have one or several.  A conflict costs 30 to 900
+// rounds (6000 to 10,000 dense particles), so events above 20,000 begin with 1.8 R: 64 events of
 // 10,000 to 60,000 particles have 3 to 11 conflicts (10 samples) and take 314 to
 // 330 ms, 333 to 345 with 2.0 R, 308 to 434 with 1.5 R.
 //
@@ -194,7 +194,7 @@ struct alignas(16) RoundSlot {
   float tlo;  // birth time's M, rounded down
   int at;     // position in its tile's list
   int parent;  // (output) what the slot was merged into, or its jet
-  float hold;  // a step of this slot with P from here on waits until all P are
+  float hold;  // a step of this slot with P from here on waits until all P are above it (0: none)
   int pad[2];
 };
 
@@ -316,6 +316,10 @@ struct RoundShared {
   // every thread of the CTA takes the same way
   int conflict[3];
   int back;  // round to go back to
+  // of the steps found to be too early: round and slot of the first, and the latest
+  // time (M, rounded down) that they should have waited for
+  unsigned long long early;
+  int hold;
   int hopeless, alive, backs;
   // rounds before `care_until` take care: 1: the wide range; 2: one step, that
   // with the earliest time
@@ -1026,9 +1030,9 @@ __device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) 
           const RoundRec q = C.W.rec(y >> 1);
           if (time_less(RoundTime{M, l, depth}, RoundTime{q.M, q.l, q.depth})) {
             bad = true;
-            atomicMin(&C.S->back, q.round);
             // (both positive: ordered as integers)
-            atomicMax(reinterpret_cast<int*>(&C.W.slots[y >> 1].hold), __float_as_int(m_lo * (1.0f - 0x1p-13f)));
+            atomicMin(&C.S->early, (unsigned long long)q.round << 32 | (unsigned)(y >> 1));
+            atomicMax(&C.S->hold, __float_as_int(m_lo));
           }
         }
         y = C.W.dnext(y);
@@ -1038,6 +1042,29 @@ __device__ __noinline__ bool round_d2(int x, int a, double M, int l, int depth) 
     x = r.x;
   }
   return bad;
+}
+
+// What came too early (whole CTA): the first such step and all of its line (the
+// steps of the same M and l, which a jet takes one after another: while its first
+// one stands, the others' turn seems to have come).  Their first round is where to
+// go back to, and their slots are held.  (Back to that one step, with its slot
+// held: up to ten conflicts with one line, each a few of its steps further back.)
+template <bool SM>
+__device__ __noinline__ void round_line() {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  RoundShared& S = *C.S;
+  if (S.early == ~0ull) return;
+  const RoundRec first = C.W.rec((int)(unsigned)S.early);
+#pragma unroll 1
+  for (int s = threadIdx.x; s < S.X.N; s += blockDim.x) {
+    if (C.W.tile(s) != (typename RoundWs<SM>::Idx)RoundWs<SM>::kNone) continue;
+    const RoundRec r = C.W.rec(s);
+    if (r.M != first.M || r.l != first.l) continue;
+    atomicMin(&S.back, r.round);
+    atomicMax(reinterpret_cast<int*>(&C.W.slots[s].hold), S.hold);
+    if (r.a >= 0) atomicMax(reinterpret_cast<int*>(&C.W.slots[r.a].hold), S.hold);
+  }
+  __syncthreads();
 }
 
 // What the time of a step is made of: of c and of its partner j.
@@ -1087,6 +1114,13 @@ __device__ __forceinline__ RoundStep round_step(int c, int j, const RoundPair& p
   s.chained = s.t.M < tp.M || (s.t.M == tp.M && s.t.l <= tp.l);
   if (s.chained) s.t = RoundTime{tp.M, tp.l, tp.depth + 1};
   return s;
+}
+
+// Whether a step of time P has to wait: its slots are held until nothing with a
+// time up to `hold` (0: not held) is left, and the earliest step of all never is.
+// The bounds on times are good to 2^-15.
+__device__ __forceinline__ bool round_held(float hold, float P, float p_min) {
+  return hold > 0.0f && P >= hold * (1.0f - 0x1p-13f) && p_min < P && p_min <= hold * (1.0f + 0x1p-13f);
 }
 
 // The order of steps: those of the same time follow the same one, the smallest
@@ -1666,6 +1700,8 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   if (tid == 0) {
     S.n_dirty = 0;
     S.back = 0x7fffffff;
+    S.early = ~0ull;
+    S.hold = 0;
   }
   FJG_PH(mark(kPhRSetup);)
 
@@ -1787,7 +1823,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         const int bc = round_bit<SM>(c), bj = round_bit<SM>(jc);
         bool ok = care == 2;
         if (SM) pair = round_pair(Wk, c, jc);
-        if (!ok && !(__uint_as_float(me) >= pair.hold && __uint_as_float(S.p_min) < pair.hold)) {
+        if (!ok && !round_held(pair.hold, __uint_as_float(me), __uint_as_float(S.p_min))) {
           ok = round_first(S.taken, min(bc, bj));
           if (ok && bc != bj) ok = round_first(S.taken, max(bc, bj));
         }
@@ -2068,8 +2104,9 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   }
   __syncthreads();
   if (!(S.conflict[0] | S.conflict[1] | S.conflict[2])) break;
-  // back to before the step that came too early (D1, and D2 within a round: this
+  // back to before the steps that came too early (D1, and D2 within a round: this
   // round's), and from there with more care
+  round_line<SM>();
   const int r0 = min(S.back, round);
   const bool again = round < S.care_until;
   const int care = !S.conflict[2] ? 2 : !again ? 0 : round - r0 <= 4 * kRoundCareRounds ? 2 : 1;
