@@ -89,37 +89,65 @@ namespace fjg {
 
 // Which events the rounds kernel takes.  Its gain is the number of steps a round
 // holds, which falls with R^2 (the area a step keeps to itself), and a round
-// costs about three steps of the step-by-step kernels.  kRoundsFew: an SM per
-// event, both kernels run it with their widest CTA; kRoundsSome: half an SM or
-// more, the event's latency counts; kRoundsMany: the SMs are shared,
-// instructions count, of which a round's fixed part is many for small events.
-// Measured (GB300; step by step -> rounds, anti-kt unless noted):
-//   one event    R 0.4: 200 particles 0.60 -> 0.67 ms, 256 0.76 -> 0.64, 500 1.62 -> 0.87, 2000 8.4 -> 2.9
-//   (Few)        R 0.8: 400 1.43 -> 1.52, 500 1.81 -> 1.77, 2000 8.7 -> 7.8
-//                kt R 0.6: 150 0.52 -> 0.61, 200 0.68 -> 0.65, 2000 9.0 -> 2.7;  C/A R 0.8: 200 0.74 -> 0.71
-//   Some         R 0.4 (64 x 4 threads x slots to 512 x 8): 80 0.44 -> 0.50, 120 0.56 -> 0.53, 250 1.18 -> 0.67
-//                R 0.8: 300 1.87 -> 1.31, 3000 15.3 -> 12.4;  R 1.0: 800 4.2 -> 3.3, 1500 6.8 -> 7.9
-//                C/A R 1.2: 300 1.95 -> 1.23, 3000 16.3 -> 10.4
-//   batches      R 0.4: 2000 of 260-512 6.9 -> 6.3, 1000 of 600-1000 11.1 -> 5.9, 600 of 1100-2000 18.0 -> 6.9
-//                R 0.6: 1000 of 600-1000 11.1 -> 9.3, 600 of 1100-2000 17.8 -> 17.9
-//                kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
-//                kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
-//   above 4096   R 0.4: 12,000 123 -> 31, 58,000 700 -> 285, 250,000 6760 -> 3190;  R 0.6: 100,000 2350 -> 1610
-//                R 0.8: 4500 44.5 -> 26, 12,000 141 -> 89, 30,000 528 -> 394;  R 1.0: 44.7 -> 36, 165 -> 124, 658 -> 546
-//                R 1.2: 46 -> 40 to 46, 187 -> 150 to 199 (conflicts), 804 -> 694
-//                kt R 1.8: 63.7 -> 40, 310 -> 178, 1498 -> 869;  C/A R 2.0: 72.6 -> 45.5, 376 -> 209, 1895 -> 1045
-enum { kRoundsNone = 0, kRoundsMany = 1, kRoundsSome = 2, kRoundsFew = 3 };
+// costs about three steps of the step-by-step kernels.
+//   One    a single event, in the widest CTA of either kernel.
+//   Few    up to an SM per event, and Some, half an SM: the call lasts as long as
+//          its slowest event, one with conflicts, or one left to the step-by-step
+//          kernel after all, so the rounds have to win by more than in the mean.
+//   Many   the SMs are shared, instructions count, of which a round's fixed part is
+//          many for small events.
+//   ServeOne, Serve   a server's micro-batch of one request, and of several: as One
+//          and Few, but the step-by-step kernels run in the shapes with the most
+//          events per second, and the rounds kernel with 128 to 512 threads.
+// Measured on GB300, rounds / step by step (in its best shape but for the server),
+// anti-kt unless noted.  One: 24 events, mean (worst).  Few and Some: calls of 20 to
+// 300 events of a size, best to worst of the calls.  Serve: bursts of 16, 64 and 170
+// requests of a size, the burst's time.
+//   One    R 0.4: 160 0.98 (1.36), 200 0.85 (1.24), 256 0.69 (0.96), 1000 0.36;  R 0.6: 256 0.79 (1.04), 320 0.74 (0.94)
+//          R 0.8: 512 0.92 (1.14), 1000 0.82 (0.98), 3000 0.88 (1.01);  R 1.0: 512 1.22, 2000 1.33
+//          kt R 0.6: 200 0.72 (0.95), R 1.0: 320 0.64 (0.83), R 1.3: 600 0.77 (0.90), R 1.5: 700 0.92, 3000 1.03
+//          C/A R 0.8: 160 0.80, R 1.2: 320 0.74 (0.93)
+//   Few,   R 0.4: 200 1.15-1.38, 256 1.02-1.12 (Some: 1.04-1.26), 320 0.76-0.86, 1000 0.37-0.53;  R 0.5: 320 0.76-0.94
+//   Some   R 0.6: 320 0.89-1.06, 512 0.78-0.99, 600 0.68-0.82;  R 0.7: 600 0.83-0.95, 2000 0.77-0.89
+//          R 0.8: 320 1.15-1.31, 1000 0.89-1.02, 3000 0.87-1.11
+//          kt R 0.6: 256 0.84-1.03, 320 0.63-0.84, R 1.0: 320 0.82-1.09, 700 0.59-0.71, R 1.3: 600 0.87-0.99,
+//          R 1.5: 700 1.04-1.17;  C/A R 0.8: 256 0.87-1.18, 320 0.71-0.92, R 1.2: 512 0.80-1.05, 700 0.72-0.88
+//   Many   (ms) R 0.4: 2000 of 260-512 6.9 -> 6.3, 1000 of 600-1000 11.1 -> 5.9, 600 of 1100-2000 18.0 -> 6.9
+//          R 0.6: 1000 of 600-1000 11.1 -> 9.3, 600 of 1100-2000 17.8 -> 17.9
+//          kt R 0.6: 3000 of 150-256 4.7 -> 7.1, 1000 of 600-1000 9.8 -> 5.7
+//          kt R 1.0: 1000 of 600-1000 9.9 -> 9.6, 600 of 1100-2000 17.8 -> 10.4;  C/A R 1.2: 10.1 -> 14.5, 18.3 -> 12.8
+//   ServeOne  R 0.4: 112 0.87, 400 0.42;  R 0.8: 112 0.92, 1000 0.64, 4000 0.87;  R 1.0: 112 1.15, 1500 1.00
+//          kt R 1.2: 112 0.84, 1000 0.55;  C/A R 1.2: 112 0.91, 1000 0.52
+//   Serve  R 0.4: 200 1.48 1.22 1.12, 400 1.10 0.76 0.79, 512 1.01 0.62 0.79, 1000 0.62 0.43 0.73
+//          R 0.5: 700 1.22 0.64 0.98, 1000 0.81 0.61 0.78, 1500 1.00 0.74 0.71;  R 0.6: 1500 1.16 0.90 0.87
+//          kt R 0.6: 512 0.89 0.62 0.77;  R 1.0: 700 1.37 0.73 0.90, 1000 0.91 0.67 0.85, 1500 1.08 0.80 0.81
+//          C/A R 0.8: 512 0.96 0.53 0.76, R 1.2: 1500 1.28 0.96 0.95
+//   above 4096   alone / calls of 40 to 320:  R 0.4: 0.20-0.24 / 0.17-0.32;  R 0.8: 0.47-0.63 / 0.42-0.76
+//                R 1.0: 0.64-0.83 (0.91) / 0.85-1.20;  R 1.05: 0.70-0.87 (0.97) / 0.91-1.05
+//                kt R 1.5: 0.40-0.48 / 0.35-0.54, R 2.0: 0.54-0.64 / 0.50-0.70;  C/A R 2.0: 0.53-0.63 / 0.50-0.68
+//                (ms) R 0.4: 12,000 123 -> 31, 58,000 700 -> 285, 250,000 6760 -> 3190;  R 0.6: 100,000 2350 -> 1610
+enum { kRoundsNone = 0, kRoundsMany, kRoundsSome, kRoundsFew, kRoundsOne, kRoundsServe, kRoundsServeOne };
 
+// In each mode the rule falls with R, and with n it changes at most once among the
+// sizes of one list (rounds_share counts on both).
 __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
   if (mode == kRoundsNone) return false;
-  if (n > 4096) return R <= (algo == -1 ? 1.05 : 2.0);
-  if (mode == kRoundsFew) {
-    if (algo == -1) return R <= 0.45 ? n >= 224 : R <= 0.65 ? n >= 320 : R <= 0.85 && n > 512;
-    return R <= 0.8 ? n >= 200 : R <= 1.2 ? n >= 320 : R <= 1.5 && n > 512;
+  const bool antikt = algo == -1, alone = mode == kRoundsOne || mode == kRoundsServeOne;
+  if (n > 4096) return R <= (!antikt ? 2.0 : alone ? 1.05 : 0.85);
+  switch (mode) {
+    case kRoundsOne:
+      if (antikt) return R <= 0.45 ? n >= 224 : R <= 0.65 ? n >= 320 : R <= 0.85 && n > 512;
+      return R <= 0.8 ? n >= 200 : R <= 1.3 && n >= 320;
+    case kRoundsFew:
+      if (R <= (antikt ? 0.45 : 0.8)) return n > 256;
+      return R <= (antikt ? 0.55 : 1.0) ? n >= 320 : R <= (antikt ? 0.7 : 1.3) && n >= 600;
+    case kRoundsSome: return R <= (antikt ? 0.55 : 0.8) ? n >= 320 : R <= (antikt ? 0.7 : 1.3) && n >= 600;
+    case kRoundsServeOne: return R <= (antikt ? 0.85 : 1.2) && n >= 112;
+    case kRoundsServe: return R <= (antikt ? 0.45 : 0.8) ? n > 512 : R <= (antikt ? 0.55 : 1.0) && n >= 1000;
+    default:
+      if (n <= 512) return n >= 400 && R <= (antikt ? 0.42 : 0.6);
+      return R <= (antikt ? 0.55 : n <= 1024 ? 1.0 : 1.3);
   }
-  if (mode == kRoundsSome) return n >= 112 && (algo == -1 ? R <= 0.85 || (R <= 1.05 && n <= 1024) : R <= 1.5);
-  if (n <= 512) return n >= 400 && R <= (algo == -1 ? 0.42 : 0.6);
-  return R <= (algo == -1 ? 0.55 : n <= 1024 ? 1.0 : 1.3);
 }
 
 // The same for an event of a batch.

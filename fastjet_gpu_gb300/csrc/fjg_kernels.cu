@@ -392,16 +392,20 @@ static int bucket_grid(const Tuning& tune, int b, int num_sms, int n_events) {
   return grid < 1 ? 1 : grid;
 }
 
-// Shape of the step-by-step kernel where an event has an SM to itself: its
-// latency counts, so the widest CTA that holds the bucket's slots, two to eight a
-// thread (the configured shapes are those with the most events per second: one to
-// four merge warps, many CTAs per SM).  One event, GB300, 64 x 4 to 256 x 8 -> 256
-// x 2 to 512 x 4: 50 particles 0.33 -> 0.24 ms, 111 0.55 -> 0.38; anti-kt R = 1.2,
-// 500 3.6 -> 1.9, 1000 5.7 -> 4.2, 2000 10.1 -> 8.7.
+// Shape of the step-by-step kernel where an event has an SM to itself, or (lists of
+// up to 1024 particles) half of one: its latency counts, so the widest CTA that
+// holds the bucket's slots, two to eight a thread (the configured shapes are those
+// with the most events per second: one to four merge warps, many CTAs per SM).
+// GB300, 64 x 4 to 256 x 8 -> 256 x 2 to 512 x 4: one event of 50 particles 0.33 ->
+// 0.24 ms, 111 0.55 -> 0.38; anti-kt R = 1.2, 500 3.6 -> 1.9, 1000 5.7 -> 4.2, 2000
+// 10.1 -> 8.7.  Calls of 160 and 300 events, widest / configured: 100 particles 0.71
+// and 0.81, 256 0.71 and 0.84, 512 0.67 and 0.57, 1000 0.83; of 1500 particles (512
+// threads, one CTA per SM) 1.44: those keep their shape.
 static int lone_variant(int b) {
   constexpr int v[kNumBuckets] = {4, 4, 6, 8, 9};
   return v[b];
 }
+constexpr int kSharedBuckets = 3;  // two CTAs of lone_variant share an SM
 
 // Whether the rounds kernel takes some, and all, of list q's events, as far as
 // the host knows (per-event algorithms and radii are the device's).
@@ -436,7 +440,8 @@ static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, 
     return launch_rounds(q, A, grid > n_events ? n_events : grid, s);
   }
   if (q == kLargeQueue) return launch_large(base, sc, n_events, num_sms, tune, s);
-  if (n_events <= num_sms) return launch_variant(lone_variant(q), A, n_events, 1, s);
+  if (n_events <= num_sms || (n_events <= 2 * num_sms && q < kSharedBuckets))
+    return launch_variant(lone_variant(q), A, n_events, 1, s);
   return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
 }
 
@@ -463,10 +468,11 @@ static cudaError_t launch_retries(const BatchArgs& base, const Scratch& sc, int 
   return launch_tiled(A, grid, s);
 }
 
-// Few events: each has an SM to itself; some: two CTAs of the rounds kernel share
-// one.
+// The rounds kernel's rule by the number of events (rounds_take).
 static int rounds_mode_of(const Scratch& sc, int n_events, int num_sms) {
-  return !sc.round_ws ? kRoundsNone : n_events <= num_sms ? kRoundsFew : n_events <= 2 * num_sms ? kRoundsSome : kRoundsMany;
+  if (!sc.round_ws) return kRoundsNone;
+  if (n_events == 1) return kRoundsOne;
+  return n_events <= num_sms ? kRoundsFew : n_events <= 2 * num_sms ? kRoundsSome : kRoundsMany;
 }
 
 cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
@@ -552,8 +558,8 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
   A.queue = sc.queues;
   A.ws = sc.ws;
   A.ws_stride = sc.ws_stride;
-  if (sc.round_ws && rounds_take(kRoundsFew, n, base.algo_all, base.r_all)) {
-    A.rounds_mode = kRoundsFew;
+  if (sc.round_ws && rounds_take(kRoundsOne, n, base.algo_all, base.r_all)) {
+    A.rounds_mode = kRoundsOne;
     const int q = b < 0 ? kLargeQueue : b, r = b < 0 ? kRetryLargeQueue : kRetryQueue;
     A.round_ws = sc.round_ws;
     A.retry = sc.order + r * sc.cap_events;

@@ -50,7 +50,7 @@ struct RoundConfig {
 };
 
 //
-// An event with an SM to itself (kRoundsFew) has the widest: one event, anti-kt R
+// An event with an SM to itself (kRoundsFew, kRoundsOne) has the widest: one event, anti-kt R
 // = 0.4, 128 / 256 -> 512 threads: 300 particles 0.90 -> 0.71 ms, 500 1.27 -> 0.87,
 // 1000 1.61 -> 1.44, 2000 3.41 -> 2.91.
 constexpr int kWidest = 4;
@@ -95,7 +95,8 @@ int rounds_occupancy(int q) {
 }
 
 cudaError_t launch_rounds(int q, BatchArgs A, int grid, cudaStream_t s) {
-  const int shape = A.rounds_mode == kRoundsFew && q != kLargeQueue ? kWidest : q;
+  const bool alone = A.rounds_mode == kRoundsFew || A.rounds_mode == kRoundsOne;
+  const int shape = alone && q != kLargeQueue ? kWidest : q;
   rounds_occupancy(shape);  // sets the shared-memory attribute
   const RoundConfig c = config_of(shape);
   A.round_tiles = c.tiles;

@@ -244,11 +244,12 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
   };
   // the rounds kernel's events (the latency rule), the others, and what the
   // rounds kernel left
+  const int mode = m == 1 ? fjg::kRoundsServeOne : fjg::kRoundsServe;
   int taken = 0;
   if (S->d_rounds)
-    for (Req* r : L.batch) taken += fjg::rounds_take(fjg::kRoundsSome, r->n, r->algo, r->r) ? 1 : 0;
+    for (Req* r : L.batch) taken += fjg::rounds_take(mode, r->n, r->algo, r->r) ? 1 : 0;
   if (taken) {
-    A.rounds_mode = fjg::kRoundsSome;
+    A.rounds_mode = mode;
     fjg::BatchArgs B = A;
     B.queue = L.d_queue + 2;
     B.round_ws = S->d_rounds;
