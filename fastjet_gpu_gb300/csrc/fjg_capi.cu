@@ -50,16 +50,17 @@ cudaError_t ScratchSet::reserve_lists(int n_events) {
   if (sc.order && sc.cap_events >= n_events) return cudaSuccess;
   int cap = n_events + n_events / 4 + 64;
   const size_t hist_bytes = (sizeof(int32_t) * kHistBins + 255) & ~size_t(255);
-  size_t bytes = sizeof(int32_t) * (size_t)kNumLists * cap + 256 + hist_bytes;
+  size_t bytes = sizeof(int32_t) * (size_t)kNumLists * cap + 512 + hist_bytes;
   cudaError_t err = lists.reserve(bytes);
   if (err != cudaSuccess) return err;
   char* p = static_cast<char*>(lists.ptr);
   sc.offsets1 = reinterpret_cast<int64_t*>(p);
   sc.counts = reinterpret_cast<int32_t*>(p + 64);
   sc.queues = reinterpret_cast<int*>(p + 128);
-  sc.status = reinterpret_cast<int*>(p + 192);
-  sc.hist = reinterpret_cast<int32_t*>(p + 256);
-  sc.order = reinterpret_cast<int32_t*>(p + 256 + hist_bytes);
+  static_assert(sizeof(int32_t) * kNumLists <= 64 && sizeof(int) * (kNumLists + kNumQueues) <= 128, "their room");
+  sc.status = reinterpret_cast<int*>(p + 256);
+  sc.hist = reinterpret_cast<int32_t*>(p + 512);
+  sc.order = reinterpret_cast<int32_t*>(p + 512 + hist_bytes);
   sc.cap_events = cap;
   err = cudaMemset(sc.status, 0, sizeof(int));
   if (err == cudaSuccess) err = cudaDeviceSynchronize();

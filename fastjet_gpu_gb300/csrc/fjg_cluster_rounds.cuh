@@ -1642,7 +1642,10 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
   for (int k = tid; k < kRoundSmemMaxN / 32; k += T) S.taken[k] = S.claimed[k] = 0;
   if (tid < 16) S.lut[tid] = tid ? (65536 + tid - 1) / tid : 0;
-  if (__syncthreads_or(refused)) return false;
+  if (__syncthreads_or(refused)) {
+    FJG_PH(if (A.phase && tid == 0) atomicAdd(A.phase + kPhRRetries, 1ull);)
+    return false;
+  }
   if (tid == 0) {
     double lo = 1e300, hi = -1e300, rmax = 0.0;
 #pragma unroll 1

@@ -39,7 +39,6 @@ fjg_status fjg_graph_capture_batch(fjg_ctx* ctx, const double* p4, const int64_t
   for (int b = 0; b < fjg::kNumBuckets && err == cudaSuccess; ++b) fjg::variant_occupancy(ctx->tune.bucket[b].variant);
   if (err == cudaSuccess) err = fjg::configure_tiled();
   for (int q = 0; q < fjg::kNumQueues && err == cudaSuccess; ++q) fjg::rounds_occupancy(q);
-  fjg::variant_occupancy(fjg::kRetryVariant);
   fjg::launch_priority(0);
   if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
   if (err != cudaSuccess) {

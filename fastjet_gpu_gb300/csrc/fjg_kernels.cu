@@ -300,7 +300,7 @@ static cudaError_t launch_sort(const BatchArgs& base, const Scratch& sc, int n_e
   cudaError_t err;
   if ((err = cudaMemsetAsync(sc.hist, 0, sizeof(int32_t) * kHistBins, stream)) != cudaSuccess) return err;
   if ((err = cudaMemsetAsync(sc.queues, 0, sizeof(int) * (sc.round_ws ? kNumLists + kNumQueues : kNumQueues), stream)) != cudaSuccess) return err;
-  if ((err = cudaMemsetAsync(sc.counts + kLargeQueue, 0, sizeof(int32_t) * (sc.round_ws ? 3 : 1), stream)) != cudaSuccess) return err;
+  if ((err = cudaMemsetAsync(sc.counts + kLargeQueue, 0, sizeof(int32_t) * (sc.round_ws ? kNumLists - kLargeQueue : 1), stream)) != cudaSuccess) return err;
   const int grid = (n_events + 255) / 256 < 1 ? 1 : ((n_events + 255) / 256 > 1024 ? 1024 : (n_events + 255) / 256);
   const int64_t limit = base.particles < sc.ws_stride ? base.particles : sc.ws_stride;
   k_check_args<<<grid, 256, 0, stream>>>(base.offsets, n_events, base.n_jets, limit, base.algo, base.radius);
@@ -318,15 +318,8 @@ static cudaError_t launch_sort(const BatchArgs& base, const Scratch& sc, int n_e
 
 // The large list: one CTA per event, a few per SM at most (the events are
 // few and long; the small buckets fill the rest of each SM).
-static cudaError_t launch_large(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms,
-                                const Tuning& tune, cudaStream_t s) {
-  if (!sc.large_ws) return cudaSuccess;
-  BatchArgs A = base;
-  A.order = sc.order + kLargeQueue * sc.cap_events;
-  A.n_order = sc.counts + kLargeQueue;
-  A.queue = sc.queues + kLargeQueue;
-  A.ws = sc.ws;
-  A.ws_stride = sc.ws_stride;
+static cudaError_t launch_large(BatchArgs A, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
+                                cudaStream_t s) {
   A.large_ws = sc.large_ws;
   A.tile_factor = tune.tile_factor;
   int grid = tune.large_ctas_per_sm * num_sms;
@@ -420,52 +413,38 @@ static void rounds_share(const BatchArgs& A, int q, bool* some, bool* all) {
   *all = at_lo && at_hi;
 }
 
-// List q (a bucket, or kLargeQueue) of a batch: the rounds kernel for its
-// events, or the step-by-step kernel for the others.
-static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, int n_events, int num_sms,
-                               const Tuning& tune, bool rounds, cudaStream_t s) {
+// The launches of list q (a bucket, or kLargeQueue) of a batch: the rounds kernel
+// for its events, the step-by-step kernel for the others, and the step-by-step
+// kernel, in the list's shape, for the events that the rounds kernel left (mostly
+// none: it ends at once).  One launch of 512 threads per event for all lists, after
+// the last of them, took 19.2 ms instead of 9.0 for 1024 kt events of 700 particles of
+// which each has one without pT, 32.8 instead of 20.8 for C/A events with particles on a
+// lattice; and cost a captured graph of 662 events that uses no rounds 2.2 of 15.7 ms.
+// In the CTA of the rounds, whose shape is not made for it: 12.7 and 29.2.
+enum ListPart { kPartRounds, kPartSteps, kPartRetry };
+
+static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, ListPart part, int n_events,
+                               int num_sms, const Tuning& tune, cudaStream_t s) {
   BatchArgs A = base;
-  A.order = sc.order + q * sc.cap_events;
-  A.n_order = sc.counts + q;
-  A.queue = sc.queues + q;
+  const int list = part == kPartRetry ? retry_list(q) : q;
+  A.order = sc.order + list * sc.cap_events;
+  A.n_order = sc.counts + list;
+  A.queue = sc.queues + list;
   A.ws = sc.ws;
   A.ws_stride = sc.ws_stride;
-  if (rounds) {
-    const int r = q == kLargeQueue ? kRetryLargeQueue : kRetryQueue;
+  if (part == kPartRounds) {
     A.queue = sc.queues + kNumLists + q;
     A.round_ws = sc.round_ws;
-    A.retry = sc.order + r * sc.cap_events;
-    A.n_retry = sc.counts + r;
+    A.retry = sc.order + retry_list(q) * sc.cap_events;
+    A.n_retry = sc.counts + retry_list(q);
     const int grid = num_sms * rounds_occupancy(q);
     return launch_rounds(q, A, grid > n_events ? n_events : grid, s);
   }
-  if (q == kLargeQueue) return launch_large(base, sc, n_events, num_sms, tune, s);
+  if (part == kPartRetry) A.rounds_mode = kRoundsNone;
+  if (q == kLargeQueue) return launch_large(A, sc, n_events, num_sms, tune, s);
   if (n_events <= num_sms || (n_events <= 2 * num_sms && q < kSharedBuckets))
     return launch_variant(lone_variant(q), A, n_events, 1, s);
   return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
-}
-
-// The events the rounds kernels left: almost always none, then both launches
-// end at once.
-static cudaError_t launch_retries(const BatchArgs& base, const Scratch& sc, int n_events, int num_sms,
-                                  cudaStream_t s) {
-  if (base.rounds_mode == kRoundsNone) return cudaSuccess;
-  BatchArgs A = base;
-  A.rounds_mode = kRoundsNone;
-  A.order = sc.order + kRetryQueue * sc.cap_events;
-  A.n_order = sc.counts + kRetryQueue;
-  A.queue = sc.queues + kRetryQueue;
-  A.ws = sc.ws;
-  A.ws_stride = sc.ws_stride;
-  const int grid = n_events < num_sms ? n_events : num_sms;
-  cudaError_t err = launch_variant(kRetryVariant, A, grid, 1, s);
-  if (err != cudaSuccess || !sc.large_ws) return err;
-  A.order = sc.order + kRetryLargeQueue * sc.cap_events;
-  A.n_order = sc.counts + kRetryLargeQueue;
-  A.queue = sc.queues + kRetryLargeQueue;
-  A.large_ws = sc.large_ws;
-  A.tile_factor = 1.0;
-  return launch_tiled(A, grid, s);
 }
 
 // The rounds kernel's rule by the number of events (rounds_take).
@@ -480,44 +459,31 @@ cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events,
   BatchArgs base = args;
   base.rounds_mode = rounds_mode_of(sc, n_events, num_sms);
   cudaError_t err = launch_sort(base, sc, n_events, stream);
-  if (err != cudaSuccess) return err;
-  if ((err = cudaEventRecord(*ev_fork, stream)) != cudaSuccess) return err;
+  if (err == cudaSuccess && side) err = cudaEventRecord(*ev_fork, stream);
   // largest events first: their list is launched first.  A list that both
   // kernels work on has them side by side (the rounds kernel's streams come
-  // first).
-  for (int q = kLargeQueue; q >= 0; --q) {
+  // first); what the rounds kernel leaves follows it on its stream.
+  for (int q = kLargeQueue; q >= 0 && err == cudaSuccess; --q) {
     if (q == kLargeQueue && !sc.large_ws) continue;
     bool some, all;
     rounds_share(base, q, &some, &all);
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 2 && err == cudaSuccess; ++k) {
       if (k == 0 ? !some : all) continue;
       const int i = q + (k ? kNumQueues : 0);
       cudaStream_t s = side ? side[i] : stream;
-      if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) return err;
-      if ((err = launch_list(base, sc, q, n_events, num_sms, tune, k == 0, s)) != cudaSuccess) return err;
-      if (side) {
-        if ((err = cudaEventRecord(ev_join[i], s)) != cudaSuccess) return err;
-        if ((err = cudaStreamWaitEvent(stream, ev_join[i], 0)) != cudaSuccess) return err;
-      }
+      if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) break;
+      err = launch_list(base, sc, q, k ? kPartSteps : kPartRounds, n_events, num_sms, tune, s);
+      if (err == cudaSuccess && k == 0) err = launch_list(base, sc, q, kPartRetry, n_events, num_sms, tune, s);
+      if (err == cudaSuccess && side) err = cudaEventRecord(ev_join[i], s);
+      if (err == cudaSuccess && side) err = cudaStreamWaitEvent(stream, ev_join[i], 0);
     }
   }
-  return launch_retries(base, sc, n_events, num_sms, stream);
+  return err;
 }
 
 cudaError_t launch_batch_on_stream(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms,
                                    const Tuning& tune, cudaStream_t stream) {
-  BatchArgs base = args;
-  base.rounds_mode = rounds_mode_of(sc, n_events, num_sms);
-  cudaError_t err = launch_sort(base, sc, n_events, stream);
-  if (err != cudaSuccess) return err;
-  for (int q = kLargeQueue; q >= 0; --q) {
-    if (q == kLargeQueue && !sc.large_ws) continue;
-    bool some, all;
-    rounds_share(base, q, &some, &all);
-    if (some && (err = launch_list(base, sc, q, n_events, num_sms, tune, true, stream)) != cudaSuccess) return err;
-    if (!all && (err = launch_list(base, sc, q, n_events, num_sms, tune, false, stream)) != cudaSuccess) return err;
-  }
-  return launch_retries(base, sc, n_events, num_sms, stream);
+  return launch_batch(args, sc, n_events, num_sms, tune, stream, nullptr, nullptr, nullptr);
 }
 
 // The single-event path's descriptors and input check in one launch: an event
@@ -560,7 +526,7 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
   A.ws_stride = sc.ws_stride;
   if (sc.round_ws && rounds_take(kRoundsOne, n, base.algo_all, base.r_all)) {
     A.rounds_mode = kRoundsOne;
-    const int q = b < 0 ? kLargeQueue : b, r = b < 0 ? kRetryLargeQueue : kRetryQueue;
+    const int q = b < 0 ? kLargeQueue : b, r = retry_list(q);
     A.round_ws = sc.round_ws;
     A.retry = sc.order + r * sc.cap_events;
     A.n_retry = sc.counts + r;

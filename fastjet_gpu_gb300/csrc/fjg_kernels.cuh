@@ -19,11 +19,10 @@ constexpr int kSmemMaxN = 4096;
 // kernel (one CTA of 256 threads per event, state in the large workspace).
 constexpr int kLargeQueue = kNumBuckets;
 constexpr int kNumQueues = kNumBuckets + 1;
-// Two more lists: events that the rounds kernel left to the step-by-step
-// kernels, of up to kSmemMaxN particles and above.
-constexpr int kRetryQueue = kNumQueues;
-constexpr int kRetryLargeQueue = kNumQueues + 1;
-constexpr int kNumLists = kNumQueues + 2;
+// A second list for each: events that the rounds kernel left to the step-by-step
+// kernels.
+__host__ __device__ inline int retry_list(int q) { return kNumQueues + q; }
+constexpr int kNumLists = 2 * kNumQueues;
 // Side streams of a batch: per list one for each of its two kernels.
 constexpr int kNumSide = 2 * kNumQueues;
 constexpr int kLargeMaxN = 1 << 24;
@@ -66,7 +65,6 @@ __host__ __device__ inline VariantShape variant_shape(int v) {
 // Launch configuration the autotuner chooses: per bucket a variant and the
 // CTAs per SM of its persistent grid (0: as many as fit), the CTAs per SM of
 // the tiled kernel, and its tile side in units of R (>= 1).
-constexpr int kRetryVariant = 9;  // any event of up to kSmemMaxN particles
 struct BucketConfig {
   int variant;
   int ctas_per_sm;

@@ -10,6 +10,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -59,6 +60,48 @@ def test_steps_taken_back(counters):
         assert e["r_undone"] < e["r_rounds"] / 2, e
 
 
+# (one event; an SM each; an SM for two; many)
+@pytest.mark.parametrize("count", [1, 60, 200, 330])
+def test_events_left_to_the_other_kernels(counters, count):
+    """Particles without pT (kt), and particles on a lattice (ties): events that the
+    rounds hand on, from every list, beside events that they keep."""
+    sizes = [5000, 4097, 4000, 2100, 2048, 1500, 1025, 1024, 700, 600, 513, 512, 450] * 20 + [256, 200, 100] * 24
+    sizes = sizes[:count - 3] + [700, 2049, 300] if count > 1 else [700]
+    batch, = counters([{"sizes": sizes, "algo": 1, "radius": 0.6, "kinds": ["no pT", "lattice", "jets"]}])
+    row, = batch
+    assert row["r_retries"] > 0
+    assert row["r_events"] > 0 or count == 1
+    # every event is clustered by one kernel, and only what that one hands on by a second
+    assert row["events"] + row["t_events"] + row["r_events"] == count
+    assert row["events"] + row["t_events"] >= row["r_retries"]
+
+
+def _particles(kind, n, i):
+    from fastjet_gpu_gb300 import events as E
+    if kind == "lattice":
+        r = np.random.default_rng(i)
+        y, phi, pt = r.integers(-30, 31, n) * 0.125, r.integers(0, 50, n) * 0.125, r.integers(1, 8, n) * 0.5
+        return np.stack([pt * np.cos(phi), pt * np.sin(phi), pt * np.sinh(y), pt * np.cosh(y)], 1)
+    p4 = E.single_event(n, 1 + i % 5, 5000 * n + i)
+    if kind == "no pT":
+        p4[n // 2, :2] = 0.0
+    return p4
+
+
+def _batch(ctx, g):
+    import gpu_util as U
+    evs = [_particles(g["kinds"][i % len(g["kinds"])], n, i) for i, n in enumerate(g["sizes"])]
+    off = np.concatenate([[0], np.cumsum(g["sizes"])]).astype(np.int64)
+    ctx.phase_clocks(reset=True)
+    res = ctx.cluster_batch(np.concatenate(evs), off, g["algo"], g["radius"], history=True, owner=True)
+    counts = ctx.phase_clocks()
+    for e, p4 in enumerate(evs):
+        s = slice(off[e], off[e + 1])
+        U.compare_event(p4, g["algo"], g["radius"], res["jets"][s], res["n_jets"][e], res["history"][s],
+                        res["owner"][s], res["jet_label"][s], f"event {e} of {len(p4)}")
+    return counts
+
+
 def _main(groups):
     import torch
 
@@ -69,7 +112,9 @@ def _main(groups):
     out = []
     for g in groups:
         rows = []
-        for i in g["which"]:
+        if "sizes" in g:
+            rows.append(_batch(ctx, g))
+        for i in g.get("which", []):
             n = g["n"]
             p4 = E.single_event(n, 1 + i % 5, 5000 * n + i, **(DENSE if g.get("dense") else {}))
             ctx.phase_clocks(reset=True)
