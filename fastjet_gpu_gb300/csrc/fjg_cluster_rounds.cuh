@@ -171,6 +171,14 @@ constexpr int kRoundMaxCand = 704;            // 5x5 minima among 2048 tiles, al
 constexpr float kRoundReach = 1.5f, kRoundReachLarge = 1.8f, kRoundReachKt = 1.0f, kRoundReachWide = 2.25f;
 constexpr int kRoundLargeFrom = 20000;
 constexpr int kRoundCareRounds = 64;          // rounds that take care, more than twice those taken back
+// Particles on a lattice (calorimeter towers) have many neighbours as far as another,
+// whose steps' times tie in FP32: one conflict after the other.  An event in which
+// more than one slot in kRoundTies has two such neighbours at first is left to the
+// other kernels (events of free directions have none).  GB300, C/A R = 0.8, 0.087 x
+// 0.087, step by step / in rounds until given up / left at once, ms: 1024 events of 700
+// 13.2 / 20.0 / 14.2, of 1500 54.5 / 65.5 / 56.3; 100 of 700 4.5 / 6.2 / 3.9.  0.005 x 0.005,
+// one in 300: 1024 of 1500 38.4 / 26.2 / -, kept.
+constexpr int kRoundTies = 128;
 constexpr int kRoundMaxBacks = 8;             // conflicts of an event, and one more per 2048 particles
 constexpr int kRoundMaxTiles = 2048;
 constexpr int kRoundMaxCells = 3072;          // with the frame
@@ -349,6 +357,7 @@ struct RoundShared {
   unsigned long long early;
   int hold;
   int hopeless, alive, backs;
+  int ties;  // searches with two neighbours as far
   // rounds before `care_until` take care: 1: the wide range; 2: one step, that
   // with the earliest time
   int care, care_until;
@@ -688,7 +697,8 @@ __device__ __noinline__ void round_set(int t, int nn, float lo, float hi, int ke
 }
 
 // Slot t's neighbour by the exact minimum (dR2, label) over its window (whole
-// warp), among those whose FP32 lower bound does not exceed u1.
+// warp), among those whose FP32 lower bound does not exceed u1.  Counts in S.ties if
+// the second one is as far, in FP32.
 template <bool SM>
 __device__ __noinline__ int round_exact(int t, float u1) {
   const RoundCtx<SM> C = round_ctx<SM>();
@@ -696,7 +706,7 @@ __device__ __noinline__ int round_exact(int t, float u1) {
   const RoundBox b = round_box(*C.S, tile, tile);
   const float2 gt = C.W.xy(t);
   const Bound bd = C.S->X.bd;
-  unsigned long long bk = ~0ull;
+  unsigned long long bk = ~0ull, b2 = ~0ull;
   int bi = 0x7fffffff;
   for_box(C, b, 32, gt, [&](int, float2 g) { return g; },
           [&](int u, float2 gu) {
@@ -705,11 +715,18 @@ __device__ __noinline__ int round_exact(int t, float u1) {
             if (u == t || l > u1) return;
             const unsigned long long k = dbits(C.W.dr2(t, u));
             if (arg_less(k, u, bk, bi)) {
+              b2 = bk;
               bk = k;
               bi = u;
+            } else if (k < b2) {
+              b2 = k;
             }
           });
-  return arg_warp(bk, bi, bi).idx;
+  const Arg r = arg_warp(bk, bi, bi);
+  const double best = __longlong_as_double((long long)r.key);
+  const double next = __longlong_as_double((long long)(bi == r.idx ? b2 : bk));  // (~0: a NaN)
+  if (__any_sync(kFull, next - best <= best * 0x1p-22) && (threadIdx.x & 31) == 0) atomicAdd(&C.S->ties, 1);
+  return r.idx;
 }
 
 // Stores slot t's neighbour from its group's certificate (every lane calls;
@@ -1697,7 +1714,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
     S.side_r = (float)(1.0 / S.inv_side_r);
     S.side_phi = (float)(1.0 / S.inv_side_phi);
     S.conflict[0] = S.conflict[1] = S.conflict[2] = 0;
-    S.overflow = S.hopeless = S.backs = S.care = S.care_until = 0;
+    S.overflow = S.hopeless = S.backs = S.ties = S.care = S.care_until = 0;
     S.p_min = kRoundNone;
     S.reach = algo != -1 ? kRoundReachKt : N > kRoundLargeFrom ? kRoundReachLarge : kRoundReach;
     S.n_cand = S.n_fire = S.n_targets = S.n_dirty = 0;
@@ -1725,6 +1742,10 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   // ---- neighbours (round_set marks tiles as changed: cleared after)
   round_init(C, n >= kRoundDense * nt);
   __syncthreads();
+  if (round == 0 && S.ties > 1 + N / kRoundTies) {
+    FJG_PH(if (A.phase && tid == 0) atomicAdd(A.phase + kPhRRetries, 1ull);)
+    return false;
+  }
   for (int t = tid; t < nt; t += T) round_summary_thread<SM>(t);
   for (int k = tid; k < kRoundMaxTiles / 32; k += T) S.dirty_bits[k] = 0;
   __syncthreads();

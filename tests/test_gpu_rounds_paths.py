@@ -76,6 +76,16 @@ def test_events_left_to_the_other_kernels(counters, count):
     assert row["events"] + row["t_events"] >= row["r_retries"]
 
 
+def test_lattice_is_left_at_once(counters):
+    """Neighbours at the same distance by the hundred: no round is tried."""
+    for algo, radius in ((-1, 0.4), (0, 0.8)):
+        batch, = counters([{"sizes": [700, 1024, 1500, 3000, 5000], "algo": algo, "radius": radius,
+                            "kinds": ["lattice"]}])
+        row, = batch
+        assert row["r_retries"] == 5 and row["events"] + row["t_events"] == 5
+        assert row["r_conflict_a"] + row["r_conflict_b"] + row["r_conflict_d"] + row["r_events"] == 0
+
+
 def _particles(kind, n, i):
     from fastjet_gpu_gb300 import events as E
     if kind == "lattice":
