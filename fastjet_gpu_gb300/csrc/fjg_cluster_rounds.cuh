@@ -1503,16 +1503,14 @@ __device__ __forceinline__ void round_new_jet(const RoundCtx<SM>& C, bool have, 
   round_settle<SM>(have, (lane & (G - 1)) == 0, a, ca, Ws_::kTarget);
 }
 
-// Records of at most 4096 slots in time order: bitonic sort in shared memory
-// (the room of the tile arrays and of the slots' state up to `members`, which
-// takes the order).  Labels and depths are below 4096.  4000 particles: 0.55 M
-// cycles in the workspace, where the tile arrays alone were too small, now 0.2 M.
-constexpr int kRoundSortMax = 4096;
-constexpr size_t kRoundSortBytes = 14;  // per record, of a power of two
-
-template <bool SM>
-__device__ __forceinline__ void round_sort_smem(const RoundCtx<SM>& C, int N, int n2,
-                                                typename RoundWs<SM>::Idx* order) {
+// Records of an event with its slots in shared memory in time order: bitonic sort
+// there (in the room of the tile arrays and of the slots' state up to `members`,
+// which takes the order: 30 bytes a slot and more, for 14 a record; the slots are a
+// power of two).  Labels and depths are below 4096.  4000 particles: 0.2 M cycles,
+// 0.55 M in the workspace.
+__device__ __forceinline__ void round_sort_smem(const RoundCtx<true>& C, int N, int n2,
+                                                RoundWs<true>::Idx* order) {
+  static_assert(kRoundSlotBytes - RoundWs<true>::kRoom * sizeof(RoundWs<true>::Idx) >= 14, "room for the sort");
   const int T = blockDim.x;
   unsigned long long* M = reinterpret_cast<unsigned long long*>(C.tmin);
   unsigned* sec = reinterpret_cast<unsigned*>(M + n2);
@@ -1560,9 +1558,8 @@ __device__ __forceinline__ void round_sort_smem(const RoundCtx<SM>& C, int N, in
 // Any number of records, in the workspace.  The first stride of a size pairs
 // mirrored entries, so that every run ascends and the missing entries past N
 // act as the largest.
-template <bool SM>
-__device__ __forceinline__ void round_sort(const RoundCtx<SM>& C, int N, int n2, typename RoundWs<SM>::Idx* order) {
-  using Idx = typename RoundWs<SM>::Idx;
+__device__ __forceinline__ void round_sort(const RoundCtx<false>& C, int N, int n2, RoundWs<false>::Idx* order) {
+  using Idx = RoundWs<false>::Idx;
   const int T = blockDim.x;
   for (int s = threadIdx.x; s < N; s += T) order[s] = (Idx)s;
   __syncthreads();
@@ -2185,12 +2182,10 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
   Idx* order = Wk.members;
   int n2 = 1;
   while (n2 < N) n2 <<= 1;
-  if (n2 <= kRoundSortMax &&
-      n2 * kRoundSortBytes <= (SM ? round_tile_bytes_sm(S.tiles, S.cells) + 30 * (size_t)S.slots
-                                  : round_tile_bytes(S.tiles, S.cells)))
-    round_sort_smem<SM>(C, N, n2, order);
+  if constexpr (SM)
+    round_sort_smem(C, N, n2, order);
   else
-    round_sort<SM>(C, N, n2, order);
+    round_sort(C, N, n2, order);
   FJG_PH(mark(kPhRSort);)
   // ---- outputs
   int jets = 0;
