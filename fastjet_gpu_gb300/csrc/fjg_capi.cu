@@ -45,61 +45,6 @@ fjg_status status_to_error(fjg_ctx* ctx, int st) {
 
 bool valid_algo(int a) { return a == FJG_KT || a == FJG_CAM || a == FJG_ANTIKT; }
 
-cudaError_t ScratchSet::reserve_lists(int n_events) {
-  if (n_events < 1) n_events = 1;
-  if (sc.order && sc.cap_events >= n_events) return cudaSuccess;
-  int cap = n_events + n_events / 4 + 64;
-  const size_t hist_bytes = (sizeof(int32_t) * kHistBins + 255) & ~size_t(255);
-  size_t bytes = sizeof(int32_t) * (size_t)kNumLists * cap + 512 + hist_bytes;
-  cudaError_t err = lists.reserve(bytes);
-  if (err != cudaSuccess) return err;
-  char* p = static_cast<char*>(lists.ptr);
-  sc.offsets1 = reinterpret_cast<int64_t*>(p);
-  sc.counts = reinterpret_cast<int32_t*>(p + 64);
-  sc.queues = reinterpret_cast<int*>(p + 128);
-  static_assert(sizeof(int32_t) * kNumLists <= 64 && sizeof(int) * (kNumLists + kNumQueues) <= 128, "their room");
-  sc.status = reinterpret_cast<int*>(p + 256);
-  sc.hist = reinterpret_cast<int32_t*>(p + 512);
-  sc.order = reinterpret_cast<int32_t*>(p + 512 + hist_bytes);
-  sc.cap_events = cap;
-  err = cudaMemset(sc.status, 0, sizeof(int));
-  if (err == cudaSuccess) err = cudaDeviceSynchronize();
-  return err;
-}
-
-cudaError_t ScratchSet::reserve_ws(int64_t particles) {
-  if (particles < 1) particles = 1;
-  if (sc.ws && sc.ws_stride >= particles) return cudaSuccess;
-  const int64_t stride = particles + particles / 4 + 1024;
-  cudaError_t err = ws.reserve(sizeof(double) * kWsFields * (size_t)stride);
-  if (err != cudaSuccess) return err;
-  sc.ws = static_cast<double*>(ws.ptr);
-  sc.ws_stride = (int64_t)(ws.cap / (sizeof(double) * kWsFields));
-  return cudaSuccess;
-}
-
-cudaError_t ScratchSet::reserve_large(int64_t particles) {
-  if (particles <= kSmemMaxN) return cudaSuccess;
-  if (sc.large_ws && sc.large_ws_particles >= particles) return cudaSuccess;
-  cudaError_t err = large.reserve((size_t)kLargeWsBytesPerParticle * (size_t)particles + 256);
-  if (err != cudaSuccess) return err;
-  sc.large_ws = static_cast<unsigned char*>(large.ptr);
-  sc.large_ws_particles = (int64_t)((large.cap - 256) / kLargeWsBytesPerParticle);
-  return cudaSuccess;
-}
-
-void ScratchSet::reserve_rounds(int64_t particles) {
-  if (sc.round_ws && sc.round_ws_particles >= particles) return;
-  sc.round_ws = nullptr;
-  sc.round_ws_particles = 0;
-  if (rounds.reserve((size_t)kRoundBytesPerParticle * (size_t)particles + 256) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  sc.round_ws = static_cast<unsigned char*>(rounds.ptr);
-  sc.round_ws_particles = (int64_t)((rounds.cap - 256) / kRoundBytesPerParticle);
-}
-
 }  // namespace fjg
 
 using fjg::cuda_error;
@@ -160,7 +105,7 @@ fjg_status fjg_ctx_create(int device, fjg_ctx** out) {
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&ctx->ev_join[b], cudaEventDisableTiming);
   }
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
-  if (err == cudaSuccess) err = ctx->scratch.reserve_lists(1024);
+  if (err == cudaSuccess) err = ctx->scratch.reserve(1024, 0, false);
 #ifdef FJG_PHASE_CLOCKS
   if (err == cudaSuccess) err = cudaMalloc(&ctx->phase, sizeof(unsigned long long) * fjg::kPhSlots);
   if (err == cudaSuccess) err = cudaMemset(ctx->phase, 0, sizeof(unsigned long long) * fjg::kPhSlots);
@@ -227,10 +172,8 @@ fjg_status fjg_cluster_batch(fjg_ctx* ctx, const double* p4, const int64_t* offs
   if (!algo && !valid_algo(algo_all)) return set_error(ctx, FJG_EINVAL, "bad algorithm");
   if (!radius && !fjg::valid_radius(r_all)) return set_error(ctx, FJG_EINVAL, "R must be finite and >= 0");
   DeviceGuard g(ctx->device);
-  cudaError_t err = ctx->scratch.reserve_lists(n_events);
-  if (err == cudaSuccess) err = ctx->scratch.reserve_ws(total);
-  if (err == cudaSuccess) err = ctx->scratch.reserve_large(total);
-  if (err == cudaSuccess) ctx->scratch.reserve_rounds(total);
+  const bool rounds = fjg::rounds_may_run(n_events, total, ctx->num_sms, algo, algo_all, radius, r_all);
+  cudaError_t err = ctx->scratch.reserve(n_events, total, rounds);
   if (err != cudaSuccess) return cuda_error(ctx, err, "scratch allocation");
   cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
   BatchArgs A{};
@@ -329,9 +272,7 @@ fjg_status fjg_cluster_event(fjg_ctx* ctx, const double* p4, int n, int algo, do
     return err == cudaSuccess ? FJG_OK : cuda_error(ctx, err, "fjg_cluster_event");
   }
   if (n > fjg::kLargeMaxN) return set_error(ctx, FJG_ETOOBIG, "event exceeds the supported particle count");
-  cudaError_t werr = ctx->scratch.reserve_ws(n);
-  if (werr == cudaSuccess) werr = ctx->scratch.reserve_large(n);
-  if (werr == cudaSuccess) ctx->scratch.reserve_rounds(n);
+  cudaError_t werr = ctx->scratch.reserve(1, n, fjg::rounds_take(fjg::kRoundsOne, n, algo, r));
   if (werr != cudaSuccess) return cuda_error(ctx, werr, "workspace allocation");
   BatchArgs A{};
   A.phase = ctx->phase;
@@ -376,9 +317,7 @@ fjg_status fjg_cluster_pseudojets(fjg_ctx* ctx, fjg_pseudojet* particles, int si
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
   const size_t b_jets = al(sizeof(double) * 4 * size), b_lab = al(sizeof(int32_t) * size);
   cudaError_t err = ctx->single.reserve(b_jets + b_lab + 256);
-  if (err == cudaSuccess) err = ctx->scratch.reserve_ws(size);
-  if (err == cudaSuccess) err = ctx->scratch.reserve_large(size);
-  if (err == cudaSuccess) ctx->scratch.reserve_rounds(size);
+  if (err == cudaSuccess) err = ctx->scratch.reserve(1, size, fjg::rounds_take(fjg::kRoundsOne, size, algo, r));
   if (err != cudaSuccess) return cuda_error(ctx, err, "device buffers");
   char* d = static_cast<char*>(ctx->single.ptr);
   double* jets = reinterpret_cast<double*>(d);

@@ -42,10 +42,21 @@ struct DeviceBuffer {
 struct ScratchSet {
   Scratch sc{};
   DeviceBuffer lists, ws, large, rounds;
-  cudaError_t reserve_lists(int n_events);         // order/counts/queues/status/hist (+ offsets1)
-  cudaError_t reserve_ws(int64_t particles);       // kWsFields doubles per particle
-  cudaError_t reserve_large(int64_t particles);    // only when particles > kSmemMaxN
-  void reserve_rounds(int64_t particles);          // without it (no memory) the step-by-step kernels run
+  // Room for a call of n_events events and so many particles in all; `rounds`: and
+  // for the rounds kernel, if there is memory (without it the step-by-step
+  // kernels run).  Where the rest does not fit beside the rounds' workspace, that
+  // is given up.
+  cudaError_t reserve(int n_events, int64_t particles, bool rounds);
+
+ private:
+  int64_t no_room = INT64_MAX;  // particles from which on the rounds' workspace was refused
+  cudaError_t grow(DeviceBuffer& b, size_t bytes);
+  cudaError_t reserve_lists(int n_events);       // order/counts/queues/status/hist (+ offsets1)
+  cudaError_t reserve_ws(int64_t particles);     // kWsFields doubles per particle
+  cudaError_t reserve_large(int64_t particles);  // only when particles > kSmemMaxN
+  void reserve_rounds(int64_t particles);
+
+ public:
   void release() {
     lists.release();
     rounds.release();

@@ -31,10 +31,8 @@ fjg_status fjg_graph_capture_batch(fjg_ctx* ctx, const double* p4, const int64_t
   fjg_graph* g = new (std::nothrow) fjg_graph();
   if (!g) return set_error(ctx, FJG_ENOMEM, "host allocation failed");
   g->ctx = ctx;
-  cudaError_t err = g->scratch.reserve_lists(n_events);
-  if (err == cudaSuccess) err = g->scratch.reserve_ws(total);
-  if (err == cudaSuccess) err = g->scratch.reserve_large(total);
-  if (err == cudaSuccess) g->scratch.reserve_rounds(total);
+  cudaError_t err = g->scratch.reserve(n_events, total,
+                                       fjg::rounds_may_run(n_events, total, ctx->num_sms, algo, algo_all, radius, r_all));
   // resolve the per-device launch attributes and occupancies outside the capture
   for (int b = 0; b < fjg::kNumBuckets && err == cudaSuccess; ++b) fjg::variant_occupancy(ctx->tune.bucket[b].variant);
   if (err == cudaSuccess) err = fjg::configure_tiled();

@@ -400,17 +400,36 @@ static int lone_variant(int b) {
 }
 constexpr int kSharedBuckets = 3;  // two CTAs of lone_variant share an SM
 
-// Whether the rounds kernel takes some, and all, of list q's events, as far as
-// the host knows (per-event algorithms and radii are the device's).
-static void rounds_share(const BatchArgs& A, int q, bool* some, bool* all) {
-  *some = A.rounds_mode != kRoundsNone;
-  *all = false;
-  if (!*some || A.algo || A.radius) return;
-  const int lo = q == 0 ? 1 : (128 << q) + 1, hi = q == kLargeQueue ? kLargeMaxN : 256 << q;
-  const bool at_lo = rounds_take(A.rounds_mode, lo, A.algo_all, A.r_all);
-  const bool at_hi = rounds_take(A.rounds_mode, hi, A.algo_all, A.r_all);
-  *some = at_lo || at_hi;  // the rule changes at most once inside a list's range
-  *all = at_lo && at_hi;
+// Whether the rounds kernel takes some, and all, of list q's events, of up to
+// `largest` particles, as far as the host knows (per-event algorithms and radii are
+// the device's: R = 0 stands for any).  The rule changes at most once inside a
+// list's range.
+static void rounds_share(int mode, const int32_t* algo, int algo_all, const double* radius, double r_all, int q,
+                         int64_t largest, bool* some, bool* all) {
+  const int lo = q == 0 ? 1 : (128 << q) + 1, top = q == kLargeQueue ? kLargeMaxN : 256 << q;
+  const int hi = largest < top ? (int)largest : top;
+  const double R = radius ? 0.0 : r_all;
+  *some = false;
+  *all = !algo && !radius;
+  for (int a = algo ? -1 : algo_all; a <= (algo ? 1 : algo_all); ++a) {
+    const bool at_lo = lo <= largest && rounds_take(mode, lo, a, R), at_hi = lo <= largest && rounds_take(mode, hi, a, R);
+    *some |= at_lo || at_hi;
+    *all &= at_lo && at_hi;
+  }
+}
+
+// The rounds kernel's rule by the number of events (rounds_take).
+static int rounds_mode_for(int n_events, int num_sms) {
+  if (n_events == 1) return kRoundsOne;
+  return n_events <= num_sms ? kRoundsFew : n_events <= 2 * num_sms ? kRoundsSome : kRoundsMany;
+}
+
+bool rounds_may_run(int n_events, int64_t particles, int num_sms, const int32_t* algo, int algo_all,
+                    const double* radius, double r_all) {
+  bool some = false, all;
+  for (int q = 0; q < kNumQueues && !some; ++q)
+    rounds_share(rounds_mode_for(n_events, num_sms), algo, algo_all, radius, r_all, q, particles, &some, &all);
+  return some;
 }
 
 // The launches of list q (a bucket, or kLargeQueue) of a batch: the rounds kernel
@@ -447,17 +466,11 @@ static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, 
   return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
 }
 
-// The rounds kernel's rule by the number of events (rounds_take).
-static int rounds_mode_of(const Scratch& sc, int n_events, int num_sms) {
-  if (!sc.round_ws) return kRoundsNone;
-  if (n_events == 1) return kRoundsOne;
-  return n_events <= num_sms ? kRoundsFew : n_events <= 2 * num_sms ? kRoundsSome : kRoundsMany;
-}
-
 cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
                          cudaStream_t stream, cudaStream_t* side, cudaEvent_t* ev_fork, cudaEvent_t* ev_join) {
   BatchArgs base = args;
-  base.rounds_mode = rounds_mode_of(sc, n_events, num_sms);
+  const bool room = sc.round_ws && sc.round_ws_particles >= base.particles;
+  base.rounds_mode = room ? rounds_mode_for(n_events, num_sms) : kRoundsNone;
   cudaError_t err = launch_sort(base, sc, n_events, stream);
   if (err == cudaSuccess && side) err = cudaEventRecord(*ev_fork, stream);
   // largest events first: their list is launched first.  A list that both
@@ -466,7 +479,7 @@ cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events,
   for (int q = kLargeQueue; q >= 0 && err == cudaSuccess; --q) {
     if (q == kLargeQueue && !sc.large_ws) continue;
     bool some, all;
-    rounds_share(base, q, &some, &all);
+    rounds_share(base.rounds_mode, base.algo, base.algo_all, base.radius, base.r_all, q, base.particles, &some, &all);
     for (int k = 0; k < 2 && err == cudaSuccess; ++k) {
       if (k == 0 ? !some : all) continue;
       const int i = q + (k ? kNumQueues : 0);
@@ -524,7 +537,7 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
   A.queue = sc.queues;
   A.ws = sc.ws;
   A.ws_stride = sc.ws_stride;
-  if (sc.round_ws && rounds_take(kRoundsOne, n, base.algo_all, base.r_all)) {
+  if (sc.round_ws && sc.round_ws_particles >= n && rounds_take(kRoundsOne, n, base.algo_all, base.r_all)) {
     A.rounds_mode = kRoundsOne;
     const int q = b < 0 ? kLargeQueue : b, r = retry_list(q);
     A.round_ws = sc.round_ws;

@@ -114,6 +114,10 @@ cudaError_t configure_tiled();
 // The rounds kernel over the work list of A; q: the list's bucket (kLargeQueue
 // above kSmemMaxN particles), which sets threads and tiles.
 cudaError_t launch_rounds(int q, BatchArgs A, int grid, cudaStream_t s);
+// Whether the rounds kernel may take an event of a call of n_events events and so
+// many particles in all (algorithms and radii per event, or for all).
+bool rounds_may_run(int n_events, int64_t particles, int num_sms, const int32_t* algo, int algo_all,
+                    const double* radius, double r_all);
 int rounds_occupancy(int q);  // resident CTAs per SM (sets the launch attributes on first use)
 
 // Launch variant v (a persistent grid of `grid` CTAs); resident CTAs per SM of

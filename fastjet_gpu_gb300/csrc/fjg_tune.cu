@@ -186,8 +186,7 @@ fjg_status fjg_autotune(fjg_ctx* ctx, int algo, double r, int flags, fjg_tuning*
     const int n_events = 3 * ctx->num_sms * max_occ;
     make_events(rng, n_events, lo, cap, hp4, hoff);
     err = tb.load(hp4, hoff, ctx->stream);
-    if (err == cudaSuccess) err = ctx->scratch.reserve_lists(n_events);
-    if (err == cudaSuccess) err = ctx->scratch.reserve_ws(hoff.back());
+    if (err == cudaSuccess) err = ctx->scratch.reserve(n_events, hoff.back(), false);
     double best_s = 1e30;
     for (int v = 0; v < fjg::kNumVariants && err == cudaSuccess; ++v) {
       const fjg::VariantShape sh = fjg::variant_shape(v);

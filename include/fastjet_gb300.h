@@ -46,8 +46,11 @@ typedef enum {
 
 /* Largest event the library clusters (particles per event); larger events
  * are refused with FJG_ETOOBIG.  Events above 4096 particles also need the
- * tiled kernel's workspace (96 bytes per particle of the batch); the rounds
- * kernel's (384 bytes per particle) is used where it can be allocated. */
+ * tiled kernel's workspace (96 bytes per particle of the batch).  The rounds
+ * kernel's (384 bytes per particle) is allocated for calls of which it may take an
+ * event, where there is memory, and given up where another allocation of the
+ * library does not fit beside it.  Workspaces are kept, and made a quarter larger
+ * than the call that they are made for: 120 and 480 bytes. */
 #define FJG_MAX_EVENT_PARTICLES 16777216
 
 /* I/O record of the reference (PseudoJet.h:4-11): 40 bytes, px at offset 8. */

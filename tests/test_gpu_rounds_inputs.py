@@ -73,3 +73,25 @@ def test_sums_that_overflow(ctx):
             except F.FjgError:
                 pass
     _check_event(ctx, base, -1, 0.4, "after")
+
+
+def test_no_workspace_where_the_rounds_take_nothing():
+    """The rounds kernel's workspace (480 bytes a particle) is not allocated for calls
+    that its rule refuses; with it, the results are the same as without."""
+    ctx = F.Context(0)
+    evs = [E.single_event(600, 3, i) for i in range(8)]
+    p4 = torch.from_numpy(np.concatenate(evs * 250)).cuda()
+    off = torch.arange(0, 600 * 2000 + 1, 600, dtype=torch.int64, device="cuda")
+    out = ctx.cluster_batch_device(p4, off, -1, 0.4, out=None)
+    torch.cuda.synchronize()
+    ctx.close()
+    ctx = F.Context(0)
+    free = [torch.cuda.mem_get_info()[0]]
+    for radius in (1.2, 0.4):
+        ctx.cluster_batch_device(p4, off, -1, radius, out=out)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    n = p4.shape[0]
+    assert free[0] - free[1] < 300 * n  # the other workspaces: 70 + 120 bytes a particle
+    assert free[1] - free[2] > 384 * n
+    ctx.close()
