@@ -539,7 +539,7 @@ class Server:
 
     @property
     def launches(self):
-        """Clustering kernels launched so far (one per micro-batch)."""
+        """Clustering kernels launched so far (one per micro-batch, two for the rounds kernel's)."""
         return int(lib().fjg_server_launches(self._h))
 
     def replay(self, particles, offsets, algo, radius, arrival_us):

@@ -20,9 +20,11 @@
 //      complete (flags and its CUDA event) becomes idle again;
 //   2. admission, first come first served: the head request gets an arena
 //      range (first fit) and a slot, or everything waits;
-//   3. launches: per size bucket (largest first), admitted requests go out as
-//      one micro-batch on an idle stream, up to max_batch events and up to
-//      the bucket's in-flight limit (its resident CTAs times oversubscribe).
+//   3. launches: per size bucket (smallest first) and kernel, admitted requests
+//      go out as one micro-batch on an idle stream, up to max_batch events and up
+//      to the bucket's in-flight limit (its resident CTAs times oversubscribe).
+//      A micro-batch is all for the rounds kernel or all for the step-by-step one:
+//      neither waits for the other on the stream.
 // Micro-batches of different buckets and of the same bucket run concurrently
 // on different streams, so requests that arrive while others are running
 // start without waiting for them.
@@ -122,7 +124,7 @@ struct fjg_server {
   std::map<int64_t, int64_t> free_ranges;  // start -> length
   std::vector<int> free_slots;
   std::deque<Req*> pending;
-  std::deque<Req*> admitted[fjg::kNumQueues];
+  std::deque<Req*> admitted[fjg::kNumQueues][2];  // for the step-by-step kernel, and for the rounds kernel
   std::deque<Req*> completed;
   std::unordered_map<uint64_t, Req*> returned;
   std::vector<Lane> lanes;
@@ -185,11 +187,11 @@ void finish(fjg_server* S, Req* r, int status) {
   S->completed.push_back(r);
 }
 
-cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
+cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int route, int m) {
   fjg_ctx* ctx = S->ctx;
   for (int i = 0; i < m; ++i) {
-    Req* r = S->admitted[q].front();
-    S->admitted[q].pop_front();
+    Req* r = S->admitted[q][route].front();
+    S->admitted[q][route].pop_front();
     L.host.offsets[2 * i] = r->start;
     L.host.offsets[2 * i + 1] = r->start + r->n;
     L.host.algo[i] = r->algo;
@@ -242,31 +244,27 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int m) {
     const int per_sm = fjg::bucket_per_sm(ctx->tune, q);
     return fjg::launch_variant(ctx->tune.bucket[q].variant, B, std::min(m, ctx->num_sms * per_sm), per_sm, L.stream);
   };
-  // the rounds kernel's events (the latency rule), the others, and what the
-  // rounds kernel left
-  const int mode = m == 1 ? fjg::kRoundsServeOne : fjg::kRoundsServe;
-  int taken = 0;
-  if (S->d_rounds)
-    for (Req* r : L.batch) taken += fjg::rounds_take(mode, r->n, r->algo, r->r) ? 1 : 0;
-  if (taken) {
-    A.rounds_mode = mode;
+  // a request that has the GPU to itself has a rule of its own
+  bool alone = m == 1;
+  for (const Lane& other : S->lanes) alone &= !other.busy;
+  const Req* first = L.batch[0];
+  if (alone) route = S->d_rounds && fjg::rounds_take(fjg::kRoundsServeOne, first->n, first->algo, first->r) ? 1 : 0;
+  if (route) {
+    // the rounds kernel, then step by step what it left
     fjg::BatchArgs B = A;
+    B.rounds_mode = alone ? fjg::kRoundsServeOne : fjg::kRoundsServe;
     B.queue = L.d_queue + 2;
     B.round_ws = S->d_rounds;
     B.retry = L.d_retry;
     B.n_retry = L.d_queue + 3;
     err = fjg::launch_rounds(q, B, std::min(m, ctx->num_sms * fjg::rounds_occupancy(q)), L.stream);
     if (err != cudaSuccess) return err;
-  }
-  if (taken < m) err = step_by_step(A);
-  if (err == cudaSuccess && taken) {
-    A.rounds_mode = fjg::kRoundsNone;
     A.order = L.d_retry;
     A.n_order = L.d_queue + 3;
     A.queue = L.d_queue + 4;
-    err = step_by_step(A);
   }
-  if (err == cudaSuccess) ++S->launches;
+  err = step_by_step(A);
+  if (err == cudaSuccess) S->launches += route ? 2 : 1;
   if (err == cudaSuccess) err = cudaMemcpyAsync(L.h_status, L.d_status, sizeof(int), cudaMemcpyDeviceToHost, L.stream);
   if (err == cudaSuccess) err = cudaEventRecord(L.ev, L.stream);
   L.busy = true;
@@ -332,7 +330,8 @@ bool progress(fjg_server* S) {
     r->src = nullptr;
     __atomic_store_n(&S->h_done[r->slot], 0, __ATOMIC_RELEASE);
     r->state = kAdmitted;
-    S->admitted[r->bucket].push_back(r);
+    const bool rounds = S->d_rounds && fjg::rounds_take(fjg::kRoundsServe, r->n, r->algo, r->r);
+    S->admitted[r->bucket][rounds ? 1 : 0].push_back(r);
   }
   if (copied && cudaEventRecord(S->ev_copy, S->copy_stream) != cudaSuccess) {
     S->failed = true;
@@ -342,24 +341,24 @@ bool progress(fjg_server* S) {
   // requests); events above 4096 particles take at most half of the streams
   // and of the SMs (a tiled-kernel CTA fills an SM's registers for the whole
   // event), so that they cannot hold every SM away from the small ones
-  for (int q = 0; q <= fjg::kLargeQueue; ++q) {
-    while (!S->admitted[q].empty() && S->inflight[q] < S->limit[q]) {
-      Lane* idle = nullptr;
-      int large_lanes = 0;
-      for (Lane& L : S->lanes) {
-        if (L.busy && L.q == fjg::kLargeQueue) ++large_lanes;
-        if (!L.busy && !idle) idle = &L;
+  for (int q = 0; q <= fjg::kLargeQueue; ++q)
+    for (int route = 0; route < 2; ++route)
+      while (!S->admitted[q][route].empty() && S->inflight[q] < S->limit[q]) {
+        Lane* idle = nullptr;
+        int large_lanes = 0;
+        for (Lane& L : S->lanes) {
+          if (L.busy && L.q == fjg::kLargeQueue) ++large_lanes;
+          if (!L.busy && !idle) idle = &L;
+        }
+        if (!idle) return true;
+        if (q == fjg::kLargeQueue && 2 * large_lanes >= (int)S->lanes.size()) break;
+        const int m = (int)std::min<int64_t>({(int64_t)S->admitted[q][route].size(), (int64_t)S->cfg.max_batch,
+                                              (int64_t)(S->limit[q] - S->inflight[q])});
+        if (launch_lane(S, *idle, q, route, m) != cudaSuccess) {
+          S->failed = true;
+          return false;
+        }
       }
-      if (!idle) return true;
-      if (q == fjg::kLargeQueue && 2 * large_lanes >= (int)S->lanes.size()) break;
-      const int m = (int)std::min<int64_t>(
-          {(int64_t)S->admitted[q].size(), (int64_t)S->cfg.max_batch, (int64_t)(S->limit[q] - S->inflight[q])});
-      if (launch_lane(S, *idle, q, m) != cudaSuccess) {
-        S->failed = true;
-        return false;
-      }
-    }
-  }
   return true;
 }
 
@@ -532,7 +531,8 @@ void fjg_server_destroy(fjg_server* S) {
   }
   for (Req* r : S->pending) delete r;
   for (auto& q : S->admitted)
-    for (Req* r : q) delete r;
+    for (auto& queue : q)
+      for (Req* r : queue) delete r;
   for (Lane& L : S->lanes)
     for (Req* r : L.batch) delete r;  // entries of completed requests are null
   for (Req* r : S->completed) delete r;
