@@ -34,10 +34,8 @@ fjg_status fjg_graph_capture_batch(fjg_ctx* ctx, const double* p4, const int64_t
   cudaError_t err = g->scratch.reserve(n_events, total,
                                        fjg::rounds_may_run(n_events, total, ctx->num_sms, algo, algo_all, radius, r_all));
   // resolve the per-device launch attributes and occupancies outside the capture
-  for (int b = 0; b < fjg::kNumBuckets && err == cudaSuccess; ++b) fjg::variant_occupancy(ctx->tune.bucket[b].variant);
   if (err == cudaSuccess) err = fjg::configure_tiled();
-  for (int q = 0; q < fjg::kNumQueues && err == cudaSuccess; ++q) fjg::rounds_occupancy(q);
-  fjg::launch_priority(0);
+  if (err == cudaSuccess) fjg::prepare_launches(ctx->tune);
   if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
   if (err != cudaSuccess) {
     fjg_graph_destroy(g);

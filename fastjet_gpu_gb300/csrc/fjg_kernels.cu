@@ -466,6 +466,15 @@ static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, 
   return launch_variant(tune.bucket[q].variant, A, bucket_grid(tune, q, num_sms, n_events), bucket_per_sm(tune, q), s);
 }
 
+void prepare_launches(const Tuning& tune) {
+  for (int b = 0; b < kNumBuckets; ++b) {
+    variant_occupancy(tune.bucket[b].variant);
+    variant_occupancy(lone_variant(b));
+  }
+  for (int q = 0; q < kNumQueues; ++q) rounds_occupancy(q);
+  launch_priority(0);
+}
+
 cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events, int num_sms, const Tuning& tune,
                          cudaStream_t stream, cudaStream_t* side, cudaEvent_t* ev_fork, cudaEvent_t* ev_join) {
   BatchArgs base = args;

@@ -127,6 +127,11 @@ int variant_occupancy(int v);        // most CTAs per SM of any build of variant
 int variant_occupancy_plain(int v);  // of its plain build (more takes the register-capped one)
 int bucket_per_sm(const Tuning& tune, int b);  // CTAs per SM that bucket b runs with
 
+// Sets the launch attributes and resolves the occupancies and the priority range of
+// every kernel that launch_batch may launch with `tune` on the current device, so
+// that a launch inside a capture asks the runtime for none of them.
+void prepare_launches(const Tuning& tune);
+
 // Device-side batch descriptor scratch owned by a context.
 struct Scratch {
   int32_t* order;   // [kNumLists][cap_events] (kNumQueues without a rounds workspace)
