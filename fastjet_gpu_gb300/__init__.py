@@ -239,7 +239,9 @@ class Context:
               "r_setup", "r_candidates", "r_range", "r_backs", "r_b", "r_c", "r_d", "r_e", "r_f", "r_sort", "r_outputs",
               "r_rounds", "r_steps", "r_events", "r_retries", "r_cands",
               "r_conflict_a", "r_conflict_b", "r_conflict_d", "r_targets", "r_kin",
-              "r_role0", "r_role1", "r_role2", "r_scan", "r_new_jet", "r_search", "r_dead", "r_overflows", "r_undone")
+              "r_role0", "r_role1", "r_role2", "r_scan", "r_new_jet", "r_search", "r_dead", "r_overflows", "r_undone",
+              "shape_64x4", "shape_128x2", "shape_64x8", "shape_128x4", "shape_256x2", "shape_128x8", "shape_256x4",
+              "shape_256x8", "shape_512x4", "shape_512x8", "shape_256x16", "shape_capped")
 
     def phase_clocks(self, reset=False):
         """Per-step phase counters of the clustering kernels (only in the

@@ -75,7 +75,10 @@ enum PhaseSlot {
   kPhRSteps, kPhREvents, kPhRRetries, kPhRCands,
   kPhRConflictA, kPhRConflictB, kPhRConflictD, kPhRTargets, kPhRKin,
   kPhRRole0, kPhRRole1, kPhRRole2, kPhRScan, kPhRNewJet, kPhRSearch, kPhRDead, kPhROverflows, kPhRUndone,
-  kPhSlots = 62
+  // events per shape of the shared-memory kernel (variant_shape), and how many of
+  // them in its capped build
+  kPhShape = 62, kPhCapped = kPhShape + 11,
+  kPhSlots = kPhCapped + 1
 };
 #ifdef FJG_PHASE_CLOCKS
 #define FJG_PH(...) __VA_ARGS__

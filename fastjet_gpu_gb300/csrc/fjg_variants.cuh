@@ -14,7 +14,17 @@
 
 namespace fjg {
 
+#ifdef FJG_PHASE_CLOCKS
+static_assert(kPhCapped - kPhShape == kNumVariants, "a counter per shape");
 template <int T, int SPT>
+__device__ __forceinline__ void count_shape(const BatchArgs& A, bool capped) {
+  for (int v = 0; v < kNumVariants; ++v)
+    if (variant_shape(v).threads == T && variant_shape(v).spt == SPT) atomicAdd(A.phase + kPhShape + v, 1ull);
+  if (capped) atomicAdd(A.phase + kPhCapped, 1ull);
+}
+#endif
+
+template <int T, int SPT, bool CAPPED>
 __device__ __forceinline__ void smem_event_loop(const BatchArgs& A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemLayout<T, SPT>& S = *reinterpret_cast<SmemLayout<T, SPT>*>(smem_raw);
@@ -32,6 +42,7 @@ __device__ __forceinline__ void smem_event_loop(const BatchArgs& A) {
       continue;
     }
     if (refused_event(A, e)) continue;  // ends with a barrier
+    FJG_PH(if (threadIdx.x == 0 && A.phase) count_shape<T, SPT>(A, CAPPED);)
     cluster_event_smem<T, SPT>(S, A, e);  // ends with a barrier
     if (threadIdx.x == 0) signal_done(A, e);
   }
@@ -39,12 +50,12 @@ __device__ __forceinline__ void smem_event_loop(const BatchArgs& A) {
 
 template <int T, int SPT>
 __global__ void __launch_bounds__(T) k_cluster_smem(BatchArgs A) {
-  smem_event_loop<T, SPT>(A);
+  smem_event_loop<T, SPT, false>(A);
 }
 
 template <int T, int SPT, int MINB>
 __global__ void __launch_bounds__(T, MINB) k_cluster_smem_capped(BatchArgs A) {
-  smem_event_loop<T, SPT>(A);
+  smem_event_loop<T, SPT, true>(A);
 }
 
 // Dynamic shared memory attribute, set once per device and kernel.
