@@ -1118,13 +1118,11 @@ struct RoundPair {
   double2 pc, pj;
   int2 lc, lj;
   int fj;
-  float hold;
 };
 
 template <bool SM>
 __device__ __forceinline__ RoundPair round_pair(const RoundWs<SM>& W, int c, int j) {
-  return RoundPair{W.w(c), W.w(j), W.tm(c), W.tm(j), W.pos(c), W.pos(j), W.tl(c), W.tl(j), (int)W.nn(j),
-                   fmaxf(W.slots[c].hold, W.slots[j].hold)};
+  return RoundPair{W.w(c), W.w(j), W.tm(c), W.tm(j), W.pos(c), W.pos(j), W.tl(c), W.tl(j), (int)W.nn(j)};
 }
 
 // The step of slot c with partner j (-1: none): its key, its time and whether it
@@ -1161,10 +1159,13 @@ __device__ __forceinline__ RoundStep round_step(int c, int j, const RoundPair& p
   return s;
 }
 
-// Whether a step of time P has to wait: its slots are held until nothing with a
-// time up to `hold` (0: not held) is left, and the earliest step of all never is.
-// The bounds on times are good to 2^-15.
-__device__ __forceinline__ bool round_held(float hold, float P, float p_min) {
+// Whether the step of slots c and j, of time P, has to wait: they are held until
+// nothing with a time up to `hold` (0: not held) is left; the earliest step of all
+// never is.  The bounds on times are good to 2^-15.  (Asked only after a conflict.)
+template <bool SM>
+__device__ __noinline__ bool round_held(int c, int j, float P) {
+  const RoundCtx<SM> C = round_ctx<SM>();
+  const float hold = fmaxf(C.W.slots[c].hold, C.W.slots[j].hold), p_min = __uint_as_float(C.S->p_min);
   return hold > 0.0f && P >= hold * (1.0f - 0x1p-13f) && p_min < P && p_min <= hold * (1.0f + 0x1p-13f);
 }
 
@@ -1872,7 +1873,7 @@ __device__ __forceinline__ bool cluster_event_rounds(RoundShared& S, const Batch
         const int bc = round_bit<SM>(c), bj = round_bit<SM>(jc);
         bool ok = care == 2;
         if (SM) pair = round_pair(Wk, c, jc);
-        if (!ok && !round_held(pair.hold, __uint_as_float(me), __uint_as_float(S.p_min))) {
+        if (!ok && !(S.backs && round_held<SM>(c, jc, __uint_as_float(me)))) {
           ok = round_first(S.taken, min(bc, bj));
           if (ok && bc != bj) ok = round_first(S.taken, max(bc, bj));
         }
