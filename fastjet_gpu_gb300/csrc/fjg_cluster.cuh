@@ -123,6 +123,7 @@ struct BatchArgs {
   int32_t* n_retry;
   double tile_factor;      // tiled path: tile side >= tile_factor * R (>= 1)
   int serve_order;         // launch priority (host side): 0 largest events first, 1 smallest first
+  int captured;            // (host side) the launches go into a graph
   int pairs;               // offsets hold (start, end) pairs: events need not be contiguous
   int* done;               // null, or completion flags: done[done_slot[e]] = 1 (system scope) per event
   const int32_t* done_slot;

@@ -56,6 +56,7 @@ fjg_status fjg_graph_capture_batch(fjg_ctx* ctx, const double* p4, const int64_t
   A.history = reinterpret_cast<fjg::StepRec*>(out->history);
   A.owner = out->owner;
   A.status = g->scratch.sc.status;
+  A.captured = 1;
   cudaGraph_t cg = nullptr;
   err = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
   if (err == cudaSuccess) {

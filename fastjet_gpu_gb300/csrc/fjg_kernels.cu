@@ -435,11 +435,10 @@ bool rounds_may_run(int n_events, int64_t particles, int num_sms, const int32_t*
 // The launches of list q (a bucket, or kLargeQueue) of a batch: the rounds kernel
 // for its events, the step-by-step kernel for the others, and the step-by-step
 // kernel, in the list's shape, for the events that the rounds kernel left (mostly
-// none: it ends at once).  One launch of 512 threads per event for all lists, after
-// the last of them, took 19.2 ms instead of 9.0 for 1024 kt events of 700 particles of
-// which each has one without pT, 32.8 instead of 20.8 for C/A events with particles on a
-// lattice; and cost a captured graph of 662 events that uses no rounds 2.2 of 15.7 ms.
-// In the CTA of the rounds, whose shape is not made for it: 12.7 and 29.2.
+// none: it ends at once).  One launch of 512 threads per event for all lists took
+// 19.2 ms instead of 9.0 for 1024 kt events of 700 particles of which each has one
+// without pT, 45.8 instead of 32.7 for 1500; in the CTA of the rounds, whose shape is
+// not made for it, 700 took 12.7.
 enum ListPart { kPartRounds, kPartSteps, kPartRetry };
 
 static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, ListPart part, int n_events,
@@ -481,25 +480,33 @@ cudaError_t launch_batch(const BatchArgs& args, const Scratch& sc, int n_events,
   const bool room = sc.round_ws && sc.round_ws_particles >= base.particles;
   base.rounds_mode = room ? rounds_mode_for(n_events, num_sms) : kRoundsNone;
   cudaError_t err = launch_sort(base, sc, n_events, stream);
+  bool some[kNumQueues] = {}, all[kNumQueues] = {};
+  for (int q = 0; q < kNumQueues; ++q) {
+    rounds_share(base.rounds_mode, base.algo, base.algo_all, base.radius, base.r_all, q, base.particles, &some[q], &all[q]);
+    if (q == kLargeQueue && !sc.large_ws) some[q] = false, all[q] = true;
+  }
+  // Largest events first: their list is launched first.  A list that both kernels
+  // work on has them side by side (the rounds kernel's streams come first).  What the
+  // rounds leave: in a graph after the list's rounds, on their branch; else after
+  // all lists, one list after the other.  Almost always those launches have nothing
+  // to do, but they move the order in which the lists' CTAs get the SMs.  After all
+  // lists a graph of 662 events, anti-kt R = 0.8, took 15.9 instead of 13.2 ms; on the
+  // lists' streams a batch of 4096 events took 19.5 instead of 17.2 ms in 34 of 168
+  // samples, after all lists in 4 of 138.
   if (err == cudaSuccess && side) err = cudaEventRecord(*ev_fork, stream);
-  // largest events first: their list is launched first.  A list that both
-  // kernels work on has them side by side (the rounds kernel's streams come
-  // first); what the rounds kernel leaves follows it on its stream.
-  for (int q = kLargeQueue; q >= 0 && err == cudaSuccess; --q) {
-    if (q == kLargeQueue && !sc.large_ws) continue;
-    bool some, all;
-    rounds_share(base.rounds_mode, base.algo, base.algo_all, base.radius, base.r_all, q, base.particles, &some, &all);
+  for (int q = kLargeQueue; q >= 0; --q)
     for (int k = 0; k < 2 && err == cudaSuccess; ++k) {
-      if (k == 0 ? !some : all) continue;
+      if (k == 0 ? !some[q] : all[q]) continue;
       const int i = q + (k ? kNumQueues : 0);
       cudaStream_t s = side ? side[i] : stream;
       if (side && (err = cudaStreamWaitEvent(s, *ev_fork, 0)) != cudaSuccess) break;
       err = launch_list(base, sc, q, k ? kPartSteps : kPartRounds, n_events, num_sms, tune, s);
-      if (err == cudaSuccess && k == 0) err = launch_list(base, sc, q, kPartRetry, n_events, num_sms, tune, s);
+      if (err == cudaSuccess && k == 0 && base.captured) err = launch_list(base, sc, q, kPartRetry, n_events, num_sms, tune, s);
       if (err == cudaSuccess && side) err = cudaEventRecord(ev_join[i], s);
       if (err == cudaSuccess && side) err = cudaStreamWaitEvent(stream, ev_join[i], 0);
     }
-  }
+  for (int q = kLargeQueue; q >= 0 && !base.captured && err == cudaSuccess; --q)
+    if (some[q]) err = launch_list(base, sc, q, kPartRetry, n_events, num_sms, tune, stream);
   return err;
 }
 
