@@ -51,12 +51,14 @@ from fastjet_gpu_gb300 import events as E  # noqa: E402
 ALGO, RADIUS = -1, 0.4
 WORKLOADS = {
     "mixed": dict(
-        events=4096, make=lambda n: E.mixed_batch(n, 50, 2000, seed=3), flush=True, cpu_start=64,
+        # kernels a step: 2 input checks, 4 for the lists, the rounds on 5 lists and what they leave, 2 step by step
+        launches=18, events=4096, make=lambda n: E.mixed_batch(n, 50, 2000, seed=3), flush=True, cpu_start=64,
         per_event_sample=256, second=None, dominant=(1024, 2048, "k_cluster_rounds, events of 1025-2048 particles"),
         metric="events/s, batched anti-kt R=0.4 clustering of 4096 events (50-2000 particles)",
         workload="4096 events, particle counts log-uniform in [50, 2000], anti-kt R=0.4, FP64, one batched call"),
     "pileup": dict(
-        events=64, make=lambda n: E.pileup_batch(n, 10000, 60000, seed=4), flush=True, cpu_start=16,
+        # (64 events: step by step on the smallest list only)
+        launches=17, events=64, make=lambda n: E.pileup_batch(n, 10000, 60000, seed=4), flush=True, cpu_start=16,
         per_event_sample=4, second=(1, 0.6), dominant=None,
         metric="events/s, batched anti-kt R=0.4 clustering of 64 pile-up events (10k-60k particles)",
         workload="64 pile-up-like events, 10k-60k particles, anti-kt R=0.4 (kt R=0.6 beside it), FP64, "
@@ -75,8 +77,8 @@ SERVING_RATES = (2000, 4000, 20000, 50000, 100000, 200000)  # the first two belo
 # measured 336.2 MB of dram__bytes_read.sum + dram__bytes_write.sum for 604,303
 # particles, most of it the workspace's first touch and write-back
 TRAFFIC_B_PER_PARTICLE = 556.3
-# the same for its events above 4096 particles: 2.8 MB for one of 16,000
-TRAFFIC_LARGE_B_PER_PARTICLE = 173.0
+# the same for its events above 4096 particles: 2.57 MB for one of 16,000
+TRAFFIC_LARGE_B_PER_PARTICLE = 160.7
 W = WORKLOADS["mixed"]
 N_EVENTS = W["events"]
 METRIC = W["metric"]
@@ -639,7 +641,7 @@ def run_ours(args, rank, world, local_rank):
                              {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                               "frac": achieved / peak,
                               "note": f"whole step, staging only ({alg_bytes} B per step); peak {peak_kind}"}]},
-            "gpu_launches": args.steps * 15,  # 2 input checks, 4 bucketing kernels, 7 list kernels, 2 for what conflicts left
+            "gpu_launches": args.steps * W["launches"],
             "clocks": clk.summary(),
             "wall_s": t_wall}
     if second is not None:

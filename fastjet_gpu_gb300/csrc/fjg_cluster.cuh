@@ -115,7 +115,9 @@ struct BatchArgs {
   int32_t* owner;          // [total] or null
   int* status;             // device error flag (0 = ok)
   unsigned char* large_ws; // tiled-path workspace: event e at large_ws + 96 * offsets[e] (null: none)
-  int rounds_mode;         // which events the rounds kernel takes (rounds_take); the others skip them
+  int rounds_mode;         // which events the rounds kernel takes (rounds_take)
+  int rounds_from;         // of this list: those of at least so many particles (0: none; -1: by rounds_take,
+                           // per event); the other kernels skip them
   unsigned char* round_ws; // rounds kernel's workspace: event e at round_ws + kRoundBytesPerParticle * offsets[e]
   int round_tiles, round_cells, round_slots;  // rounds kernel: what its shared memory has room for (tiles,
                                               // tiles with their frame, slots)

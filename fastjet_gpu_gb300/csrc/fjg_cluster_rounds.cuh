@@ -58,9 +58,9 @@
 // in about 2 % of anti-kt R = 0.8 events of 3000 and in 2 to 8 % of dense anti-kt
 // R = 0.4 events of 8000 to 15,000; those of 40,000 and more, where a hard jet's
 // chain of steps reaches further, have one or several.  A conflict costs 30 to 900
-// rounds (6000 to 10,000 dense particles), so events above 20,000 begin with 1.8 R: 64 events of
-// 10,000 to 60,000 particles have 3 to 11 conflicts (10 samples) and take 314 to
-// 330 ms, 333 to 345 with 2.0 R, 308 to 434 with 1.5 R.
+// rounds (6000 to 10,000 dense particles), so events above 20,000 begin with 1.8 R: six
+// batches of 64 events of 10,000 to 60,000 particles take 320 to 332 ms, 320 to 338 with
+// 1.5 R, 304 to 373 with 1.65 R, 341 to 357 with 2.0 R.
 //
 // A round (F steps), eight warps or so:
 //   A   candidates (a thread per tile); range test (eight lanes per candidate),
@@ -108,7 +108,8 @@ namespace fjg {
 //          kt R 0.6: 200 0.72 (0.95), R 1.0: 320 0.64 (0.83), R 1.3: 600 0.77 (0.90), R 1.5: 700 0.92, 3000 1.03
 //          C/A R 0.8: 160 0.80, R 1.2: 320 0.74 (0.93)
 //   Few,   R 0.4: 200 1.15-1.38, 256 1.02-1.12 (Some: 1.04-1.26), 320 0.76-0.86, 1000 0.37-0.53;  R 0.5: 320 0.76-0.94
-//   Some   R 0.6: 320 0.89-1.06, 512 0.78-0.99, 600 0.68-0.82;  R 0.7: 600 0.83-0.95, 2000 0.77-0.89
+//   Some   (of 96 events of 17 to 301, few of them near the largest: rounds from 224 on 0.77 ms, from 257 on 0.83)
+//          R 0.6: 320 0.89-1.06, 512 0.78-0.99, 600 0.68-0.82;  R 0.7: 600 0.83-0.95, 2000 0.77-0.89
 //          R 0.8: 320 1.15-1.31, 1000 0.89-1.02, 3000 0.87-1.11
 //          kt R 0.6: 256 0.84-1.03, 320 0.63-0.84, R 1.0: 320 0.82-1.09, 700 0.59-0.71, R 1.3: 600 0.87-0.99,
 //          R 1.5: 700 1.04-1.17;  C/A R 0.8: 256 0.87-1.18, 320 0.71-0.92, R 1.2: 512 0.80-1.05, 700 0.72-0.88
@@ -129,7 +130,7 @@ namespace fjg {
 enum { kRoundsNone = 0, kRoundsMany, kRoundsSome, kRoundsFew, kRoundsOne, kRoundsServe, kRoundsServeOne };
 
 // In each mode the rule falls with R, and with n it changes at most once among the
-// sizes of one list (rounds_share counts on both).
+// sizes of one list, from refusing to taking (the launchers count on it).
 __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R) {
   if (mode == kRoundsNone) return false;
   const bool antikt = algo == -1, alone = mode == kRoundsOne || mode == kRoundsServeOne;
@@ -139,7 +140,7 @@ __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R)
       if (antikt) return R <= 0.45 ? n >= 224 : R <= 0.65 ? n >= 320 : R <= 0.85 && n > 512;
       return R <= 0.8 ? n >= 200 : R <= 1.3 && n >= 320;
     case kRoundsFew:
-      if (R <= (antikt ? 0.45 : 0.8)) return n > 256;
+      if (R <= (antikt ? 0.45 : 0.8)) return n >= 224;
       return R <= (antikt ? 0.55 : 1.0) ? n >= 320 : R <= (antikt ? 0.7 : 1.3) && n >= 600;
     case kRoundsSome: return R <= (antikt ? 0.55 : 0.8) ? n >= 320 : R <= (antikt ? 0.7 : 1.3) && n >= 600;
     case kRoundsServeOne: return R <= (antikt ? 0.85 : 1.2) && n >= 112;
@@ -150,13 +151,32 @@ __host__ __device__ inline bool rounds_take(int mode, int n, int algo, double R)
   }
 }
 
-// The same for an event of a batch.
+// The same for an event of a batch.  With one algorithm and R for all it is a
+// comparison, and one thread of a CTA asks (next_event): the rule in line in every
+// thread's event loop took a graph of 1024 events 5.38 -> 5.58 ms and a batch of 4096
+// 17.5 -> 18.0.
+static __device__ __noinline__ bool rounds_take_event(const BatchArgs* A, int e, int n) {
+  return rounds_take(A->rounds_mode, n, A->algo ? A->algo[e] : A->algo_all, A->radius ? A->radius[e] : A->r_all);
+}
+
 __device__ __forceinline__ bool rounds_event(const BatchArgs& A, int e) {
-  if (A.rounds_mode == kRoundsNone) return false;
+  if (A.rounds_from == 0) return false;
   int64_t off;
   int n;
   event_range(A, e, off, n);
-  return rounds_take(A.rounds_mode, n, A.algo ? A.algo[e] : A.algo_all, A.radius ? A.radius[e] : A.r_all);
+  return A.rounds_from > 0 ? n >= A.rounds_from : rounds_take_event(&A, e, n);
+}
+
+// The next event of the list that is for the rounds kernel, or for the others; -1:
+// none is left (one thread of a CTA).
+__device__ __forceinline__ int next_event(const BatchArgs& A, int count, bool rounds) {
+#pragma unroll 1
+  for (;;) {
+    const int q = atomicAdd(A.queue, 1);
+    if (q >= count) return -1;
+    const int e = A.order[q];
+    if (rounds_event(A, e) == rounds) return e;
+  }
 }
 
 constexpr int kRoundSteps = 32;               // steps per round, at most (a lane each)

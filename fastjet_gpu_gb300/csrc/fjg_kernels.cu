@@ -9,17 +9,10 @@ __global__ void __launch_bounds__(kTiledT, 1) k_cluster_tiled(BatchArgs A) {
   __shared__ TiledShared S;
   const int count = *A.n_order;
   for (;;) {
-    if (threadIdx.x == 0) {
-      const int q = atomicAdd(A.queue, 1);
-      S.event = (q < count) ? A.order[q] : -1;
-    }
+    if (threadIdx.x == 0) S.event = next_event(A, count, false);
     __syncthreads();
     const int e = S.event;
     if (e < 0) break;
-    if (rounds_event(A, e)) {
-      __syncthreads();  // everyone has read S.event
-      continue;
-    }
     if (refused_event(A, e)) continue;  // ends with a barrier
     cluster_event_tiled(S, A, A.large_ws, e);  // ends with a barrier
     if (threadIdx.x == 0) signal_done(A, e);
@@ -400,22 +393,40 @@ static int lone_variant(int b) {
 }
 constexpr int kSharedBuckets = 3;  // two CTAs of lone_variant share an SM
 
-// Whether the rounds kernel takes some, and all, of list q's events, of up to
-// `largest` particles, as far as the host knows (per-event algorithms and radii are
-// the device's: R = 0 stands for any).  The rule changes at most once inside a
-// list's range.
+// Sizes of list q's events, of up to `largest` particles.
+static bool list_sizes(int q, int64_t largest, int* lo, int* hi) {
+  const int top = q == kLargeQueue ? kLargeMaxN : 256 << q;
+  *lo = q == 0 ? 1 : (128 << q) + 1;
+  *hi = largest < top ? (int)largest : top;
+  return *lo <= *hi;
+}
+
+// Whether the rounds kernel takes some, and all, of list q's events, as far as the host
+// knows (per-event algorithms and radii are the device's: R = 0 stands for any).
 static void rounds_share(int mode, const int32_t* algo, int algo_all, const double* radius, double r_all, int q,
                          int64_t largest, bool* some, bool* all) {
-  const int lo = q == 0 ? 1 : (128 << q) + 1, top = q == kLargeQueue ? kLargeMaxN : 256 << q;
-  const int hi = largest < top ? (int)largest : top;
+  int lo, hi;
+  const bool any = list_sizes(q, largest, &lo, &hi);
   const double R = radius ? 0.0 : r_all;
   *some = false;
-  *all = !algo && !radius;
-  for (int a = algo ? -1 : algo_all; a <= (algo ? 1 : algo_all); ++a) {
-    const bool at_lo = lo <= largest && rounds_take(mode, lo, a, R), at_hi = lo <= largest && rounds_take(mode, hi, a, R);
-    *some |= at_lo || at_hi;
-    *all &= at_lo && at_hi;
+  *all = any && !algo && !radius;
+  for (int a = algo ? -1 : algo_all; any && a <= (algo ? 1 : algo_all); ++a) {
+    *some |= rounds_take(mode, hi, a, R);
+    *all &= rounds_take(mode, lo, a, R);
   }
+}
+
+// From which size on the rounds kernel takes list q's events (BatchArgs::rounds_from).
+static int rounds_from_of(const BatchArgs& A, int q) {
+  if (A.rounds_mode == kRoundsNone) return 0;
+  if (A.algo || A.radius) return -1;
+  int lo, hi;
+  if (!list_sizes(q, A.particles, &lo, &hi) || !rounds_take(A.rounds_mode, hi, A.algo_all, A.r_all)) return 0;
+  while (lo < hi) {
+    const int mid = lo + (hi - lo) / 2;
+    if (rounds_take(A.rounds_mode, mid, A.algo_all, A.r_all)) hi = mid; else lo = mid + 1;
+  }
+  return hi;
 }
 
 // The rounds kernel's rule by the number of events (rounds_take).
@@ -444,6 +455,7 @@ enum ListPart { kPartRounds, kPartSteps, kPartRetry };
 static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, ListPart part, int n_events,
                                int num_sms, const Tuning& tune, cudaStream_t s) {
   BatchArgs A = base;
+  A.rounds_from = part == kPartRetry ? 0 : rounds_from_of(base, q);
   const int list = part == kPartRetry ? retry_list(q) : q;
   A.order = sc.order + list * sc.cap_events;
   A.n_order = sc.counts + list;
@@ -458,7 +470,6 @@ static cudaError_t launch_list(const BatchArgs& base, const Scratch& sc, int q, 
     const int grid = num_sms * rounds_occupancy(q);
     return launch_rounds(q, A, grid > n_events ? n_events : grid, s);
   }
-  if (part == kPartRetry) A.rounds_mode = kRoundsNone;
   if (q == kLargeQueue) return launch_large(A, sc, n_events, num_sms, tune, s);
   if (n_events <= num_sms || (n_events <= 2 * num_sms && q < kSharedBuckets))
     return launch_variant(lone_variant(q), A, n_events, 1, s);
@@ -555,12 +566,13 @@ cudaError_t launch_single(const BatchArgs& base, const Scratch& sc, int n, const
   A.ws_stride = sc.ws_stride;
   if (sc.round_ws && sc.round_ws_particles >= n && rounds_take(kRoundsOne, n, base.algo_all, base.r_all)) {
     A.rounds_mode = kRoundsOne;
+    A.rounds_from = 1;
     const int q = b < 0 ? kLargeQueue : b, r = retry_list(q);
     A.round_ws = sc.round_ws;
     A.retry = sc.order + r * sc.cap_events;
     A.n_retry = sc.counts + r;
     if ((err = launch_rounds(q, A, 1, stream)) != cudaSuccess) return err;
-    A.rounds_mode = kRoundsNone;
+    A.rounds_from = 0;
     A.order = A.retry;
     A.n_order = A.n_retry;
     A.queue = sc.queues + r;

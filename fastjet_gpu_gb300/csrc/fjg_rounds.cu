@@ -15,17 +15,10 @@ __global__ void __launch_bounds__(T, MINB) k_cluster_rounds(BatchArgs A) {
   }
   const int count = *A.n_order;
   for (;;) {
-    if (threadIdx.x == 0) {
-      const int q = atomicAdd(A.queue, 1);
-      S.event = (q < count) ? A.order[q] : -1;
-    }
+    if (threadIdx.x == 0) S.event = next_event(A, count, true);
     __syncthreads();
     const int e = S.event;
     if (e < 0) break;
-    if (!rounds_event(A, e)) {
-      __syncthreads();  // everyone has read S.event
-      continue;
-    }
     if (refused_event(A, e)) continue;  // ends with a barrier
     const bool done = cluster_event_rounds<T, SM>(S, A, e);
     __syncthreads();

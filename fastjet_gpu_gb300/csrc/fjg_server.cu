@@ -253,6 +253,7 @@ cudaError_t launch_lane(fjg_server* S, Lane& L, int q, int route, int m) {
     // the rounds kernel, then step by step what it left
     fjg::BatchArgs B = A;
     B.rounds_mode = alone ? fjg::kRoundsServeOne : fjg::kRoundsServe;
+    B.rounds_from = 1;
     B.queue = L.d_queue + 2;
     B.round_ws = S->d_rounds;
     B.retry = L.d_retry;

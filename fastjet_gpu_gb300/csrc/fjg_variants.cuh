@@ -30,17 +30,10 @@ __device__ __forceinline__ void smem_event_loop(const BatchArgs& A) {
   SmemLayout<T, SPT>& S = *reinterpret_cast<SmemLayout<T, SPT>*>(smem_raw);
   const int count = *A.n_order;
   for (;;) {
-    if (threadIdx.x == 0) {
-      const int q = atomicAdd(A.queue, 1);
-      S.event = (q < count) ? A.order[q] : -1;
-    }
+    if (threadIdx.x == 0) S.event = next_event(A, count, false);
     __syncthreads();
     const int e = S.event;
     if (e < 0) break;
-    if (rounds_event(A, e)) {
-      __syncthreads();  // everyone has read S.event
-      continue;
-    }
     if (refused_event(A, e)) continue;  // ends with a barrier
     FJG_PH(if (threadIdx.x == 0 && A.phase) count_shape<T, SPT>(A, CAPPED);)
     cluster_event_smem<T, SPT>(S, A, e);  // ends with a barrier

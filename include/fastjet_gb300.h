@@ -215,10 +215,10 @@ void fjg_graph_destroy(fjg_graph* graph);
  * large_ctas_per_sm CTAs per SM (one is resident per SM) and rapidity-azimuth
  * tiles of side at least tile_factor * R (tile_factor >= 1), larger where an
  * event is sparse (about 32 particles per tile).  The choice concerns events
- * that are clustered step by step in calls of more events than the GPU has SMs:
- * in smaller calls each event has the widest CTA, and the events that the rounds
- * kernel takes have shapes of their own.  Every choice gives identical
- * results; only the speed differs. */
+ * that are clustered step by step in calls of more events than the GPU has SMs
+ * (buckets 0-2: than twice as many): in smaller calls each event has the widest
+ * CTA, and the events that the rounds kernel takes have shapes of their own.  Every
+ * choice gives identical results; only the speed differs. */
 #define FJG_NUM_BUCKETS 5
 typedef struct {
   int32_t threads[FJG_NUM_BUCKETS];          /* CTA size: 64 .. 512 */

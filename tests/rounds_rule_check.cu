@@ -1,7 +1,7 @@
 // Host check of the rule that hands an event to the rounds kernel (rounds_take),
 // built with nvcc and run on the CPU by tests/test_rounds_rule.py.  What the
 // launchers count on, in every mode: the rule falls with R, and along the sizes of
-// one list it changes at most once; and an event in a call of several is never
+// one list it changes at most once, from refusing to taking; and an event in a call of several is never
 // taken where it would not be alone (a call lasts as long as its slowest event).
 // Prints "ok <checks>".
 #include <cstdio>
@@ -21,6 +21,10 @@ int main() {
           int changes = 0;
           for (int n = lo; n <= hi; ++n, ++checks) {
             changes += n > lo && rounds_take(mode, n, algo, R) != rounds_take(mode, n - 1, algo, R);
+            if (n > lo && !rounds_take(mode, n, algo, R) && rounds_take(mode, n - 1, algo, R)) {
+              std::printf("mode %d algo %d R %g: %d taken, %d not\n", mode, algo, R, n - 1, n);
+              return 1;
+            }
             for (double S : radii)
               if (S < R && rounds_take(mode, n, algo, R) && !rounds_take(mode, n, algo, S)) {
                 std::printf("mode %d algo %d n %d: taken at R %g, not at %g\n", mode, algo, n, R, S);
